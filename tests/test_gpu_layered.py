@@ -87,6 +87,25 @@ def test_dense_matmul_many_tiles(cuda, dev):
     cuda.release(h)
 
 
+@pytest.mark.parametrize("n", [1030, 4700, 4740, 9400, 9500])
+def test_dense_matmul_tile_widths_of_short_prompts(cuda, dev, n):
+    """Tiles of 32, 64 and 128 columns on both sides of the lines between them (one wave of 148 CTAs), more steps than ring
+    slots, a ragged last tile; the bound of test_dense_matmul."""
+    import torch
+
+    from sharpmind_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    m, k = 97, 1416
+    w = torch.randn((n, k), generator=g, device="cuda").to(torch.bfloat16)
+    x = torch.randn((m, k), generator=g, device="cuda")
+    h = cuda.register_dev(w.view(torch.uint8).reshape(-1), ops.QuantDType.BF16, n, k, repack=False)
+    got = dev.qmatmul(x, h, ops.Mode.ACT_BF16)
+    want = x.to(torch.bfloat16).double() @ w.double().T
+    assert float((got.double() - want).abs().max()) < 1e-5 * k ** 0.5 * 4
+    cuda.release(h)
+
+
 @pytest.mark.parametrize("n", [8, 96, 1000])
 @pytest.mark.parametrize("offset", [0.0, 1.0])
 def test_scaled_add_rmsnorm(dev, n, offset):
