@@ -58,6 +58,91 @@ __device__ __forceinline__ void mma6(float (&c)[4], const uint32_t (&ah)[4], con
     mma_bf16(c, ah, b0[0], b1[0]);
 }
 
+// a float4 as three planes of four bf16 each
+__device__ __forceinline__ void split_store(float4 v, uint8_t *dst, int plane)
+{
+    __nv_bfloat16 p[3][4];
+    split3(v.x, p[0][0], p[1][0], p[2][0]), split3(v.y, p[0][1], p[1][1], p[2][1]);
+    split3(v.z, p[0][2], p[1][2], p[2][2]), split3(v.w, p[0][3], p[1][3], p[2][3]);
+#pragma unroll
+    for (int pl = 0; pl < 3; ++pl) *reinterpret_cast<uint2 *>(dst + pl * plane) = make_uint2(pack2(p[pl][0], p[pl][1]), pack2(p[pl][2], p[pl][3]));
+}
+
+// S = Q K^T of 16 rows x 16 NP keys; qa / ka: this lane's ldmatrix addresses in the first planes
+template <int HD, int NP>
+__device__ __forceinline__ void scores_of_tile(uint32_t qa, int qplane, uint32_t ka, int kplane, float (&s)[2 * NP][4])
+{
+    float s2[2 * NP][4];  // s, s2: even and odd k-steps: two independent chains of dependent MMAs per key tile
+#pragma unroll
+    for (int n = 0; n < 2 * NP; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = s2[n][0] = s2[n][1] = s2[n][2] = s2[n][3] = 0.f;
+#pragma unroll
+    for (int ks = 0; ks < HD / 16; ++ks) {
+        uint32_t ah[4], am[4], al[4];
+        ldsm4(qa + 32 * ks, ah);
+        ldsm4(qa + qplane + 32 * ks, am);
+        ldsm4(qa + 2 * qplane + 32 * ks, al);
+#pragma unroll
+        for (int np = 0; np < NP; ++np) {  // two key tiles per ldmatrix
+            uint32_t b[3][4];
+#pragma unroll
+            for (int pl = 0; pl < 3; ++pl) ldsm4(ka + pl * kplane + np * 16 * (HD * 2 + 16) + 32 * ks, b[pl]);
+            const uint32_t b0a[3] = {b[0][0], b[1][0], b[2][0]}, b1a[3] = {b[0][1], b[1][1], b[2][1]};
+            const uint32_t b0b[3] = {b[0][2], b[1][2], b[2][2]}, b1b[3] = {b[0][3], b[1][3], b[2][3]};
+            if (ks & 1) {
+                mma6(s2[2 * np], ah, am, al, b0a, b1a);
+                mma6(s2[2 * np + 1], ah, am, al, b0b, b1b);
+            } else {
+                mma6(s[2 * np], ah, am, al, b0a, b1a);
+                mma6(s[2 * np + 1], ah, am, al, b0b, b1b);
+            }
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < 2 * NP; ++n) s[n][0] += s2[n][0], s[n][1] += s2[n][1], s[n][2] += s2[n][2], s[n][3] += s2[n][3];
+}
+
+// scaled scores, -inf past the keys that rows g (len0) and g + 8 (len1) see, and the rows' maxima; key0: this lane's first key
+template <int NN>
+__device__ __forceinline__ void mask_scores(float (&s)[NN][4], int key0, int len0, int len1, float scale, float &tm0, float &tm1)
+{
+    tm0 = -INFINITY, tm1 = -INFINITY;
+#pragma unroll
+    for (int n = 0; n < NN; ++n) {
+        const int key = key0 + 8 * n;
+        s[n][0] = key < len0 ? s[n][0] * scale : -INFINITY, s[n][1] = key + 1 < len0 ? s[n][1] * scale : -INFINITY;
+        s[n][2] = key < len1 ? s[n][2] * scale : -INFINITY, s[n][3] = key + 1 < len1 ? s[n][3] * scale : -INFINITY;
+        tm0 = fmaxf(tm0, fmaxf(s[n][0], s[n][1])), tm1 = fmaxf(tm1, fmaxf(s[n][2], s[n][3]));
+    }
+    tm0 = fmaxf(tm0, __shfl_xor_sync(0xffffffffu, tm0, 1)), tm0 = fmaxf(tm0, __shfl_xor_sync(0xffffffffu, tm0, 2));
+    tm1 = fmaxf(tm1, __shfl_xor_sync(0xffffffffu, tm1, 1)), tm1 = fmaxf(tm1, __shfl_xor_sync(0xffffffffu, tm1, 2));
+}
+
+// P = exp(s - new maximum) as split A operands, the correction exp(old - new maximum) and the tile's row sums
+__device__ __forceinline__ void weights_of_tile(const float (&s)[KT / 8][4], float m0, float m1, float nm0, float nm1, float &c0, float &c1, float &ps0,
+                                                float &ps1, uint32_t (&ph)[KT / 16][4], uint32_t (&pm)[KT / 16][4], uint32_t (&pl)[KT / 16][4])
+{
+    // a row that sees no key of this tile (and none before) keeps m = -inf: its weights and corrections are 0
+    c0 = nm0 > -INFINITY ? expf(m0 - nm0) : 0.f, c1 = nm1 > -INFINITY ? expf(m1 - nm1) : 0.f;
+    ps0 = 0.f, ps1 = 0.f;
+#pragma unroll
+    for (int n = 0; n < KT / 8; ++n) {
+        float p[4];
+        p[0] = nm0 > -INFINITY ? expf(s[n][0] - nm0) : 0.f, p[1] = nm0 > -INFINITY ? expf(s[n][1] - nm0) : 0.f;
+        p[2] = nm1 > -INFINITY ? expf(s[n][2] - nm1) : 0.f, p[3] = nm1 > -INFINITY ? expf(s[n][3] - nm1) : 0.f;
+        ps0 += p[0] + p[1], ps1 += p[2] + p[3];
+        __nv_bfloat16 hi[4], mi[4], lo[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) split3(p[i], hi[i], mi[i], lo[i]);
+        // accumulator (row g: cols 2tg, 2tg+1 | row g+8) of key tile n -> A regs: tile 2j -> a0 (row g), a1 (row g+8); tile 2j+1 -> a2, a3
+        const int j = n >> 1, o2 = (n & 1) * 2;
+        ph[j][o2] = pack2(hi[0], hi[1]), ph[j][o2 + 1] = pack2(hi[2], hi[3]);
+        pm[j][o2] = pack2(mi[0], mi[1]), pm[j][o2 + 1] = pack2(mi[2], mi[3]);
+        pl[j][o2] = pack2(lo[0], lo[1]), pl[j][o2 + 1] = pack2(lo[2], lo[3]);
+    }
+    ps0 += __shfl_xor_sync(0xffffffffu, ps0, 1), ps0 += __shfl_xor_sync(0xffffffffu, ps0, 2);
+    ps1 += __shfl_xor_sync(0xffffffffu, ps1, 1), ps1 += __shfl_xor_sync(0xffffffffu, ps1, 2);
+}
+
 // Shared memory (bf16 planes, plane p of a tile at p * rows * LDB bytes): Q [3][HPC * 64][LD], K [3][32][LD], V [3][32][LD]
 // Q8: the cache holds Q8_0 rows as int8 planes kc / vc [.., maxSeq, HD] with fp16 block scales kd / vd [.., maxSeq, HD / 32]
 // (QuantizedKVCache); a staged value is d * q, a 19-bit number that its three bf16 parts hold exactly, so the contraction
@@ -162,66 +247,15 @@ __global__ void __launch_bounds__(128 * HPC) sdpa_prefill_mma_kernel(const float
         if (start >= warp_len) continue;  // warp uniform: every row's causal bound lies before the tile
 
         // ---- S = Q K^T for 16 rows x 32 keys
-        float s[KT / 8][4], s2[KT / 8][4];  // even and odd k-steps: two independent chains of dependent MMAs per key tile
-#pragma unroll
-        for (int n = 0; n < KT / 8; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = s2[n][0] = s2[n][1] = s2[n][2] = s2[n][3] = 0.f;
-#pragma unroll
-        for (int ks = 0; ks < HD / 16; ++ks) {
-            uint32_t ah[4], am[4], al[4];
-            ldsm4(sq_a + a_off + 32 * ks, ah);
-            ldsm4(sq_a + QPLANE + a_off + 32 * ks, am);
-            ldsm4(sq_a + 2 * QPLANE + a_off + 32 * ks, al);
-#pragma unroll
-            for (int np = 0; np < KT / 16; ++np) {  // two key tiles per ldmatrix
-                uint32_t b[3][4];
-#pragma unroll
-                for (int pl = 0; pl < 3; ++pl) ldsm4(sk_a + pl * KPLANE + bk_off + np * 16 * LDB + 32 * ks, b[pl]);
-                const uint32_t b0a[3] = {b[0][0], b[1][0], b[2][0]}, b1a[3] = {b[0][1], b[1][1], b[2][1]};
-                const uint32_t b0b[3] = {b[0][2], b[1][2], b[2][2]}, b1b[3] = {b[0][3], b[1][3], b[2][3]};
-                if (ks & 1) {
-                    mma6(s2[2 * np], ah, am, al, b0a, b1a);
-                    mma6(s2[2 * np + 1], ah, am, al, b0b, b1b);
-                } else {
-                    mma6(s[2 * np], ah, am, al, b0a, b1a);
-                    mma6(s[2 * np + 1], ah, am, al, b0b, b1b);
-                }
-            }
-        }
-#pragma unroll
-        for (int n = 0; n < KT / 8; ++n) s[n][0] += s2[n][0], s[n][1] += s2[n][1], s[n][2] += s2[n][2], s[n][3] += s2[n][3];
+        float s[KT / 8][4];
+        scores_of_tile<HD, KT / 16>(sq_a + a_off, QPLANE, sk_a + bk_off, KPLANE, s);
         // ---- online softmax: lane holds keys start + 8n + 2tg, + 1 of rows g (s[n][0..1]) and g + 8 (s[n][2..3])
-        float tm0 = -INFINITY, tm1 = -INFINITY;
-#pragma unroll
-        for (int n = 0; n < KT / 8; ++n) {
-            const int key = start + 8 * n + 2 * tg;
-            s[n][0] = key < len0 ? s[n][0] * scale : -INFINITY, s[n][1] = key + 1 < len0 ? s[n][1] * scale : -INFINITY;
-            s[n][2] = key < len1 ? s[n][2] * scale : -INFINITY, s[n][3] = key + 1 < len1 ? s[n][3] * scale : -INFINITY;
-            tm0 = fmaxf(tm0, fmaxf(s[n][0], s[n][1])), tm1 = fmaxf(tm1, fmaxf(s[n][2], s[n][3]));
-        }
-        tm0 = fmaxf(tm0, __shfl_xor_sync(0xffffffffu, tm0, 1)), tm0 = fmaxf(tm0, __shfl_xor_sync(0xffffffffu, tm0, 2));
-        tm1 = fmaxf(tm1, __shfl_xor_sync(0xffffffffu, tm1, 1)), tm1 = fmaxf(tm1, __shfl_xor_sync(0xffffffffu, tm1, 2));
+        float tm0, tm1;
+        mask_scores<KT / 8>(s, start + 2 * tg, len0, len1, scale, tm0, tm1);
         const float nm0 = fmaxf(m0, tm0), nm1 = fmaxf(m1, tm1);
-        // a row that sees no key of this tile (and none before) keeps m = -inf: its weights and corrections are 0
-        const float c0 = nm0 > -INFINITY ? expf(m0 - nm0) : 0.f, c1 = nm1 > -INFINITY ? expf(m1 - nm1) : 0.f;
-        float ps0 = 0.f, ps1 = 0.f;
+        float c0, c1, ps0, ps1;
         uint32_t ph[KT / 16][4], pm[KT / 16][4], pl_[KT / 16][4];  // P as A operands: k16 = two key tiles
-#pragma unroll
-        for (int n = 0; n < KT / 8; ++n) {
-            float p[4];
-            p[0] = nm0 > -INFINITY ? expf(s[n][0] - nm0) : 0.f, p[1] = nm0 > -INFINITY ? expf(s[n][1] - nm0) : 0.f;
-            p[2] = nm1 > -INFINITY ? expf(s[n][2] - nm1) : 0.f, p[3] = nm1 > -INFINITY ? expf(s[n][3] - nm1) : 0.f;
-            ps0 += p[0] + p[1], ps1 += p[2] + p[3];
-            __nv_bfloat16 hi[4], mi[4], lo[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) split3(p[i], hi[i], mi[i], lo[i]);
-            // accumulator (row g: cols 2tg, 2tg+1 | row g+8) of key tile n -> A regs: tile 2j -> a0 (row g), a1 (row g+8); tile 2j+1 -> a2, a3
-            const int j = n >> 1, o2 = (n & 1) * 2;
-            ph[j][o2] = pack2(hi[0], hi[1]), ph[j][o2 + 1] = pack2(hi[2], hi[3]);
-            pm[j][o2] = pack2(mi[0], mi[1]), pm[j][o2 + 1] = pack2(mi[2], mi[3]);
-            pl_[j][o2] = pack2(lo[0], lo[1]), pl_[j][o2 + 1] = pack2(lo[2], lo[3]);
-        }
-        ps0 += __shfl_xor_sync(0xffffffffu, ps0, 1), ps0 += __shfl_xor_sync(0xffffffffu, ps0, 2);
-        ps1 += __shfl_xor_sync(0xffffffffu, ps1, 1), ps1 += __shfl_xor_sync(0xffffffffu, ps1, 2);
+        weights_of_tile(s, m0, m1, nm0, nm1, c0, c1, ps0, ps1, ph, pm, pl_);
         l0 = fmaf(l0, c0, ps0), l1 = fmaf(l1, c1, ps1);
         m0 = nm0, m1 = nm1;
 #pragma unroll
@@ -250,6 +284,225 @@ __global__ void __launch_bounds__(128 * HPC) sdpa_prefill_mma_kernel(const float
     }
 }
 
+// ------------------------------------------------------------------------------ few rows over a long cache
+// Up to 16 query rows (a draft's tokens) over an fp32 cache: the kernel above gives every head pair one CTA, whose two busy
+// warps walk the cache's tiles one after the other (5 us a tile: 384 dependent MMAs, exponentials, staging).  Here a cluster of
+// HD / 16 CTAs shares one head pair and eight rows, and cuts that walk by what its steps depend on, so that every sum is still
+// formed by the same MMAs in the same order and every output keeps its bits:
+//   1. scores and tile maxima: tiles are independent; CTA r takes tiles r, r + CS, ..., a warp per head and half tile
+//   2. with all tile maxima known (they go to every CTA of the cluster) the running maximum before and after a tile is a
+//      maximum over earlier tiles: weights, corrections and row sums of all tiles at once
+//   3. only O += P V and l follow the tiles in order; CTA r does it for its 16 output dims (a warp per head), reading the
+//      weights from the CTA that made them through distributed shared memory, while the other warps stage V
+// Shared memory stays below half an SM's: with one CTA per SM fewer than 16 clusters of eight were resident at once, and the
+// 16 head pairs of a 32-head model took two waves.  What bounds it: step 1's MMAs and step 3's chain of 12 MMAs per tile.
+// Six rows over 1021 keys, 32 heads on 8 KV heads of 128, one layer: 175 us in the kernel above,
+// 41 us here; the whole 32-layer pass 8.59 -> 4.32 ms.
+constexpr int FEW_ROWS = 8;  // per cluster: rows 8 .. 15 of the MMAs are not used
+template <int HD>
+struct FewShape {
+    static constexpr int CS = HD / 16, LDB = HD * 2 + 16;
+    static constexpr int LOCAL = 14, TILES = LOCAL * CS;  // key tiles of one CTA, and in all
+    static constexpr int QPLANE = 2 * FEW_ROWS * LDB, KPLANE = 2 * KT * LDB, S_JOB = 1024, P_JOB = 3 * 512;
+    static constexpr int V_LD = 48, V_TILES = 5, V_KEYS = V_TILES * KT, VPLANE = V_KEYS * V_LD;  // 16 dims of a key: 32 bytes, padded to an odd multiple of 16
+    // Q and K, then scores; later weights where Q and K were, then two stages of V over the rest and the scores
+    static constexpr int QK = 3 * (QPLANE + KPLANE) > 2 * LOCAL * P_JOB ? 3 * (QPLANE + KPLANE) : 2 * LOCAL * P_JOB;
+    static constexpr int OFF_K = 3 * QPLANE, OFF_S = QK, OFF_P = 0, OFF_V = 2 * LOCAL * P_JOB;
+    static constexpr int END = OFF_S + 2 * LOCAL * S_JOB > OFF_V + 2 * 3 * VPLANE ? OFF_S + 2 * LOCAL * S_JOB : OFF_V + 2 * 3 * VPLANE;
+    static constexpr int OFF_TM = END, OFF_CP = OFF_TM + 2 * 2 * TILES * FEW_ROWS * 4, SMEM = OFF_CP + 2 * LOCAL * FEW_ROWS * 8;
+    static_assert(SMEM <= 113 * 1024, "two CTAs per SM");
+};
+__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t cta)
+{
+    uint32_t v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(v) : "r"(addr), "r"(cta));
+    return v;
+}
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int HD>
+__global__ void __launch_bounds__(256, 2) sdpa_few_rows_kernel(const float *__restrict__ q, const float *__restrict__ kc, const float *__restrict__ vc,
+                                                               float *__restrict__ out, int T, int nh, int nkv, int pos0, int maxSeq, float scale)
+{
+    using S = FewShape<HD>;
+    constexpr int LDB = S::LDB, CS = S::CS;
+    extern __shared__ __align__(16) uint8_t sm_raw[];
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm_raw);
+    float2 *sc = reinterpret_cast<float2 *>(sm_raw + S::OFF_S);              // scores of row g [job][4][lane]
+    uint4 *sp = reinterpret_cast<uint4 *>(sm_raw + S::OFF_P);                // weights of row g [job][plane][lane]
+    const float *tmx = reinterpret_cast<const float *>(sm_raw + S::OFF_TM);  // maxima [head][half tile][row]
+    float2 *cp = reinterpret_cast<float2 *>(sm_raw + S::OFF_CP);             // (correction, row sum) [job][row]
+    smc_grid_dep_sync();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tg = lane & 3;
+    const int hg = blockIdx.x / CS, rank = blockIdx.x % CS, kvh = hg * 2 / (nh / nkv), t0 = (int)blockIdx.y * FEW_ROWS;
+    const int len = pos0 + T, tiles = (len + KT - 1) / KT, local = tiles > rank ? (tiles - rank + CS - 1) / CS : 0;
+    const float *kbase = kc + (size_t)kvh * maxSeq * HD, *vbase = vc + (size_t)kvh * maxSeq * HD;
+
+    constexpr int PF = 2 * KT * (HD / 4) / 256;  // K: two tiles at a time, requested before the previous two are multiplied
+    float4 pk[PF];
+    auto fetch_k = [&](int lt0) {
+#pragma unroll
+        for (int i = 0; i < PF; ++i) {
+            const int e = threadIdx.x + i * 256, r = e / (HD / 4), c = e % (HD / 4);
+            const int key = ((lt0 + r / KT) * CS + rank) * KT + r % KT;
+            pk[i] = key < len ? *reinterpret_cast<const float4 *>(kbase + (size_t)key * HD + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    fetch_k(0);
+    for (int e = threadIdx.x; e < 2 * FEW_ROWS * (HD / 4); e += 256) {  // Q: split once
+        const int c = e % (HD / 4), r = (e / (HD / 4)) % FEW_ROWS, hh = e / (FEW_ROWS * (HD / 4));
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t0 + r < T) v = *reinterpret_cast<const float4 *>(q + ((size_t)(t0 + r) * nh + hg * 2 + hh) * HD + 4 * c);
+        split_store(v, sm_raw + (hh * FEW_ROWS + r) * LDB + 8 * c, S::QPLANE);
+    }
+    cluster_sync();  // every CTA of the cluster runs: its shared memory may be written
+    const int len0 = t0 + g < T ? pos0 + t0 + g + 1 : 0;  // keys that row g sees
+
+    // ---- 1: scores of this CTA's tiles, two at a time
+    {
+        const int hl = warp >> 2, tl = (warp >> 1) & 1, np = warp & 1;
+        // rows 8 .. 15 of the A operand come from the same addresses as rows 0 .. 7: what they yield is not used
+        const uint32_t qa = base + (uint32_t)((hl * FEW_ROWS + (lane & 7)) * LDB + 16 * (lane >> 4));
+        const uint32_t ka = base + S::OFF_K + (uint32_t)((tl * KT + np * 16 + (lane & 7) + 8 * (lane >> 4)) * LDB + 16 * ((lane >> 3) & 1));
+        for (int lt0 = 0; lt0 < local; lt0 += 2) {
+            __syncthreads();  // the previous two tiles have been read
+#pragma unroll
+            for (int i = 0; i < PF; ++i) {
+                const int e = threadIdx.x + i * 256, r = e / (HD / 4), c = e % (HD / 4);
+                split_store(pk[i], sm_raw + S::OFF_K + r * LDB + 8 * c, S::KPLANE);
+            }
+            __syncthreads();
+            if (lt0 + 2 < local) fetch_k(lt0 + 2);
+            const int lt = lt0 + tl, tile = lt * CS + rank;
+            if (lt >= local) continue;  // warp uniform
+            float s[2][4];
+            scores_of_tile<HD, 1>(qa, S::QPLANE, ka, S::KPLANE, s);
+            float tm0, tm1;
+            mask_scores<2>(s, tile * KT + np * 16 + 2 * tg, len0, 0, scale, tm0, tm1);
+            const int job = hl * S::LOCAL + lt;
+#pragma unroll
+            for (int n = 0; n < 2; ++n) sc[(job * 4 + 2 * np + n) * 32 + lane] = make_float2(s[n][0], s[n][1]);
+            const uint32_t at = base + S::OFF_TM + 4u * (uint32_t)((hl * 2 * S::TILES + 2 * tile + np) * FEW_ROWS + g);
+            for (int cta = tg; cta < CS; cta += 4)
+                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_map(at, (uint32_t)cta)), "f"(tm0) : "memory");
+        }
+    }
+    cluster_sync();
+    // ---- 2: weights, corrections and row sums of this CTA's tiles
+    for (int j = warp; j < 2 * local; j += 8) {
+        const int hl = j & 1, lt = j >> 1, tile = lt * CS + rank, job = hl * S::LOCAL + lt;
+        const float *tmh = tmx + hl * 2 * S::TILES * FEW_ROWS + g;
+        float m0 = -INFINITY;
+        for (int t = tg; t < 2 * tile; t += 4) m0 = fmaxf(m0, tmh[t * FEW_ROWS]);
+        m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, 1)), m0 = fmaxf(m0, __shfl_xor_sync(0xffffffffu, m0, 2));
+        const float nm0 = fmaxf(m0, fmaxf(tmh[2 * tile * FEW_ROWS], tmh[(2 * tile + 1) * FEW_ROWS]));
+        float s[KT / 8][4];
+#pragma unroll
+        for (int n = 0; n < KT / 8; ++n) {
+            const float2 v = sc[(job * 4 + n) * 32 + lane];
+            s[n][0] = v.x, s[n][1] = v.y, s[n][2] = s[n][3] = -INFINITY;
+        }
+        float c0, c1, ps0, ps1;
+        uint32_t ph[KT / 16][4], pm[KT / 16][4], pl[KT / 16][4];
+        weights_of_tile(s, m0, -INFINITY, nm0, -INFINITY, c0, c1, ps0, ps1, ph, pm, pl);
+        uint4 *dst = sp + job * 3 * 32 + lane;
+        dst[0] = make_uint4(ph[0][0], ph[0][2], ph[1][0], ph[1][2]);
+        dst[32] = make_uint4(pm[0][0], pm[0][2], pm[1][0], pm[1][2]);
+        dst[64] = make_uint4(pl[0][0], pl[0][2], pl[1][0], pl[1][2]);
+        if (tg == 0) cp[job * FEW_ROWS + g] = make_float2(c0, ps0);
+    }
+    cluster_sync();  // and nobody needs its scores any more: V goes there
+    // ---- 3: O and l in tile order, 16 dims per CTA
+    auto stage_v = [&](int chunk, int t, int threads) {  // V_KEYS keys x 16 dims
+        uint8_t *dst = sm_raw + S::OFF_V + (chunk & 1) * 3 * S::VPLANE;
+        for (int e0 = t; e0 < S::V_KEYS * 4; e0 += 4 * threads) {
+            float4 v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int e = e0 + i * threads, key = chunk * S::V_KEYS + e / 4;
+                v[i] = e < S::V_KEYS * 4 && key < len ? *reinterpret_cast<const float4 *>(vbase + (size_t)key * HD + rank * 16 + 4 * (e & 3))
+                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int e = e0 + i * threads;
+                if (e < S::V_KEYS * 4) split_store(v[i], dst + (e / 4) * S::V_LD + 8 * (e & 3), S::VPLANE);
+            }
+        }
+    };
+    stage_v(0, threadIdx.x, 256);
+    const int chunks = (tiles + S::V_TILES - 1) / S::V_TILES;
+    if (warp >= 2) {
+        for (int chunk = 0; chunk < chunks; ++chunk) {
+            __syncthreads();  // this chunk is staged and the other buffer has been read
+            if (chunk + 1 < chunks) stage_v(chunk + 1, threadIdx.x - 64, 192);
+        }
+    } else {
+        const int hl = warp;
+        constexpr int AHEAD = 4;  // tiles whose weights are on their way
+        uint4 wp[AHEAD][3];
+        float2 wr[AHEAD];
+        auto fetch = [&](int tile, int u) {
+            const uint32_t job = (uint32_t)(hl * S::LOCAL + tile / CS);
+            const uint32_t at = cluster_map(base + S::OFF_P, (uint32_t)(tile % CS)) + job * S::P_JOB + 16u * (uint32_t)lane;
+            const uint32_t ac = cluster_map(base + S::OFF_CP, (uint32_t)(tile % CS)) + 8u * (job * FEW_ROWS + (uint32_t)g);
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+                asm volatile("ld.shared::cluster.v4.u32 {%0,%1,%2,%3}, [%4];"
+                             : "=r"(wp[u][i].x), "=r"(wp[u][i].y), "=r"(wp[u][i].z), "=r"(wp[u][i].w)
+                             : "r"(at + 512u * i)
+                             : "memory");
+            asm volatile("ld.shared::cluster.v2.f32 {%0,%1}, [%2];" : "=f"(wr[u].x), "=f"(wr[u].y) : "r"(ac) : "memory");
+        };
+#pragma unroll
+        for (int u = 0; u < AHEAD; ++u)
+            if (u < tiles) fetch(u, u);
+        float o[2][4], l0 = 0.f;
+#pragma unroll
+        for (int n = 0; n < 2; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
+        const uint32_t va = base + S::OFF_V + (uint32_t)(((lane & 7) + 8 * ((lane >> 3) & 1)) * S::V_LD + 16 * (lane >> 4));
+        int in_chunk = 0, chunk = 0;
+        for (int tile0 = 0; tile0 < tiles; tile0 += AHEAD) {
+#pragma unroll
+            for (int u = 0; u < AHEAD; ++u) {
+                const int tile = tile0 + u;
+                if (tile >= tiles) break;
+                if (in_chunk == 0) __syncthreads();  // the chunk is staged
+                const uint32_t vt = va + (uint32_t)((chunk & 1) * 3 * S::VPLANE + in_chunk * KT * S::V_LD);
+                if (++in_chunk == S::V_TILES) in_chunk = 0, ++chunk;
+                const float c0 = wr[u].x;
+                l0 = fmaf(l0, c0, wr[u].y);
+                const uint4 w[3] = {wp[u][0], wp[u][1], wp[u][2]};
+                if (tile + AHEAD < tiles) fetch(tile + AHEAD, u);
+#pragma unroll
+                for (int n = 0; n < 2; ++n) o[n][0] *= c0, o[n][1] *= c0;
+#pragma unroll
+                for (int j = 0; j < KT / 16; ++j) {
+                    uint32_t b[3][4];
+#pragma unroll
+                    for (int pl = 0; pl < 3; ++pl) ldsm4t(vt + (uint32_t)(pl * S::VPLANE + j * 16 * S::V_LD), b[pl]);
+                    const uint32_t ph[4] = {j ? w[0].z : w[0].x, 0u, j ? w[0].w : w[0].y, 0u}, pm[4] = {j ? w[1].z : w[1].x, 0u, j ? w[1].w : w[1].y, 0u},
+                                   pl[4] = {j ? w[2].z : w[2].x, 0u, j ? w[2].w : w[2].y, 0u};
+                    const uint32_t b0a[3] = {b[0][0], b[1][0], b[2][0]}, b1a[3] = {b[0][1], b[1][1], b[2][1]};
+                    const uint32_t b0b[3] = {b[0][2], b[1][2], b[2][2]}, b1b[3] = {b[0][3], b[1][3], b[2][3]};
+                    mma6(o[0], ph, pm, pl, b0a, b1a);
+                    mma6(o[1], ph, pm, pl, b0b, b1b);
+                }
+            }
+        }
+        const float i0 = l0 > 0.f ? 1.0f / l0 : 0.f;
+        if (t0 + g < T) {
+            float *dst = out + ((size_t)(t0 + g) * nh + hg * 2 + hl) * HD + rank * 16 + 2 * tg;
+            *reinterpret_cast<float2 *>(dst) = make_float2(o[0][0] * i0, o[0][1] * i0);
+            *reinterpret_cast<float2 *>(dst + 8) = make_float2(o[1][0] * i0, o[1][1] * i0);
+        }
+    }
+    cluster_sync();  // nobody leaves while its weights are read
+}
+
 }  // namespace
 
 bool smc_sdpa_prefill_mma_supported(int nh, int nkv, int hd) { return (hd == 64 || hd == 128) && nkv > 0 && nh % nkv == 0; }
@@ -267,6 +520,19 @@ static int launch_prefill_mma(smc_ctx *ctx, const float *q, const void *kc, cons
         smc_launch_dep(ctx->use_pdl, kernel, grid, dim3(128 * hpc), smem, s, q, kc, vc, kd, vd, out, T, nh, nkv, pos0, maxSeq, scale);
     };
     const bool two = G % 2 == 0 && ctx->attn_hpc != 1;
+    // a few rows over more than a few tiles of an fp32 cache: the same bits from a cluster per head pair and eight rows
+    const int tiles = (pos0 + T + KT - 1) / KT;
+    if (two && !kd && T <= 2 * FEW_ROWS && tiles >= 4 && tiles <= (hd == 128 ? FewShape<128>::TILES : FewShape<64>::TILES)) {
+        auto few = [&](auto kernel, int cs, size_t smem) {
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            smc_launch_dep_cluster(ctx->use_pdl, cs, kernel, dim3(nh / 2 * cs, (T + FEW_ROWS - 1) / FEW_ROWS), dim3(256), smem, s, q,
+                                   static_cast<const float *>(kc), static_cast<const float *>(vc), out, T, nh, nkv, pos0, maxSeq, scale);
+        };
+        if (hd == 128) few(sdpa_few_rows_kernel<128>, FewShape<128>::CS, FewShape<128>::SMEM);
+        else few(sdpa_few_rows_kernel<64>, FewShape<64>::CS, FewShape<64>::SMEM);
+        SMC_LAUNCH_CHECK(ctx);
+        return SMC_OK;
+    }
     if (kd) {
         if (hd == 128) two ? go(sdpa_prefill_mma_kernel<128, 2, true>, 2) : go(sdpa_prefill_mma_kernel<128, 1, true>, 1);
         else two ? go(sdpa_prefill_mma_kernel<64, 2, true>, 2) : go(sdpa_prefill_mma_kernel<64, 1, true>, 1);

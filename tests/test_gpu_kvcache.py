@@ -214,3 +214,35 @@ def test_prompt_attention_on_tensor_cores_over_a_q8_0_cache(oracle, cuda, hd, he
         assert np.array_equal(old.view(np.uint32), got.view(np.uint32)) == (s < 16)  # which kernel ran
     kv.Dispose()
     assert cuda.device_status() == 0
+
+
+@pytest.mark.parametrize("hd,heads,kvh,most", [(128, 32, 8, 3584), (128, 4, 2, 3584), (64, 8, 4, 1792)])
+@pytest.mark.parametrize("rows,length", [(2, 97), (2, 98), (6, 128), (8, 129), (9, 257), (16, 1027), (5, 1700), (3, -1), (3, 0), (3, 1)])
+def test_few_rows_over_a_long_cache(cuda, hd, heads, kvh, most, rows, length):
+    """A draft's rows over an fp32 cache run on a cluster of CTAs per head pair: the same bits as the one-CTA walk (here reached
+    by padding the same queries to 17 rows: a row's sums do not depend on the rows behind it), around the key tiles, with CTAs
+    that get no tile, at the largest cache the cluster holds and past it (length counted from there when below 2).  Also against
+    float64: an output is a convex combination of value rows whose weights are off by the scores' absolute error, a few
+    roundings (2^-24) of the largest |q| |k| scale."""
+    import torch
+
+    length = length if length > 1 else most + length
+    g = torch.Generator(device="cuda").manual_seed(rows * 7919 + length)
+    pad = 17 - rows  # later positions, seen by the padding rows alone
+    k, v = (torch.randn((1, length + pad, kvh, hd), generator=g, device="cuda") for _ in range(2))
+    q = torch.randn((1, 17, heads, hd), generator=g, device="cuda")
+    scale = hd ** -0.5
+    kv = ops.KVCache(cuda, 1, kvh, length + pad, hd, ops.KVCache.F32)
+    kv.Update(k, v)
+    want = kv.attention(q, scale)[0, :rows]
+    kv.Truncate(length)
+    got = kv.attention(q[:, :rows].contiguous(), scale)[0]
+    assert torch.equal(got.view(torch.int32), want.view(torch.int32)), int((got != want).sum())
+    kd, vd = (t[0, :length].double().repeat_interleave(heads // kvh, 1).permute(1, 0, 2) for t in (k, v))
+    s = q[0, :rows].double().permute(1, 0, 2) @ kd.transpose(1, 2) * scale
+    pos = length - rows + torch.arange(rows, device="cuda")
+    s = s.masked_fill(torch.arange(length, device="cuda")[None] > pos[:, None], -torch.inf)
+    exact = (torch.softmax(s, -1) @ vd).permute(1, 0, 2)
+    reach = float(q.norm(dim=-1).max() * k.norm(dim=-1).max()) * scale
+    assert (got.double() - exact).abs().max() <= 4 * 2.0 ** -24 * reach * v.abs().max()
+    kv.Dispose()
