@@ -535,6 +535,9 @@ static int qmatmul_impl(smc_ctx *ctx, const float *d_in, const smc_weight *w, fl
         // prefill-sized batches of Q4_K run on the tcgen05 tensor cores (same parity bound, see smc_prefill.cu)
         if (M >= 64 && smc_prefill_supported(w, M) && (reinterpret_cast<uintptr_t>(d_in) & 15) == 0)
             return smc_launch_prefill_q4k(ctx, d_in, w, d_out, M, s);
+        // Q6_K too, where the digit planes are on (the option that selects the CUDA-core kernel instead also covers this one)
+        if (ctx->f32_digits && smc_prefill_q6k_supported(ctx, w, M) && M >= ctx->f32_digits && (reinterpret_cast<uintptr_t>(d_in) & 15) == 0)
+            return smc_launch_prefill_q6k(ctx, d_in, w, d_out, M, s);
         if (ctx->f32_digits && M >= (ctx->f32_digits > 1 ? ctx->f32_digits : 2) && w->fast && (reinterpret_cast<uintptr_t>(d_in) & 15) == 0)
             return qmatmul_f32_digits(ctx, d_in, w, d_out, M, s);
         // one row over a large matrix: its three digit rows through the several-row integer kernel beat the fp32 one-row kernel

@@ -155,6 +155,8 @@ int smc_launch_gemv_tma_gather(smc_ctx *, const float *x, const smc_weight *, fl
                                cudaStream_t s);
 int smc_qmatmul_dev_gather(smc_ctx *, const float *d_in, const smc_weight *, float *d_out, int M, int mode, cudaStream_t s,
                            const smc_gather_dev *, bool *fused);
+bool smc_prefill_q6k_supported(const smc_ctx *, const smc_weight *, int M);
+int smc_launch_prefill_q6k(smc_ctx *, const float *x, const smc_weight *, float *out, int M, cudaStream_t s);
 bool smc_prefill_supported(const smc_weight *, int M);
 int smc_launch_prefill_q4k(smc_ctx *, const float *x, const smc_weight *, float *out, int M, cudaStream_t s);
 int smc_launch_prefill_q4k_q8(smc_ctx *, const smc_q8act *a, const smc_weight *, float *out, cudaStream_t s, bool scratch_locked = false);

@@ -254,6 +254,7 @@ __global__ void __launch_bounds__(256) prefill_image_kernel(const float *__restr
                             (size_t)(c & 7) * 64 + (size_t)(tl & 7) * 8;
         *reinterpret_cast<uint4 *>(img + base) = *reinterpret_cast<const uint4 *>(hi);
         *reinterpret_cast<uint4 *>(img + base + TN * KS) = *reinterpret_cast<const uint4 *>(lo);
+        if (!mimg) continue;  // Q6_K has no min term
         // sub-block sums: chunks 4j .. 4j+3 are adjacent lanes
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);
         sum += __shfl_xor_sync(0xffffffffu, sum, 2);
@@ -526,6 +527,241 @@ prefill_q4k_kernel(const uint8_t *__restrict__ raw, const __half *__restrict__ i
     }
 }
 
+// ------------------------------------------------------------------------------ Q6_K
+// The same contraction over Q6_K:  w[r, k] = d_b * v,  v = sc_j * (q_k - 32)  with sc_j an int8 per 16 elements, |v| <= 4096.
+// Not every v is an fp16 (odd ones above 2048 are not), so the weights travel as an exact pair v = v_hi + v_lo, v_hi the
+// rounded product and v_lo in {-1, 0, 1}; the dropped v_lo x_lo is below 2^-22 of a product and rare:
+//   acc_d[r, t] = sum_{k in g} v_lo x_hi + v_hi x_lo + v_hi x_hi     12 MMAs of K = 16 per quarter g of a block, smallest first
+//   out[t, r]   = s_t * sum_b d_b * sum_{g in b} acc_d(g)
+// The tensor cores cut their sums off instead of rounding them: with one accumulator for a whole block (16 MMAs at full size in
+// one chain) the result was five times further from 64 bits than the kernels this one replaces; quarters put that right.
+// Warp roles as above; tensor memory holds two accumulators and four A stages of {hi, lo} (no min term).  A block's bytes lie in
+// five places of its unit, so they come by 16-byte asynchronous copies: a warp of the first four (plane 0) fetches the rows of its
+// quarter for both warps of the quarter and the pair meets at a named barrier; plane 0 unpacks the first 32 elements of each
+// stage, plane 1 the second 32.
+// What bounds it: the tensor cores, three MMAs per product, and the activation stages' way into the SM.  Before, fp32 rows went through
+// mma.sync as three int8 digit planes, one scaling on the CUDA cores per output, plane and 16 elements.
+// 4096 x 14336 with 500 rows: 1595 -> 346 us (169 useful TFLOP/s); distance from 64 bits 1.84e-7 -> 1.54e-7, 8192 x 28672
+// 2.26e-7 -> 1.69e-7, 1024 x 4096 1.50e-7 -> 1.42e-7.
+constexpr int Q6_RAW = 240;                        // bytes of a row and block in shared memory: X, Y, Z (64 each), 16 scales, padding to an odd multiple of 16
+constexpr int Q6_NW = 3;                           // blocks in flight
+constexpr uint32_t Q6_W_BYTES = TM * Q6_RAW;
+constexpr uint32_t Q6_OFF_W = NB * SLOT_BYTES, Q6_OFF_BAR = Q6_OFF_W + Q6_NW * Q6_W_BYTES, Q6_SMEM = Q6_OFF_BAR + 256;
+static_assert(Q6_SMEM <= 227 * 1024, "shared memory budget");
+constexpr uint32_t Q6_COL_A = 256;                 // NA x 64 columns: 32 of v_hi, 32 of v_lo
+enum { Q6_FULL_B = 0, Q6_EMPTY_B = Q6_FULL_B + NB, Q6_FULL_A = Q6_EMPTY_B + NB, Q6_EMPTY_A = Q6_FULL_A + NA, Q6_ACC_FULL = Q6_EMPTY_A + NA,
+       Q6_ACC_EMPTY = Q6_ACC_FULL + 2, Q6_BARS = Q6_ACC_EMPTY + 2 };
+static_assert(Q6_BARS * 8 + 8 <= 256, "barrier area");
+
+// four codes 0..63 in the bytes of `q` -> two fp16 pairs each of v_hi and v_lo
+__device__ __forceinline__ void expand_q6(uint32_t q, __half2 sc, uint32_t (&hi)[2], uint32_t (&lo)[2])
+{
+    const __half2 off = __half2half2(__ushort_as_half((unsigned short)0xE420u));  // -1056: takes 1024 + 32 off
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const uint32_t p = __byte_perm(q, 0x64646464u, i ? 0x4342u : 0x4140u);
+        const __half2 c = __hadd2(*reinterpret_cast<const __half2 *>(&p), off);
+        const __half2 h = __hmul2(c, sc), l = __hfma2(c, sc, __hneg2(h));  // the remainder of an fp16 product is exact
+        hi[i] = *reinterpret_cast<const uint32_t *>(&h), lo[i] = *reinterpret_cast<const uint32_t *>(&l);
+    }
+}
+
+__global__ void __launch_bounds__(THREADS, 1)
+prefill_q6k_kernel(const uint8_t *__restrict__ q6u, const __half *__restrict__ img, const float *__restrict__ scale, float *__restrict__ out, int N, int K,
+                   int M, int ntt, int *status)
+{
+    extern __shared__ __align__(1024) uint8_t smem[];
+    const uint32_t sbase = smem_u32(smem);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rt = blockIdx.x / ntt, tt = blockIdx.x % ntt, row0 = rt * TM, nsb = K / 256;
+    volatile uint32_t *abort_flag = reinterpret_cast<volatile uint32_t *>(smem + Q6_OFF_BAR + Q6_BARS * 8 + 4);
+    auto bar = [&](int i) { return sbase + Q6_OFF_BAR + 8u * (uint32_t)i; };
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < NB; ++i) mbar_init(bar(Q6_FULL_B + i), 1), mbar_init(bar(Q6_EMPTY_B + i), 1);
+        for (int i = 0; i < NA; ++i) mbar_init(bar(Q6_FULL_A + i), EXPAND_WARPS), mbar_init(bar(Q6_EMPTY_A + i), 1);
+        for (int i = 0; i < 2; ++i) mbar_init(bar(Q6_ACC_FULL + i), 1), mbar_init(bar(Q6_ACC_EMPTY + i), DRAIN_WARPS);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_proxy_async();
+    }
+    if (warp == 0) {
+        const uint32_t dst = sbase + Q6_OFF_BAR + Q6_BARS * 8;
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(smem + Q6_OFF_BAR + Q6_BARS * 8);
+
+    if (warp == 0) {
+        if (lane == 0) {
+            const __half *src = img + (size_t)tt * (K / KS) * 2 * (TN * KS);
+            int slot = 0;
+            uint32_t phase = 1;
+            for (int st = 0; st < nsb * NA; ++st) {
+                mbar_wait(bar(Q6_EMPTY_B + slot), phase, abort_flag, status);
+                mbar_expect_tx(bar(Q6_FULL_B + slot), 2 * B_BYTES);
+                bulk_g2s(sbase + (uint32_t)slot * SLOT_BYTES, src + (size_t)st * 2 * (TN * KS), 2 * B_BYTES, bar(Q6_FULL_B + slot));
+                if (++slot == NB) slot = 0, phase ^= 1;
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint64_t b_desc0 = smem_desc(sbase, 128, 1024);
+            constexpr uint64_t U_SLOT = SLOT_BYTES >> 4, U_LO = B_BYTES >> 4, U_KK = 256 >> 4;
+            int slot = 0;
+            uint32_t b_phase = 0;
+            for (int sb = 0; sb < nsb; ++sb) {
+#pragma unroll
+                for (int g = 0; g < NA; ++g) {
+                    const int buf = g & 1, use = 2 * sb + (g >> 1);  // which time this accumulator is filled
+                    const uint32_t acc_d = tmem_base + (uint32_t)buf * 128u;
+                    mbar_wait(bar(Q6_ACC_EMPTY + buf), (uint32_t)((use & 1) ^ 1), abort_flag, status);
+                    mbar_wait(bar(Q6_FULL_B + slot), b_phase, abort_flag, status);
+                    mbar_wait(bar(Q6_FULL_A + g), (uint32_t)(sb & 1), abort_flag, status);
+                    tc_fence_after();
+                    const uint64_t bh = b_desc0 + (uint64_t)slot * U_SLOT;
+                    const uint32_t a0 = tmem_base + Q6_COL_A + (uint32_t)g * 64u;
+#pragma unroll
+                    for (int kk = 0; kk < KS / 16; ++kk) tc_mma_f16_ta(acc_d, a0 + 32 + kk * 8, bh + kk * U_KK, IDESC, kk != 0 ? 1u : 0u);
+#pragma unroll
+                    for (int kk = 0; kk < KS / 16; ++kk) tc_mma_f16_ta(acc_d, a0 + kk * 8, bh + U_LO + kk * U_KK, IDESC, 1u);
+#pragma unroll
+                    for (int kk = 0; kk < KS / 16; ++kk) tc_mma_f16_ta(acc_d, a0 + kk * 8, bh + kk * U_KK, IDESC, 1u);
+                    tc_commit(bar(Q6_EMPTY_B + slot));
+                    tc_commit(bar(Q6_EMPTY_A + g));
+                    tc_commit(bar(Q6_ACC_FULL + buf));
+                    if (++slot == NB) slot = 0, b_phase ^= 1;
+                }
+            }
+        }
+    } else if (warp < WARP_DRAIN0) {
+        const int quarter = warp & 3, plane = (warp - WARP_EXPAND0) >> 2, r = quarter * 32 + lane;
+        const uint32_t a_lane = tmem_base + ((uint32_t)(quarter * 32) << 16) + Q6_COL_A + (uint32_t)plane * 16u;
+        const uint32_t w_quarter = sbase + Q6_OFF_W + (uint32_t)(quarter * 32) * Q6_RAW;
+        const uint32_t meet = 1u + (uint32_t)quarter;  // named barrier of the quarter's two warps
+        auto fetch_block = [&](int p) {  // plane 0: 13 pieces of 16 bytes for each of the quarter's 32 rows, neighbouring lanes on one row
+            if (p < nsb) {
+                const uint32_t dst = w_quarter + (uint32_t)(p % Q6_NW) * Q6_W_BYTES;
+#pragma unroll
+                for (int i = 0; i < 13; ++i) {
+                    const int idx = i * 32 + lane, rr = idx / 13, c = idx % 13;
+                    const size_t blk = (size_t)(row0 + quarter * 32 + rr) * nsb + p;
+                    const uint8_t *src = c < 12 ? q6u + smc_q6u_slot(blk, 0, 0) + 512 * (c >> 2) + 16 * (c & 3) : q6u + smc_q6u_scales(blk);
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst + (uint32_t)(rr * Q6_RAW + 16 * c)), "l"(src) : "memory");
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        if (plane == 0)
+            for (int p = 0; p < Q6_NW - 1; ++p) fetch_block(p);
+        for (int sb = 0; sb < nsb; ++sb) {
+            if (plane == 0) asm volatile("cp.async.wait_group %0;" ::"n"(Q6_NW - 2) : "memory");
+            // block sb has landed; and both warps are through with block sb - 1, whose slot is refilled next
+            asm volatile("bar.sync %0, 64;" ::"r"(meet) : "memory");
+            if (plane == 0) fetch_block(sb + Q6_NW - 1);
+            const uint32_t row = w_quarter + (uint32_t)(sb % Q6_NW) * Q6_W_BYTES + (uint32_t)lane * Q6_RAW;
+            const uint4 scw = lds128(row + 192u);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                uint4 X[2], Y[2], Z[2];
+#pragma unroll
+                for (int o = 0; o < 2; ++o)
+                    X[o] = lds128(row + 32u * h + 16u * o), Y[o] = lds128(row + 64u + 32u * h + 16u * o), Z[o] = lds128(row + 128u + 32u * h + 16u * o);
+#pragma unroll
+                for (int g2 = 0; g2 < 2; ++g2) {  // stage 2 h + g2 = columns c = 2 g2 and 2 g2 + 1 of the half: this warp's is 2 g2 + plane
+                    const int g = 2 * h + g2;
+                    uint32_t hi[16], lo[16];
+#pragma unroll
+                    for (int o = 0; o < 2; ++o) {
+                        const uint32_t xw[4] = {X[o].x, X[o].y, X[o].z, X[o].w}, yw[4] = {Y[o].x, Y[o].y, Y[o].z, Y[o].w}, zw[4] = {Z[o].x, Z[o].y, Z[o].z, Z[o].w};
+                        const int si = o + 4 * g2 + 2 * plane;  // scale byte within the half: o + 2 c
+                        const uint32_t w8 = g2 ? (h ? scw.w : scw.y) : (h ? scw.z : scw.x);
+                        const __half2 sc = __half2half2(__int2half_rn((int)(int8_t)((w8 >> (8 * (si & 3))) & 0xFFu)));
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            uint32_t q;
+                            if (g2 == 0) q = (plane ? yw[j] : xw[j]) & 0x3F3F3F3Fu;
+                            else q = plane ? (((xw[j] >> 6) & 0x03030303u) | ((yw[j] >> 4) & 0x0C0C0C0Cu) | ((zw[j] >> 2) & 0x30303030u)) : (zw[j] & 0x3F3F3F3Fu);
+                            uint32_t eh[2], el[2];
+                            expand_q6(q, sc, eh, el);
+                            hi[8 * o + 2 * j] = eh[0], hi[8 * o + 2 * j + 1] = eh[1], lo[8 * o + 2 * j] = el[0], lo[8 * o + 2 * j + 1] = el[1];
+                        }
+                    }
+                    warp_wait(bar(Q6_EMPTY_A + g), (uint32_t)((sb & 1) ^ 1), abort_flag, status);
+                    tc_fence_after();
+                    tc_st16(a_lane + (uint32_t)g * 64u, hi);
+                    tc_st16(a_lane + (uint32_t)g * 64u + 32u, lo);
+                    tc_wait_st();
+                    tc_fence_before();
+                    warp_arrive(bar(Q6_FULL_A + g));
+                }
+            }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+    } else {
+        const int quarter = warp & 3, half = (warp - WARP_DRAIN0) >> 2, rl = quarter * 32 + lane;
+        const size_t blk0 = (size_t)(row0 + rl) * nsb;
+        const int t0 = tt * TN + half * 64, live = M - t0;  // tokens of this thread
+        float *dst = out + (size_t)t0 * N + row0 + rl;
+        const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)half * 64u;
+        float acc[64];
+#pragma unroll
+        for (int i = 0; i < 64; ++i) acc[i] = 0.f;
+        bool folded = false;
+        for (int sb = 0; sb < nsb; ++sb) {
+            const float d = __half2float(*reinterpret_cast<const __half *>(q6u + smc_q6u_d(blk0 + sb)));
+#pragma unroll 1
+            for (int g = 0; g < NA; ++g) {
+                const int buf = g & 1, use = 2 * sb + (g >> 1);
+                warp_wait(bar(Q6_ACC_FULL + buf), (uint32_t)(use & 1), abort_flag, status);
+                tc_fence_after();
+                const uint32_t td = lane_base + (uint32_t)buf * 128u;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    float va[16];
+                    tc_ld16(td + (uint32_t)c * 16u, va);
+                    tc_wait_ld();
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) acc[c * 16 + i] = fmaf(d, va[i], acc[c * 16 + i]);
+                }
+                tc_fence_before();
+                warp_arrive(bar(Q6_ACC_EMPTY + buf));
+            }
+            // sixteen quarters per chain of fp32 sums, the chains' sums in `out` (each element belongs to one thread): one chain over
+            // all of K = 14336 came out 2.9e-7 from 64 bits (2-norm), against 1.8e-7 of the digit planes
+            if ((sb & 3) == 3 && sb + 1 < nsb) {
+                float *at = dst;
+#pragma unroll
+                for (int c = 0; c < 64; c += 4) {
+                    asm volatile("" : "+l"(at));  // one running pointer: 64 addresses kept over the loop would be spilled
+                    float v[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) v[i] = folded && c + i < live ? at[(size_t)i * N] : 0.f;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        if (c + i < live) at[(size_t)i * N] = v[i] + acc[c + i];
+                        acc[c + i] = 0.f;
+                    }
+                    at += (size_t)4 * N;
+                }
+                folded = true;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 64; ++i)
+            if (i < live) dst[(size_t)i * N] = (folded ? dst[(size_t)i * N] + acc[i] : acc[i]) * scale[t0 + i];
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        __syncwarp();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+    }
+}
+
 }  // namespace
 
 bool smc_prefill_supported(const smc_weight *w, int M)
@@ -611,4 +847,32 @@ int smc_launch_prefill_q4k_q8(smc_ctx *ctx, const smc_q8act *a, const smc_weight
 {
     if (a->K != w->K) return smc_fail(ctx, SMC_E_INVALID, "tensor-core matmul: activations have K=%d, weight has K=%d", a->K, w->K);
     return launch_prefill(ctx, nullptr, a, w, out, a->M, s, scratch_locked);
+}
+
+// fp32 rows over Q6_K where this kernel is the faster one.  A wave of tiles takes 22 ns per element of K whatever the tiles hold; the
+// digit planes on mma.sync take 5.5e-5 ns per element of K, weight row and activation row: the lines cross at about 410 000
+// outputs per wave.  Measured, digit planes -> here, us: 4096 x 4096 with 100 rows 109 -> 110, 200 rows 199 -> 112; 1024 x 4096
+// with 300 rows 90 -> 112, 500 rows 136 -> 112; 8192 x 28672 with 64 rows 830 -> 647, 600 rows (three waves) 7397 -> 1771.
+bool smc_prefill_q6k_supported(const smc_ctx *ctx, const smc_weight *w, int M)
+{
+    if (w->dtype != SMC_Q6_K || w->N % TM || w->K % 256 || M < 64 || !w->q6u) return false;
+    const long long tiles = (long long)(w->N / TM) * ((M + TN - 1) / TN), waves = (tiles + ctx->sm_count - 1) / ctx->sm_count;
+    return (long long)w->N * M >= 450000 * waves;
+}
+
+int smc_launch_prefill_q6k(smc_ctx *ctx, const float *x, const smc_weight *w, float *out, int M, cudaStream_t s)
+{
+    const int N = w->N, K = w->K, ntt = (M + TN - 1) / TN;
+    const size_t img_bytes = (size_t)ntt * TN * K * 2 * sizeof(__half);
+    std::lock_guard<std::mutex> lock(ctx->mu_scratch);  // held until everything is queued
+    const int rc = ensure_scratch(ctx, img_bytes + (size_t)ntt * TN * sizeof(float));
+    if (rc) return rc;
+    __half *img = reinterpret_cast<__half *>(ctx->d_prefill);
+    float *scale = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(ctx->d_prefill) + img_bytes);
+    prefill_scale_kernel<<<M, 256, 0, s>>>(x, M, K, scale);
+    prefill_image_kernel<<<ntt * (K / 256), 256, 0, s>>>(x, M, K, scale, img, nullptr);
+    SMC_CUDA(ctx, cudaFuncSetAttribute(prefill_q6k_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Q6_SMEM));
+    prefill_q6k_kernel<<<(N / TM) * ntt, THREADS, Q6_SMEM, s>>>(w->q6u, img, scale, out, N, K, M, ntt, ctx->d_status);
+    SMC_LAUNCH_CHECK(ctx);
+    return SMC_OK;
 }

@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 from sharpmind_b200 import ops, synth
-from tests.gpu_util import Q4_K, row_norm_bound, to_dev
+from tests.gpu_util import Q4_K, Q6_K, row_norm_bound, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -132,3 +132,40 @@ def test_quantised_activations_at_prefill_sizes_run_on_the_tensor_cores(oracle, 
     act.close()
     cuda.release(w)
     assert cuda.device_status() == 0
+
+
+@pytest.mark.parametrize("n,k,m", [
+    (7168, 256, 64),     # one block, half a token tile, the fewest outputs that come this way
+    (3584, 768, 128),    # rows that start inside a unit of eight blocks, fewer blocks than are folded at once
+    (3584, 2048, 129),   # a token tile of one
+    (2304, 4352, 200),   # 17 blocks: a last chain of one block
+    (8192, 1024, 300),   # two waves of tiles
+])
+def test_q6k_fp32_rows_on_the_tensor_cores(oracle, cuda, dev, n, k, m):
+    """fp32 rows over Q6_K at 64 rows and more: the weights' integer parts reach 4096 and travel as exact fp16 pairs.  Scales of
+    every size and sign (products above 2048 need the second half of the pair), rows of very different magnitude and a zero row;
+    against float64 over the dequantised weights at the bound of the mode, and no further off than the digit planes it replaces."""
+    import torch
+
+    rs = np.random.default_rng(n + k + m)
+    raw = np.array(oracle.quantize(Q6_K, synth.normal("prefill", f"w6{n}x{k}", (n, k), 0.02)), np.uint8).reshape(-1, 210)
+    raw[:, 192:208] = rs.integers(0, 256, (raw.shape[0], 16), dtype=np.uint8)
+    raw = np.ascontiguousarray(raw.reshape(-1))
+    x = synth.normal("prefill", f"x6{m}x{k}", (m, k))
+    x[1] *= 1e-6
+    x[2] *= 3e5
+    x[3] = 0.0
+    w = cuda.register(raw, Q6_K, n, k)
+    got = dev.qmatmul(to_dev(x), w, ops.Mode.ACT_F32).cpu().numpy()
+    assert cuda.device_status() == 0
+    want = x.astype(np.float64) @ oracle.dequantize(Q6_K, raw, n * k).reshape(n, k).astype(np.float64).T
+    bound = row_norm_bound(oracle, Q6_K, raw, n, k, x)
+    assert np.all(np.abs(got - want) <= bound + 1e-30), float(np.max(np.abs(got - want) / np.maximum(bound, 1e-30)))
+    assert np.all(got[3] == 0.0)
+    # the digit planes take batches below 64 rows
+    planes = torch.cat([dev.qmatmul(to_dev(x[i:i + 32]), w, ops.Mode.ACT_F32) for i in range(0, m, 32)]).cpu().numpy()
+    live = [i for i in range(m) if i != 3]
+    err = [float(np.linalg.norm(((y - want) / np.linalg.norm(want, axis=1, keepdims=True).clip(1e-30))[live])) for y in (got, planes)]
+    print(f"{n}x{k}, {m} rows: error {err[0]:.2e}, digit planes {err[1]:.2e}")
+    assert err[0] <= 1.25 * err[1]  # both are sums of roundings: a quarter more than what differs with the order
+    cuda.release(w)
