@@ -113,7 +113,7 @@ __device__ __forceinline__ void merge_heads(const float *rec0, float *out0, int 
 // dot (keys) or the softmax weight (values) once instead of every element: what ScaledDotProductFlashQ8_0*
 // (AttentionKernels.cs:489-813) computes, at a quarter of the fp32 cache's bytes.
 template <int DPL, int G, bool Q8>  // DPL = dims per lane = headDim / 8, G = query heads per KV head
-__global__ void __launch_bounds__(SPLIT_THREADS, G > 2 ? 2 : Q8 ? 4 : 3) sdpa_decode_split_kernel(
+__global__ void __launch_bounds__(SPLIT_THREADS, Q8 && G <= 2 ? 4 : 1) sdpa_decode_split_kernel(
     const float *__restrict__ q, const void *__restrict__ kc_, const void *__restrict__ vc_, const __half *__restrict__ kd,
     const __half *__restrict__ vd, float *part, int heads, int kvHeads, int kvLen, int maxSeq, float scale, int splits,
     float *__restrict__ out, unsigned *tickets, int hshare)
@@ -161,11 +161,11 @@ __global__ void __launch_bounds__(SPLIT_THREADS, G > 2 ? 2 : Q8 ? 4 : 3) sdpa_de
     // every lane group runs the same number of iterations so the shuffles below stay converged
     const int iters = k1 > k0 ? (k1 - k0 + ngroups - 1) / ngroups : 0;
     // A key's K and V pieces are requested AHEAD iterations before they are used: with a few CTAs of four warps per SM the
-    // sweep waited for one key at a time.  The order of the sums is untouched.  32 sequences over 1501 Q8_0 rows each (8 KV
-    // heads of 128, 28 layers, the whole step): 2870 -> 2640 us; fp32 rows of one sequence: no change beyond noise.
-    // Registers are capped so that the grids of the launcher (two CTAs per SM and more) still run in one wave: with two fp32
-    // CTAs per SM instead of three, 304 CTAs needed a second wave and an 8B-shaped step went from 2209 to 2389 us.
-    constexpr int AHEAD = Q8 ? 3 : 2, PIECES = Q8 ? DPL / 4 : DPL;
+    // sweep waited for one key at a time.  The order of the sums is untouched.  Q8_0 rows, three keys ahead, registers capped so that
+    // the launcher's 512 CTAs still run in one wave: 32 sequences over 1501 rows each (8 KV heads of 128, 28 layers, the whole
+    // step) 2870 -> 2642 us.  fp32 rows are four times the bytes a key: one ahead, 1004 -> 993 us a step of the 28-layer shape
+    // and 2220 -> 2186 us of the 8B shape at 2048 positions; two ahead cost 2 % (fewer CTAs per SM), none 1 to 3 %.
+    constexpr int AHEAD = Q8 ? 3 : 1, PIECES = Q8 ? DPL / 4 : DPL;
     uint32_t kw[AHEAD][PIECES], vw[AHEAD][PIECES];
     __half kh[AHEAD], vh[AHEAD];  // block scales of the lane's dims (Q8)
     auto fetch = [&](int it, int u) {
