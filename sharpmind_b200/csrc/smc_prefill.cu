@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(256) prefill_scale_kernel(const float *__restr
         if (amax > 0.f && amax < INFINITY) {
             int e;
             frexpf(amax, &e);          // amax = f * 2^e, f in [0.5, 1)
-            s = ldexpf(1.0f, e - 10);  // amax / s in [512, 1024)
+            s = ldexpf(1.0f, max(e - 10, -126));  // amax / s in [512, 1024); 1 / s stays finite for rows below 2^-117
         }
         scale[t] = s;
     }

@@ -143,7 +143,8 @@ def test_quantised_activations_at_prefill_sizes_run_on_the_tensor_cores(oracle, 
 ])
 def test_q6k_fp32_rows_on_the_tensor_cores(oracle, cuda, dev, n, k, m):
     """fp32 rows over Q6_K at 64 rows and more: the weights' integer parts reach 4096 and travel as exact fp16 pairs.  Scales of
-    every size and sign (products above 2048 need the second half of the pair), rows of very different magnitude and a zero row;
+    every size and sign (products above 2048 need the second half of the pair), rows of very different magnitude (one whose
+    scale has no finite inverse) and a zero row;
     against float64 over the dequantised weights at the bound of the mode, and no further off than the digit planes it replaces."""
     import torch
 
@@ -155,6 +156,7 @@ def test_q6k_fp32_rows_on_the_tensor_cores(oracle, cuda, dev, n, k, m):
     x[1] *= 1e-6
     x[2] *= 3e5
     x[3] = 0.0
+    x[4] *= 1e-37
     w = cuda.register(raw, Q6_K, n, k)
     got = dev.qmatmul(to_dev(x), w, ops.Mode.ACT_F32).cpu().numpy()
     assert cuda.device_status() == 0
