@@ -328,7 +328,10 @@ class DeviceOps:
         self.lib = ctx.lib
 
     def _stream(self):
-        return C.c_void_p(self.torch.cuda.current_stream().cuda_stream)
+        """The current stream's handle, without the Stream object that torch.cuda.current_stream() builds around it (a call of
+        one small row is bound by the host: 11.3 us with it, 7.3 us without)."""
+        c = self.torch._C
+        return c._cuda_getCurrentRawStream(c._cuda_getDevice())
 
     def _chk(self, t, dtype=None):
         if not t.is_cuda or not t.is_contiguous():
@@ -339,15 +342,20 @@ class DeviceOps:
 
     def qmatmul(self, x, w: Weight, mode: int = Mode.ACT_F32, out=None):
         t = self.torch
-        M = x.numel() // w.K
-        if x.numel() != M * w.K:
+        M, rest = divmod(x.numel(), w.K)
+        if rest:
             raise ArgumentException(f"input of {x.numel()} values is not a multiple of K = {w.K}")
-        if out is None:
+        own = out is None
+        if own:
             out = t.empty((M, w.N), dtype=t.float32, device=x.device)
         if M == 0:
             return out
-        self.ctx.check(self.lib.smc_qmatmul_dev(self.ctx.h, self._chk(x, t.float32), w.handle, self._chk(out, t.float32),
-                                                M, int(mode), self._stream()))
+        # (a fresh tensor needs no look; x comes first, as what is wrong with it has always been reported first)
+        xp = self._chk(x, t.float32)
+        op = out.data_ptr() if own and out.is_cuda else self._chk(out, t.float32)
+        rc = self.lib.smc_qmatmul_dev(self.ctx.h, xp, w.handle, op, M, int(mode), self._stream())
+        if rc:
+            self.ctx.check(rc)
         return out
 
     def interleave_rows(self, gate: Weight, up: Weight) -> Weight:
