@@ -808,14 +808,12 @@ static int launch_prefill(smc_ctx *ctx, const float *x, const smc_q8act *a, cons
     const size_t scale_off = (img_halves + mimg_halves) * sizeof(__half);
     const size_t x_off = (scale_off + (size_t)ntt * TN * sizeof(float) + 255) & ~(size_t)255;
     const size_t bytes = x_off + (a ? (size_t)M * K * sizeof(float) : 0);
-    if (scratch_locked) {  // the caller holds mu_scratch (its own scratch rows are the input)
-        int rc = ensure_scratch(ctx, bytes);
-        if (rc) return rc;
-    } else {
-        std::lock_guard<std::mutex> lock(ctx->mu_scratch);
-        int rc = ensure_scratch(ctx, bytes);
-        if (rc) return rc;
-    }
+    // Held until everything is queued: another host thread's launches must not come between the image and its contraction,
+    // nor may a larger call free the buffer before these are queued.
+    std::unique_lock<std::mutex> lock(ctx->mu_scratch, std::defer_lock);
+    if (!scratch_locked) lock.lock();  // else the caller holds it (its own scratch rows are the input)
+    const int rc = ensure_scratch(ctx, bytes);
+    if (rc) return rc;
     __half *img = reinterpret_cast<__half *>(ctx->d_prefill);
     __half *mimg = img + img_halves;
     float *scale = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(ctx->d_prefill) + scale_off);

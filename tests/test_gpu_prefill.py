@@ -171,3 +171,61 @@ def test_q6k_fp32_rows_on_the_tensor_cores(oracle, cuda, dev, n, k, m):
     print(f"{n}x{k}, {m} rows: error {err[0]:.2e}, digit planes {err[1]:.2e}")
     assert err[0] <= 1.25 * err[1]  # both are sums of roundings: a quarter more than what differs with the order
     cuda.release(w)
+
+
+def test_host_threads_on_one_context_and_stream(oracle):
+    """Matmuls that keep an image of their rows in the context, queued by several host threads on one stream: every result
+    has the bits of the same call made alone (no thread's image is overwritten before its contraction is queued, and no
+    buffer is freed under a call when another thread's larger one grows it; the sizes grow as the threads go on)."""
+    import threading
+
+    import torch
+
+    cases = []
+    raw4 = oracle.quantize(Q4_K, synth.normal("threads", "w4", (256, 512), 0.02))
+    raw6 = oracle.quantize(Q6_K, synth.normal("threads", "w6", (7168, 256), 0.02))
+    wb = synth.normal("threads", "wb", (256, 512), 0.02)
+
+    def weights(ctx):
+        b = torch.from_numpy(wb).cuda().to(torch.bfloat16).view(torch.uint8).reshape(-1)
+        return {"q4": ctx.register(raw4, Q4_K, 256, 512), "q6": ctx.register(raw6, Q6_K, 7168, 256),
+                "bf16": ctx.register_dev(b, ops.QuantDType.BF16, 256, 512, repack=False)}
+
+    for name, k, mode in (("q4", 512, ops.Mode.ACT_F32), ("q6", 256, ops.Mode.ACT_F32), ("q4", 512, ops.Mode.ACT_Q8), ("bf16", 512, ops.Mode.ACT_BF16)):
+        cases.append((name, mode, [to_dev(synth.normal("threads", f"x{name}{int(mode)}{m}", (m, k))) for m in (64, 70, 128, 190, 256, 391)]))
+
+    def run_all(threads):
+        ctx = ops.CudaContext(0)
+        dev, w = ops.DeviceOps(ctx), weights(ctx)
+        torch.cuda.synchronize()
+        out, failed = [[] for _ in cases], []
+
+        def body(i):
+            name, mode, xs = cases[i]
+            try:
+                for x in xs:
+                    out[i] += [dev.qmatmul(x, w[name], mode) for _ in range(24)]
+            except Exception as e:  # reported below, by the test's own thread
+                failed.append(e)
+
+        if threads:
+            ts = [threading.Thread(target=body, args=(i,)) for i in range(len(cases))]
+            for t in ts:
+                t.start()
+            for t in ts:
+                t.join()
+        else:
+            for i in range(len(cases)):
+                body(i)
+        torch.cuda.synchronize()
+        assert not failed, failed
+        assert ctx.device_status() == 0
+        for h in w.values():
+            ctx.release(h)
+        ctx.close()
+        return out
+
+    alone, together = run_all(False), run_all(True)
+    for (name, mode, xs), a, b in zip(cases, alone, together):
+        wrong = [i for i, (u, v) in enumerate(zip(a, b)) if not torch.equal(u.view(torch.int32), v.view(torch.int32))]
+        assert not wrong, (name, mode, wrong)
