@@ -241,7 +241,7 @@ void smc_destroy(smc_ctx *ctx)
     if (ctx->h_pin) cudaFreeHost(ctx->h_pin);
     smc_q8act_free(ctx->act);
     smc_q8act_free(ctx->digits);
-    cudaFree(ctx->d_digit_out);
+    cudaFree(ctx->d_fp32_rows);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
@@ -465,41 +465,54 @@ int smc_qmatmul_q8_dev(smc_ctx *ctx, const smc_q8act *a, const smc_weight *w, fl
     return smc_launch_gemv_q8(ctx, a, w, d_out, static_cast<cudaStream_t>(stream));
 }
 
+// Scratch of fp32 rows over M x K activations and N outputs (caller holds mu_scratch): the digit planes, and one block that
+// holds either the planes' products or the activation image of the tcgen05 form of Q6_K.  A call reserves for both forms
+// whichever it takes, so that after a first one no call with at most its values (M K) and outputs (M N) allocates.
+static int reserve_fp32_rows(smc_ctx *ctx, const smc_weight *w, int M)
+{
+    const size_t values = (size_t)M * w->K;
+    if (!ctx->digits || ctx->digits_cap < 3 * values) {
+        if (ctx->digits) {  // growing allocates: make the first call of a new size outside stream capture
+            cudaDeviceSynchronize();
+            smc_q8act_free(ctx->digits);
+            ctx->digits = nullptr, ctx->digits_cap = 0;
+        }
+        const int rc = smc_q8act_alloc(ctx, 3 * M, w->K, &ctx->digits);
+        if (rc) return rc;
+        ctx->digits_cap = 3 * values;
+    }
+    size_t block = (size_t)3 * M * w->N * sizeof(float);
+    if (ctx->has_q6k || w->q6u) block = std::max(block, smc_prefill_q6k_scratch(values));  // a context without such weights needs no image
+    if (ctx->fp32_rows_cap < block) {
+        if (ctx->d_fp32_rows) {
+            cudaDeviceSynchronize();
+            cudaFree(ctx->d_fp32_rows);
+            ctx->d_fp32_rows = nullptr, ctx->fp32_rows_cap = 0;
+        }
+        SMC_CUDA(ctx, cudaMalloc(&ctx->d_fp32_rows, block));
+        ctx->fp32_rows_cap = block;
+    }
+    return SMC_OK;
+}
+
 // SMC_ACT_F32 at prefill sizes over a format without a tcgen05 kernel: the fp32 rows become three int8 digit planes
 // (x = d1 q1 + d2 q2 + d3 q3 to 6e-8 of a block's largest value), each plane goes through the integer tensor-core
 // kernels and the three products are added, smallest last.  Three passes of the int8 kernels instead of M / 8 passes
 // of the CUDA-core kernel over the weights; same parity bound as that kernel (tested), other bits.
+// Q6_K has a tcgen05 kernel for the sizes that fill the device (same bound, other bits again).
 static int qmatmul_f32_digits(smc_ctx *ctx, const float *d_in, const smc_weight *w, float *d_out, int M, cudaStream_t s)
 {
     std::lock_guard<std::mutex> lock(ctx->mu_scratch);  // held until everything is queued, like the Q8 scratch
     int rc;
-    smc_q8act *&a = ctx->digits;
-    const size_t need = (size_t)3 * M * w->K;
-    if (!a || ctx->digits_cap < need) {
-        if (a) {  // growing allocates: make the first call of a new size outside stream capture
-            cudaDeviceSynchronize();
-            smc_q8act_free(a);
-            a = nullptr;
-            ctx->digits_cap = 0;
-        }
-        if ((rc = smc_q8act_alloc(ctx, 3 * M, w->K, &a))) return rc;
-        ctx->digits_cap = need;
-    }
+    if ((rc = reserve_fp32_rows(ctx, w, M))) return rc;
+    if (smc_prefill_q6k_supported(ctx, w, M)) return smc_launch_prefill_q6k(ctx, d_in, w, d_out, M, ctx->d_fp32_rows, s);
+    smc_q8act *a = ctx->digits;
+    float *products = static_cast<float *>(ctx->d_fp32_rows);
     a->max_rows = (int)(ctx->digits_cap / w->K), a->max_k = w->K;  // the same allocation (digits_cap values), seen with this K
-    const size_t out_bytes = (size_t)3 * M * w->N * sizeof(float);
-    if (ctx->digit_out_cap < out_bytes) {
-        if (ctx->d_digit_out) {
-            cudaDeviceSynchronize();
-            cudaFree(ctx->d_digit_out);
-            ctx->d_digit_out = nullptr, ctx->digit_out_cap = 0;
-        }
-        SMC_CUDA(ctx, cudaMalloc(&ctx->d_digit_out, out_bytes));
-        ctx->digit_out_cap = out_bytes;
-    }
     // the planes are 3 M rows of one batch: the weights are read once for all three
     if ((rc = smc_launch_quantize_q8_digits(ctx, d_in, M, w->K, a, s))) return rc;
-    if ((rc = smc_launch_gemv_q8(ctx, a, w, ctx->d_digit_out, s))) return rc;
-    return smc_launch_sum3(ctx, ctx->d_digit_out, d_out, (long long)M * w->N, s);
+    if ((rc = smc_launch_gemv_q8(ctx, a, w, products, s))) return rc;
+    return smc_launch_sum3(ctx, products, d_out, (long long)M * w->N, s);
 }
 
 // A dense bfloat16 weight: fp32 rows as they are (SMC_ACT_F32) or rounded to bfloat16 in the context's scratch first.
@@ -535,9 +548,6 @@ static int qmatmul_impl(smc_ctx *ctx, const float *d_in, const smc_weight *w, fl
         // prefill-sized batches of Q4_K run on the tcgen05 tensor cores (same parity bound, see smc_prefill.cu)
         if (M >= 64 && smc_prefill_supported(w, M) && (reinterpret_cast<uintptr_t>(d_in) & 15) == 0)
             return smc_launch_prefill_q4k(ctx, d_in, w, d_out, M, s);
-        // Q6_K too, where the digit planes are on (the option that selects the CUDA-core kernel instead also covers this one)
-        if (ctx->f32_digits && smc_prefill_q6k_supported(ctx, w, M) && M >= ctx->f32_digits && (reinterpret_cast<uintptr_t>(d_in) & 15) == 0)
-            return smc_launch_prefill_q6k(ctx, d_in, w, d_out, M, s);
         if (ctx->f32_digits && M >= (ctx->f32_digits > 1 ? ctx->f32_digits : 2) && w->fast && (reinterpret_cast<uintptr_t>(d_in) & 15) == 0)
             return qmatmul_f32_digits(ctx, d_in, w, d_out, M, s);
         // one row over a large matrix: its three digit rows through the several-row integer kernel beat the fp32 one-row kernel

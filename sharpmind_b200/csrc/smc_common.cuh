@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+#include <atomic>
 #include <mutex>
 #include <string>
 #include <unordered_map>
@@ -87,8 +89,9 @@ struct smc_ctx {
     unsigned pin_next = 0;
     smc_q8act *digits = nullptr;       // the three int8 digit planes of fp32 activations, stacked as 3 M rows (SMC_ACT_F32)
     size_t digits_cap = 0;             // values it holds
-    float *d_digit_out = nullptr;      // their products [3 M, N]
-    size_t digit_out_cap = 0;
+    void *d_fp32_rows = nullptr;       // their products [3 M, N], or the activation image of the tcgen05 form of Q6_K
+    size_t fp32_rows_cap = 0;
+    std::atomic<bool> has_q6k{false};  // a repacked Q6_K weight was registered: the block above is also sized for the image
     int f32_digits = 1;                // that path on (0: the CUDA-core kernel at every batch size)
     int f32_digits_row_mb = 32;        // one row: K-quant matrices of at least this many MB take that path too (0: never)
     int *d_status = nullptr;           // raised by a kernel whose bounded wait ran out
@@ -156,7 +159,8 @@ int smc_launch_gemv_tma_gather(smc_ctx *, const float *x, const smc_weight *, fl
 int smc_qmatmul_dev_gather(smc_ctx *, const float *d_in, const smc_weight *, float *d_out, int M, int mode, cudaStream_t s,
                            const smc_gather_dev *, bool *fused);
 bool smc_prefill_q6k_supported(const smc_ctx *, const smc_weight *, int M);
-int smc_launch_prefill_q6k(smc_ctx *, const float *x, const smc_weight *, float *out, int M, cudaStream_t s);
+size_t smc_prefill_q6k_scratch(size_t values);
+int smc_launch_prefill_q6k(smc_ctx *, const float *x, const smc_weight *, float *out, int M, void *scratch, cudaStream_t s);
 bool smc_prefill_supported(const smc_weight *, int M);
 int smc_launch_prefill_q4k(smc_ctx *, const float *x, const smc_weight *, float *out, int M, cudaStream_t s);
 int smc_launch_prefill_q4k_q8(smc_ctx *, const smc_q8act *a, const smc_weight *, float *out, cudaStream_t s, bool scratch_locked = false);

@@ -858,15 +858,16 @@ bool smc_prefill_q6k_supported(const smc_ctx *ctx, const smc_weight *w, int M)
     return (long long)w->N * M >= 450000 * waves;
 }
 
-int smc_launch_prefill_q6k(smc_ctx *ctx, const float *x, const smc_weight *w, float *out, int M, cudaStream_t s)
+// Bytes that hold the image and scales of every call with at most `values` = M K activations: M >= 64 rows (K >= 256) are at most
+// doubled by rounding them up to whole tiles, and a row has a scale of four bytes.
+size_t smc_prefill_q6k_scratch(size_t values) { return 2 * values * 2 * sizeof(__half) + values / 32; }
+
+// scratch: smc_prefill_q6k_scratch(M K) bytes; the caller holds mu_scratch until this returns
+int smc_launch_prefill_q6k(smc_ctx *ctx, const float *x, const smc_weight *w, float *out, int M, void *scratch, cudaStream_t s)
 {
     const int N = w->N, K = w->K, ntt = (M + TN - 1) / TN;
-    const size_t img_bytes = (size_t)ntt * TN * K * 2 * sizeof(__half);
-    std::lock_guard<std::mutex> lock(ctx->mu_scratch);  // held until everything is queued
-    const int rc = ensure_scratch(ctx, img_bytes + (size_t)ntt * TN * sizeof(float));
-    if (rc) return rc;
-    __half *img = reinterpret_cast<__half *>(ctx->d_prefill);
-    float *scale = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(ctx->d_prefill) + img_bytes);
+    __half *img = static_cast<__half *>(scratch);
+    float *scale = reinterpret_cast<float *>(img + (size_t)ntt * TN * K * 2);
     prefill_scale_kernel<<<M, 256, 0, s>>>(x, M, K, scale);
     prefill_image_kernel<<<ntt * (K / 256), 256, 0, s>>>(x, M, K, scale, img, nullptr);
     SMC_CUDA(ctx, cudaFuncSetAttribute(prefill_q6k_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Q6_SMEM));

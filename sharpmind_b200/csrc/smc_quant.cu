@@ -500,6 +500,7 @@ int smc_launch_repack(smc_ctx *ctx, smc_weight *w, cudaStream_t s)
     } else if (w->dtype == SMC_Q6_K) {
         long long nblocks = (long long)w->N * w->K / 256;
         SMC_CUDA(ctx, cudaMalloc(&w->q6u, smc_q6u_bytes((size_t)nblocks)));
+        ctx->has_q6k = true;
         if (nblocks % 8)  // the blocks missing from the last unit read as zero weights
             SMC_CUDA(ctx, cudaMemsetAsync(w->q6u + smc_q6u_bytes((size_t)nblocks) - SMC_Q6U_BYTES, 0, SMC_Q6U_BYTES, s));
         repack_q6_K_kernel<<<grid_for(nblocks * 64, 256, ctx->sm_count * 16), 256, 0, s>>>(w->d_raw, w->q6u, nblocks);

@@ -229,3 +229,48 @@ def test_host_threads_on_one_context_and_stream(oracle):
     for (name, mode, xs), a, b in zip(cases, alone, together):
         wrong = [i for i, (u, v) in enumerate(zip(a, b)) if not torch.equal(u.view(torch.int32), v.view(torch.int32))]
         assert not wrong, (name, mode, wrong)
+
+
+def _capture(body):
+    """Captures `body` and replays the graph."""
+    import torch
+
+    g = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(g):
+        body()
+    g.replay()
+    torch.cuda.synchronize()
+    return g
+
+
+@pytest.mark.parametrize("warm,then", [
+    ((200, 3584, 256), [(200, 3584, 256), (126, 3584, 256), (125, 3584, 256), (64, 3584, 256), (2, 3584, 256)]),  # both sides of the line between the forms
+    ((63, 7296, 512), [(64, 7168, 256), (63, 7296, 512)]),   # first the digit planes
+    ((201, 2304, 4352), [(129, 3584, 6656)]),                # fewer values, but as many tiles of rows of a longer K
+])
+def test_fp32_rows_over_q6k_reserve_for_both_forms(oracle, warm, then):
+    """SMC_ACT_F32 over Q6_K takes one of two forms by M and N.  A call with no more values and no more outputs than an earlier
+    one does not allocate, whichever forms the two take: it can be captured."""
+    import torch
+
+    ctx = ops.CudaContext(0)
+    dev, ws = ops.DeviceOps(ctx), {}
+    for m, n, k in [warm] + then:
+        if (n, k) not in ws:
+            ws[n, k] = ctx.register(oracle.quantize(Q6_K, synth.normal("both", f"w{n}x{k}", (n, k), 0.02)), Q6_K, n, k)
+
+    def call(m, n, k):
+        return dev.qmatmul(to_dev(synth.normal("both", f"x{m}x{k}", (m, k))), ws[n, k], ops.Mode.ACT_F32)
+
+    call(*warm)
+    xs = [to_dev(synth.normal("both", f"x{m}x{k}", (m, k))) for m, n, k in then]
+    outs = [torch.empty((m, n), device="cuda") for m, n, k in then]
+    g = _capture(lambda: [dev.qmatmul(x, ws[n, k], ops.Mode.ACT_F32, out=o) for x, o, (m, n, k) in zip(xs, outs, then)])
+    for o, c in zip(outs, then):
+        assert torch.equal(o, call(*c)), c
+    del g
+    for w in ws.values():
+        ctx.release(w)
+    assert ctx.device_status() == 0
+    ctx.close()
