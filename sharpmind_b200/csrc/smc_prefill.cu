@@ -26,6 +26,7 @@
 // A stages of 32 columns.  Every mbarrier wait is bounded; a wait that runs out raises the context's status
 // word and a CTA-wide abort flag that makes every later wait return at once, so the kernel still ends and
 // frees its TMEM.
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -197,7 +198,7 @@ constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)
 //   mimg [token tile][block = k / 256][hi | lo][token / 8][2][token % 8][8]                          fp16
 //        (tile hi: sx~ hi of sub-blocks 0..7, twice; tile lo: sx~ lo, twice)
 //   scale[token]  fp32 power of two
-__global__ void __launch_bounds__(256) prefill_scale_kernel(const float *__restrict__ x, int M, int K, float *__restrict__ scale)
+__global__ void __launch_bounds__(256) prefill_scale_kernel(const float *__restrict__ x, int M, int K, int top, float *__restrict__ scale)
 {
     __shared__ float red[8];
     const int t = blockIdx.x;
@@ -212,8 +213,8 @@ __global__ void __launch_bounds__(256) prefill_scale_kernel(const float *__restr
         float s = 1.0f;
         if (amax > 0.f && amax < INFINITY) {
             int e;
-            frexpf(amax, &e);          // amax = f * 2^e, f in [0.5, 1)
-            s = ldexpf(1.0f, max(e - 10, -126));  // amax / s in [512, 1024); 1 / s stays finite for rows below 2^-117
+            frexpf(amax, &e);                      // amax = f * 2^e, f in [0.5, 1)
+            s = ldexpf(1.0f, max(e - top, -126));  // amax / s in [2^(top - 1), 2^top); 1 / s stays finite for the smallest rows
         }
         scale[t] = s;
     }
@@ -254,7 +255,6 @@ __global__ void __launch_bounds__(256) prefill_image_kernel(const float *__restr
                             (size_t)(c & 7) * 64 + (size_t)(tl & 7) * 8;
         *reinterpret_cast<uint4 *>(img + base) = *reinterpret_cast<const uint4 *>(hi);
         *reinterpret_cast<uint4 *>(img + base + TN * KS) = *reinterpret_cast<const uint4 *>(lo);
-        if (!mimg) continue;  // Q6_K has no min term
         // sub-block sums: chunks 4j .. 4j+3 are adjacent lanes
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);
         sum += __shfl_xor_sync(0xffffffffu, sum, 2);
@@ -529,45 +529,84 @@ prefill_q4k_kernel(const uint8_t *__restrict__ raw, const __half *__restrict__ i
 
 // ------------------------------------------------------------------------------ Q6_K
 // The same contraction over Q6_K:  w[r, k] = d_b * v,  v = sc_j * (q_k - 32)  with sc_j an int8 per 16 elements, |v| <= 4096.
-// Not every v is an fp16 (odd ones above 2048 are not), so the weights travel as an exact pair v = v_hi + v_lo, v_hi the
-// rounded product and v_lo in {-1, 0, 1}; the dropped v_lo x_lo is below 2^-22 of a product and rare:
-//   acc_d[r, t] = sum_{k in g} v_lo x_hi + v_hi x_lo + v_hi x_hi     12 MMAs of K = 16 per quarter g of a block, smallest first
+// Operands are exact: thirteen-bit v as a pair of bfloat16 (v = v_hi + v_lo), an fp32 activation as three (x = x0 + x1 + x2, each the
+// rounded rest; the row scale only keeps x2 above bfloat16's smallest numbers, down to 2^-170 of the row's largest element), and
+// their products are summed smallest first, without v_lo x2 (below 2^-27 of the whole product):
+//   acc_d[r, t] = sum_{k in g} v_lo x1 + v_hi x2 + v_lo x0 + v_hi x1 + v_hi x0     20 MMAs of K = 16 per quarter g of a block
 //   out[t, r]   = s_t * sum_b d_b * sum_{g in b} acc_d(g)
+// (An fp16 pair per activation, as for Q4_K, takes twelve, but fp16 has no range below a row's largest element: one element of 1e5 in
+// columns of zero weights put the row's other products 12 times further from 64 bits than three int8 digits with a scale per 32
+// elements do, one of 1e12 lost them all.)
 // The tensor cores cut their sums off instead of rounding them: with one accumulator for a whole block (16 MMAs at full size in
 // one chain) the result was five times further from 64 bits than the kernels this one replaces; quarters put that right.
 // Warp roles as above; tensor memory holds two accumulators and four A stages of {hi, lo} (no min term).  A block's bytes lie in
 // five places of its unit, so they come by 16-byte asynchronous copies: a warp of the first four (plane 0) fetches the rows of its
 // quarter for both warps of the quarter and the pair meets at a named barrier; plane 0 unpacks the first 32 elements of each
 // stage, plane 1 the second 32.
-// What bounds it: the tensor cores, three MMAs per product, and the activation stages' way into the SM.  Before, fp32 rows went through
-// mma.sync as three int8 digit planes, one scaling on the CUDA cores per output, plane and 16 elements.
-// 4096 x 14336 with 500 rows: 1595 -> 346 us (169 useful TFLOP/s); distance from 64 bits 1.84e-7 -> 1.54e-7, 8192 x 28672
-// 2.26e-7 -> 1.69e-7, 1024 x 4096 1.50e-7 -> 1.42e-7.
-constexpr int Q6_RAW = 240;                        // bytes of a row and block in shared memory: X, Y, Z (64 each), 16 scales, padding to an odd multiple of 16
+// What bounds it: the MMAs (twelve fewer per stage took 80 of 447 us off) on top of about 1 us per stage that stays when the drain, the fold, the
+// unpacking or the copies are left out one by one.  Before, fp32 rows went through mma.sync as three int8 digit planes, one scaling on
+// the CUDA cores per output, plane and 16 elements.
+// 4096 x 14336 with 500 rows: 1595 -> 404 us (145 useful TFLOP/s); distance from 64 bits 1.84e-7 -> 1.33e-7, 8192 x 28672
+// 2.26e-7 -> 1.42e-7, 1024 x 4096 1.50e-7 -> 1.26e-7.
+constexpr int Q6_RAW = 208;                        // bytes of a row and block in shared memory: X, Y, Z (64 each), 16 scales: an odd multiple of 16
 constexpr int Q6_NW = 3;                           // blocks in flight
 constexpr uint32_t Q6_W_BYTES = TM * Q6_RAW;
-constexpr uint32_t Q6_OFF_W = NB * SLOT_BYTES, Q6_OFF_BAR = Q6_OFF_W + Q6_NW * Q6_W_BYTES, Q6_SMEM = Q6_OFF_BAR + 256;
+constexpr int Q6_NB = 3;                           // activation stages in shared memory
+constexpr uint32_t Q6_SLOT = 3 * B_BYTES;          // x0, x1, x2
+constexpr uint32_t Q6_OFF_W = Q6_NB * Q6_SLOT, Q6_OFF_BAR = Q6_OFF_W + Q6_NW * Q6_W_BYTES, Q6_SMEM = Q6_OFF_BAR + 256;
 static_assert(Q6_SMEM <= 227 * 1024, "shared memory budget");
 constexpr uint32_t Q6_COL_A = 256;                 // NA x 64 columns: 32 of v_hi, 32 of v_lo
-enum { Q6_FULL_B = 0, Q6_EMPTY_B = Q6_FULL_B + NB, Q6_FULL_A = Q6_EMPTY_B + NB, Q6_EMPTY_A = Q6_FULL_A + NA, Q6_ACC_FULL = Q6_EMPTY_A + NA,
+enum { Q6_FULL_B = 0, Q6_EMPTY_B = Q6_FULL_B + Q6_NB, Q6_FULL_A = Q6_EMPTY_B + Q6_NB, Q6_EMPTY_A = Q6_FULL_A + NA, Q6_ACC_FULL = Q6_EMPTY_A + NA,
        Q6_ACC_EMPTY = Q6_ACC_FULL + 2, Q6_BARS = Q6_ACC_EMPTY + 2 };
 static_assert(Q6_BARS * 8 + 8 <= 256, "barrier area");
 
-// four codes 0..63 in the bytes of `q` -> two fp16 pairs each of v_hi and v_lo
-__device__ __forceinline__ void expand_q6(uint32_t q, __half2 sc, uint32_t (&hi)[2], uint32_t (&lo)[2])
+constexpr uint32_t Q6_IDESC = IDESC | (1u << 7) | (1u << 10);  // bfloat16 A and B
+
+// img [token tile][stage = k / 64][x0 | x1 | x2][token / 8][k chunk = (k % 64) / 8][token % 8][k % 8]; one CTA per (token tile, block of 256)
+__global__ void __launch_bounds__(256) prefill_q6k_image_kernel(const float *__restrict__ x, int M, int K, const float *__restrict__ scale,
+                                                                __nv_bfloat16 *__restrict__ img)
 {
-    const __half2 off = __half2half2(__ushort_as_half((unsigned short)0xE420u));  // -1056: takes 1024 + 32 off
+    const int nsb = K / 256, tt = blockIdx.x / nsb, sb = blockIdx.x % nsb;
+    for (int it = threadIdx.x; it < TN * 32; it += blockDim.x) {
+        const int tl = it >> 5, c = it & 31, t = tt * TN + tl;  // token in tile, chunk in block
+        float v[8] = {};
+        if (t < M) {
+            const float inv = 1.0f / scale[t];  // exact: a power of two
+            const float4 a = *reinterpret_cast<const float4 *>(x + (size_t)t * K + sb * 256 + c * 8);
+            const float4 b = *reinterpret_cast<const float4 *>(x + (size_t)t * K + sb * 256 + c * 8 + 4);
+            v[0] = a.x * inv, v[1] = a.y * inv, v[2] = a.z * inv, v[3] = a.w * inv;
+            v[4] = b.x * inv, v[5] = b.y * inv, v[6] = b.z * inv, v[7] = b.w * inv;
+        }
+        __nv_bfloat16 *dst = img + ((size_t)(tt * (K / KS) + sb * 4 + (c >> 3)) * 3) * (TN * KS) + (size_t)(tl >> 3) * (KS / 8 * 64) +
+                             (size_t)(c & 7) * 64 + (size_t)(tl & 7) * 8;
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            __align__(16) __nv_bfloat16 part[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                part[i] = __float2bfloat16_rn(v[i]);
+                v[i] -= __bfloat162float(part[i]);  // exact
+            }
+            *reinterpret_cast<uint4 *>(dst + (size_t)p * (TN * KS)) = *reinterpret_cast<const uint4 *>(part);
+        }
+    }
+}
+
+// four codes 0..63 in the bytes of `q` -> two bfloat16 pairs each of v_hi and v_lo
+__device__ __forceinline__ void expand_q6(uint32_t q, __nv_bfloat162 sc, uint32_t (&hi)[2], uint32_t (&lo)[2])
+{
+    const __nv_bfloat162 off = __bfloat162bfloat162(__ushort_as_bfloat16((unsigned short)0xC320u));  // -160: takes 128 + 32 off
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-        const uint32_t p = __byte_perm(q, 0x64646464u, i ? 0x4342u : 0x4140u);
-        const __half2 c = __hadd2(*reinterpret_cast<const __half2 *>(&p), off);
-        const __half2 h = __hmul2(c, sc), l = __hfma2(c, sc, __hneg2(h));  // the remainder of an fp16 product is exact
+        const uint32_t p = __byte_perm(q, 0x43434343u, i ? 0x4342u : 0x4140u);  // 128 + code
+        const __nv_bfloat162 c = __hadd2(*reinterpret_cast<const __nv_bfloat162 *>(&p), off);
+        const __nv_bfloat162 h = __hmul2(c, sc), l = __hfma2(c, sc, __hneg2(h));  // the remainder of a thirteen-bit product is exact
         hi[i] = *reinterpret_cast<const uint32_t *>(&h), lo[i] = *reinterpret_cast<const uint32_t *>(&l);
     }
 }
 
 __global__ void __launch_bounds__(THREADS, 1)
-prefill_q6k_kernel(const uint8_t *__restrict__ q6u, const __half *__restrict__ img, const float *__restrict__ scale, float *__restrict__ out, int N, int K,
+prefill_q6k_kernel(const uint8_t *__restrict__ q6u, const __nv_bfloat16 *__restrict__ img, const float *__restrict__ scale, float *__restrict__ out, int N, int K,
                    int M, int ntt, int *status)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -578,7 +617,7 @@ prefill_q6k_kernel(const uint8_t *__restrict__ q6u, const __half *__restrict__ i
     auto bar = [&](int i) { return sbase + Q6_OFF_BAR + 8u * (uint32_t)i; };
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < NB; ++i) mbar_init(bar(Q6_FULL_B + i), 1), mbar_init(bar(Q6_EMPTY_B + i), 1);
+        for (int i = 0; i < Q6_NB; ++i) mbar_init(bar(Q6_FULL_B + i), 1), mbar_init(bar(Q6_EMPTY_B + i), 1);
         for (int i = 0; i < NA; ++i) mbar_init(bar(Q6_FULL_A + i), EXPAND_WARPS), mbar_init(bar(Q6_EMPTY_A + i), 1);
         for (int i = 0; i < 2; ++i) mbar_init(bar(Q6_ACC_FULL + i), 1), mbar_init(bar(Q6_ACC_EMPTY + i), DRAIN_WARPS);
         *abort_flag = 0;
@@ -597,20 +636,20 @@ prefill_q6k_kernel(const uint8_t *__restrict__ q6u, const __half *__restrict__ i
 
     if (warp == 0) {
         if (lane == 0) {
-            const __half *src = img + (size_t)tt * (K / KS) * 2 * (TN * KS);
+            const __nv_bfloat16 *src = img + (size_t)tt * (K / KS) * 3 * (TN * KS);
             int slot = 0;
             uint32_t phase = 1;
             for (int st = 0; st < nsb * NA; ++st) {
                 mbar_wait(bar(Q6_EMPTY_B + slot), phase, abort_flag, status);
-                mbar_expect_tx(bar(Q6_FULL_B + slot), 2 * B_BYTES);
-                bulk_g2s(sbase + (uint32_t)slot * SLOT_BYTES, src + (size_t)st * 2 * (TN * KS), 2 * B_BYTES, bar(Q6_FULL_B + slot));
-                if (++slot == NB) slot = 0, phase ^= 1;
+                mbar_expect_tx(bar(Q6_FULL_B + slot), Q6_SLOT);
+                bulk_g2s(sbase + (uint32_t)slot * Q6_SLOT, src + (size_t)st * 3 * (TN * KS), Q6_SLOT, bar(Q6_FULL_B + slot));
+                if (++slot == Q6_NB) slot = 0, phase ^= 1;
             }
         }
     } else if (warp == 1) {
         if (lane == 0) {
             const uint64_t b_desc0 = smem_desc(sbase, 128, 1024);
-            constexpr uint64_t U_SLOT = SLOT_BYTES >> 4, U_LO = B_BYTES >> 4, U_KK = 256 >> 4;
+            constexpr uint64_t U_SLOT = Q6_SLOT >> 4, U_X = B_BYTES >> 4, U_KK = 256 >> 4;
             int slot = 0;
             uint32_t b_phase = 0;
             for (int sb = 0; sb < nsb; ++sb) {
@@ -622,23 +661,24 @@ prefill_q6k_kernel(const uint8_t *__restrict__ q6u, const __half *__restrict__ i
                     mbar_wait(bar(Q6_FULL_B + slot), b_phase, abort_flag, status);
                     mbar_wait(bar(Q6_FULL_A + g), (uint32_t)(sb & 1), abort_flag, status);
                     tc_fence_after();
-                    const uint64_t bh = b_desc0 + (uint64_t)slot * U_SLOT;
-                    const uint32_t a0 = tmem_base + Q6_COL_A + (uint32_t)g * 64u;
+                    const uint64_t x0 = b_desc0 + (uint64_t)slot * U_SLOT, x1 = x0 + U_X, x2 = x1 + U_X;
+                    const uint32_t v_hi = tmem_base + Q6_COL_A + (uint32_t)g * 64u, v_lo = v_hi + 32;
+                    auto products = [&](uint32_t v, uint64_t x, bool first) {
 #pragma unroll
-                    for (int kk = 0; kk < KS / 16; ++kk) tc_mma_f16_ta(acc_d, a0 + 32 + kk * 8, bh + kk * U_KK, IDESC, kk != 0 ? 1u : 0u);
-#pragma unroll
-                    for (int kk = 0; kk < KS / 16; ++kk) tc_mma_f16_ta(acc_d, a0 + kk * 8, bh + U_LO + kk * U_KK, IDESC, 1u);
-#pragma unroll
-                    for (int kk = 0; kk < KS / 16; ++kk) tc_mma_f16_ta(acc_d, a0 + kk * 8, bh + kk * U_KK, IDESC, 1u);
+                        for (int kk = 0; kk < KS / 16; ++kk) tc_mma_f16_ta(acc_d, v + kk * 8, x + kk * U_KK, Q6_IDESC, first && kk == 0 ? 0u : 1u);
+                    };
+                    products(v_lo, x1, true), products(v_hi, x2, false);
+                    products(v_lo, x0, false), products(v_hi, x1, false);
+                    products(v_hi, x0, false);
                     tc_commit(bar(Q6_EMPTY_B + slot));
                     tc_commit(bar(Q6_EMPTY_A + g));
                     tc_commit(bar(Q6_ACC_FULL + buf));
-                    if (++slot == NB) slot = 0, b_phase ^= 1;
+                    if (++slot == Q6_NB) slot = 0, b_phase ^= 1;
                 }
             }
         }
     } else if (warp < WARP_DRAIN0) {
-        const int quarter = warp & 3, plane = (warp - WARP_EXPAND0) >> 2, r = quarter * 32 + lane;
+        const int quarter = warp & 3, plane = (warp - WARP_EXPAND0) >> 2;
         const uint32_t a_lane = tmem_base + ((uint32_t)(quarter * 32) << 16) + Q6_COL_A + (uint32_t)plane * 16u;
         const uint32_t w_quarter = sbase + Q6_OFF_W + (uint32_t)(quarter * 32) * Q6_RAW;
         const uint32_t meet = 1u + (uint32_t)quarter;  // named barrier of the quarter's two warps
@@ -679,7 +719,7 @@ prefill_q6k_kernel(const uint8_t *__restrict__ q6u, const __half *__restrict__ i
                         const uint32_t xw[4] = {X[o].x, X[o].y, X[o].z, X[o].w}, yw[4] = {Y[o].x, Y[o].y, Y[o].z, Y[o].w}, zw[4] = {Z[o].x, Z[o].y, Z[o].z, Z[o].w};
                         const int si = o + 4 * g2 + 2 * plane;  // scale byte within the half: o + 2 c
                         const uint32_t w8 = g2 ? (h ? scw.w : scw.y) : (h ? scw.z : scw.x);
-                        const __half2 sc = __half2half2(__int2half_rn((int)(int8_t)((w8 >> (8 * (si & 3))) & 0xFFu)));
+                        const __nv_bfloat162 sc = __float2bfloat162_rn((float)(int8_t)((w8 >> (8 * (si & 3))) & 0xFFu));
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
                             uint32_t q;
@@ -720,19 +760,19 @@ prefill_q6k_kernel(const uint8_t *__restrict__ q6u, const __half *__restrict__ i
                 tc_fence_after();
                 const uint32_t td = lane_base + (uint32_t)buf * 128u;
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
+                for (int c = 0; c < 64; c += 16) {
                     float va[16];
-                    tc_ld16(td + (uint32_t)c * 16u, va);
+                    tc_ld16(td + (uint32_t)c, va);
                     tc_wait_ld();
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) acc[c * 16 + i] = fmaf(d, va[i], acc[c * 16 + i]);
+                    for (int i = 0; i < 16; ++i) acc[c + i] = fmaf(d, va[i], acc[c + i]);
                 }
                 tc_fence_before();
                 warp_arrive(bar(Q6_ACC_EMPTY + buf));
             }
-            // sixteen quarters per chain of fp32 sums, the chains' sums in `out` (each element belongs to one thread): one chain over
-            // all of K = 14336 came out 2.9e-7 from 64 bits (2-norm), against 1.8e-7 of the digit planes
-            if ((sb & 3) == 3 && sb + 1 < nsb) {
+            // 32 quarters per chain of fp32 sums, the chains' sums in `out` (each element belongs to one thread).  4096 x 14336, distance from
+            // 64 bits (2-norm) and time of 500 rows: 16 quarters 1.23e-7, 420 us; 32 1.33e-7, 404 us; 64 1.60e-7, 394 us; one chain 2.8e-7
+            if ((sb & 7) == 7 && sb + 1 < nsb) {
                 float *at = dst;
 #pragma unroll
                 for (int c = 0; c < 64; c += 4) {
@@ -823,7 +863,7 @@ static int launch_prefill(smc_ctx *ctx, const float *x, const smc_q8act *a, cons
         dequant_q8_rows_kernel<<<(unsigned)((nquads + 255) / 256), 256, 0, s>>>(a->q, a->d, xd, nquads);
         x = xd;
     }
-    prefill_scale_kernel<<<M, 256, 0, s>>>(x, M, K, scale);
+    prefill_scale_kernel<<<M, 256, 0, s>>>(x, M, K, 10, scale);
     prefill_image_kernel<<<ntt * nsb, 256, 0, s>>>(x, M, K, scale, img, mimg);
     static bool attr_set = false;
     if (!attr_set) {
@@ -847,29 +887,31 @@ int smc_launch_prefill_q4k_q8(smc_ctx *ctx, const smc_q8act *a, const smc_weight
     return launch_prefill(ctx, nullptr, a, w, out, a->M, s, scratch_locked);
 }
 
-// fp32 rows over Q6_K where this kernel is the faster one.  A wave of tiles takes 22 ns per element of K whatever the tiles hold; the
-// digit planes on mma.sync take 5.5e-5 ns per element of K, weight row and activation row: the lines cross at about 410 000
-// outputs per wave.  Measured, digit planes -> here, us: 4096 x 4096 with 100 rows 109 -> 110, 200 rows 199 -> 112; 1024 x 4096
-// with 300 rows 90 -> 112, 500 rows 136 -> 112; 8192 x 28672 with 64 rows 830 -> 647, 600 rows (three waves) 7397 -> 1771.
+// fp32 rows over Q6_K where this kernel is the faster one.  A wave of tiles takes about 28 ns per element of K whatever the tiles hold; the
+// digit planes on mma.sync take 5.5e-5 ns per element of K, weight row and activation row, in steps of 16 rows: the lines cross at
+// about 500 000 outputs per wave.  Measured, digit planes -> here, us: 3584 x 4096 with 137 rows 121 -> 129, 143 rows 130 -> 129, 168
+// rows 152 -> 128; 1024 x 4096 with 479 rows 125 -> 130, 499 rows 135 -> 130; 3584 x 14336 with 143 rows 428 -> 382; 8192 x 28672
+// with 65 rows 942 -> 757, 600 rows (three waves) 7397 -> 2120.
 bool smc_prefill_q6k_supported(const smc_ctx *ctx, const smc_weight *w, int M)
 {
     if (w->dtype != SMC_Q6_K || w->N % TM || w->K % 256 || M < 64 || !w->q6u) return false;
     const long long tiles = (long long)(w->N / TM) * ((M + TN - 1) / TN), waves = (tiles + ctx->sm_count - 1) / ctx->sm_count;
-    return (long long)w->N * M >= 450000 * waves;
+    return (long long)w->N * M >= 500000 * waves;
 }
 
 // Bytes that hold the image and scales of every call with at most `values` = M K activations: M >= 64 rows (K >= 256) are at most
 // doubled by rounding them up to whole tiles, and a row has a scale of four bytes.
-size_t smc_prefill_q6k_scratch(size_t values) { return 2 * values * 2 * sizeof(__half) + values / 32; }
+size_t smc_prefill_q6k_scratch(size_t values) { return 2 * values * 3 * sizeof(__nv_bfloat16) + values / 32; }
 
 // scratch: smc_prefill_q6k_scratch(M K) bytes; the caller holds mu_scratch until this returns
 int smc_launch_prefill_q6k(smc_ctx *ctx, const float *x, const smc_weight *w, float *out, int M, void *scratch, cudaStream_t s)
 {
     const int N = w->N, K = w->K, ntt = (M + TN - 1) / TN;
-    __half *img = static_cast<__half *>(scratch);
-    float *scale = reinterpret_cast<float *>(img + (size_t)ntt * TN * K * 2);
-    prefill_scale_kernel<<<M, 256, 0, s>>>(x, M, K, scale);
-    prefill_image_kernel<<<ntt * (K / 256), 256, 0, s>>>(x, M, K, scale, img, nullptr);
+    __nv_bfloat16 *img = static_cast<__nv_bfloat16 *>(scratch);
+    float *scale = reinterpret_cast<float *>(img + (size_t)ntt * TN * K * 3);
+    // rows at 2^64: far from bfloat16's smallest numbers and from overflow (64 + 12 of v + 16 of d + 15 of K)
+    prefill_scale_kernel<<<M, 256, 0, s>>>(x, M, K, 64, scale);
+    prefill_q6k_image_kernel<<<ntt * (K / 256), 256, 0, s>>>(x, M, K, scale, img);
     SMC_CUDA(ctx, cudaFuncSetAttribute(prefill_q6k_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Q6_SMEM));
     prefill_q6k_kernel<<<(N / TM) * ntt, THREADS, Q6_SMEM, s>>>(w->q6u, img, scale, out, N, K, M, ntt, ctx->d_status);
     SMC_LAUNCH_CHECK(ctx);

@@ -135,10 +135,10 @@ def test_quantised_activations_at_prefill_sizes_run_on_the_tensor_cores(oracle, 
 
 
 @pytest.mark.parametrize("n,k,m", [
-    (7168, 256, 64),     # one block, half a token tile, the fewest outputs that come this way
-    (3584, 768, 128),    # rows that start inside a unit of eight blocks, fewer blocks than are folded at once
-    (3584, 2048, 129),   # a token tile of one
-    (2304, 4352, 200),   # 17 blocks: a last chain of one block
+    (7936, 256, 64),     # one block, half a token tile, the fewest outputs that come this way
+    (3968, 768, 128),    # rows that start inside a unit of eight blocks, fewer blocks than are folded at once
+    (3968, 2048, 129),   # a token tile of one
+    (2560, 4352, 200),   # 17 blocks: a last chain of one block
     (8192, 1024, 300),   # two waves of tiles
 ])
 def test_q6k_fp32_rows_on_the_tensor_cores(oracle, cuda, dev, n, k, m):
@@ -169,7 +169,7 @@ def test_q6k_fp32_rows_on_the_tensor_cores(oracle, cuda, dev, n, k, m):
     live = [i for i in range(m) if i != 3]
     err = [float(np.linalg.norm(((y - want) / np.linalg.norm(want, axis=1, keepdims=True).clip(1e-30))[live])) for y in (got, planes)]
     print(f"{n}x{k}, {m} rows: error {err[0]:.2e}, digit planes {err[1]:.2e}")
-    assert err[0] <= 1.25 * err[1]  # both are sums of roundings: a quarter more than what differs with the order
+    assert err[0] <= err[1]
     cuda.release(w)
 
 
@@ -183,12 +183,12 @@ def test_host_threads_on_one_context_and_stream(oracle):
 
     cases = []
     raw4 = oracle.quantize(Q4_K, synth.normal("threads", "w4", (256, 512), 0.02))
-    raw6 = oracle.quantize(Q6_K, synth.normal("threads", "w6", (7168, 256), 0.02))
+    raw6 = oracle.quantize(Q6_K, synth.normal("threads", "w6", (7936, 256), 0.02))
     wb = synth.normal("threads", "wb", (256, 512), 0.02)
 
     def weights(ctx):
         b = torch.from_numpy(wb).cuda().to(torch.bfloat16).view(torch.uint8).reshape(-1)
-        return {"q4": ctx.register(raw4, Q4_K, 256, 512), "q6": ctx.register(raw6, Q6_K, 7168, 256),
+        return {"q4": ctx.register(raw4, Q4_K, 256, 512), "q6": ctx.register(raw6, Q6_K, 7936, 256),
                 "bf16": ctx.register_dev(b, ops.QuantDType.BF16, 256, 512, repack=False)}
 
     for name, k, mode in (("q4", 512, ops.Mode.ACT_F32), ("q6", 256, ops.Mode.ACT_F32), ("q4", 512, ops.Mode.ACT_Q8), ("bf16", 512, ops.Mode.ACT_BF16)):
@@ -245,9 +245,9 @@ def _capture(body):
 
 
 @pytest.mark.parametrize("warm,then", [
-    ((200, 3584, 256), [(200, 3584, 256), (126, 3584, 256), (125, 3584, 256), (64, 3584, 256), (2, 3584, 256)]),  # both sides of the line between the forms
-    ((63, 7296, 512), [(64, 7168, 256), (63, 7296, 512)]),   # first the digit planes
-    ((201, 2304, 4352), [(129, 3584, 6656)]),                # fewer values, but as many tiles of rows of a longer K
+    ((200, 3584, 256), [(200, 3584, 256), (140, 3584, 256), (139, 3584, 256), (64, 3584, 256), (2, 3584, 256)]),  # both sides of the line between the forms
+    ((63, 8192, 512), [(64, 7936, 256), (63, 8192, 512)]),   # first the digit planes
+    ((201, 2560, 4352), [(129, 3968, 6656)]),                # fewer values, but as many tiles of rows of a longer K
 ])
 def test_fp32_rows_over_q6k_reserve_for_both_forms(oracle, warm, then):
     """SMC_ACT_F32 over Q6_K takes one of two forms by M and N.  A call with no more values and no more outputs than an earlier
@@ -274,3 +274,30 @@ def test_fp32_rows_over_q6k_reserve_for_both_forms(oracle, warm, then):
         ctx.release(w)
     assert ctx.device_status() == 0
     ctx.close()
+
+
+@pytest.mark.parametrize("outlier", [1e4, 1e5, 1e12, 1e30])
+def test_q6k_fp32_rows_with_an_element_far_above_the_others(oracle, cuda, dev, outlier):
+    """A row's largest element lies where the weights are zero: the others keep the accuracy that they have in the digit planes,
+    whose scales are per 32 elements.  Bounds as in test_q6k_fp32_rows_on_the_tensor_cores."""
+    import torch
+
+    n, k, m = 3968, 768, 129
+    raw = np.array(oracle.quantize(Q6_K, synth.normal("prefill", f"w6o{n}x{k}", (n, k), 0.02)), np.uint8).reshape(n, k // 256, 210)
+    raw[:, 1, 192 + 4:192 + 6] = 0  # scales of elements 64 .. 95 of the second block
+    raw = np.ascontiguousarray(raw.reshape(-1))
+    x = synth.normal("prefill", f"x6o{m}x{k}", (m, k))
+    rest = x.copy()
+    rest[:, 256 + 64:256 + 96] = 0.0
+    x[::2, 256 + 70] = outlier
+    w = cuda.register(raw, Q6_K, n, k)
+    got = dev.qmatmul(to_dev(x), w, ops.Mode.ACT_F32).cpu().numpy()
+    planes = torch.cat([dev.qmatmul(to_dev(x[i:i + 32]), w, ops.Mode.ACT_F32) for i in range(0, m - 1, 32)]).cpu().numpy()
+    assert cuda.device_status() == 0
+    want = x.astype(np.float64) @ oracle.dequantize(Q6_K, raw, n * k).reshape(n, k).astype(np.float64).T
+    bound = row_norm_bound(oracle, Q6_K, raw, n, k, rest)  # the outlier does not widen it
+    assert np.all(np.abs(got - want) <= bound), float(np.max(np.abs(got - want) / bound))
+    err = [float(np.linalg.norm((y - want[:m - 1]) / np.linalg.norm(want[:m - 1], axis=1, keepdims=True))) for y in (got[:m - 1], planes)]
+    print(f"outlier {outlier:.0e}: error {err[0]:.2e}, digit planes {err[1]:.2e}")
+    assert err[0] <= err[1]
+    cuda.release(w)
