@@ -21,7 +21,6 @@
 namespace {
 
 constexpr int LPK = 8;          // lanes per key
-constexpr int MAXG = 8;         // query heads per KV head handled by one CTA pass
 constexpr int SPLIT_THREADS = 128;
 
 constexpr int MERGE_MAX_SPLITS = 128;
@@ -112,8 +111,21 @@ __device__ __forceinline__ void merge_heads(const float *rec0, float *out0, int 
 // 32-element block; bytes become floats through a PRMT + FADD pair, and the block scale multiplies the lane's partial
 // dot (keys) or the softmax weight (values) once instead of every element: what ScaledDotProductFlashQ8_0*
 // (AttentionKernels.cs:489-813) computes, at a quarter of the fp32 cache's bytes.
-template <int DPL, int G, bool Q8>  // DPL = dims per lane = headDim / 8, G = query heads per KV head
-__global__ void __launch_bounds__(SPLIT_THREADS, Q8 && G <= 2 ? 4 : 1) sdpa_decode_split_kernel(
+//
+// A key's K and V pieces are requested some iterations before their use: with a few CTAs of four warps per SM the sweep waited for
+// one key at a time.  The registers of the look-ahead cost resident CTAs, so each variant has two forms with the same order of sums:
+// DEEP for grids that run in few waves, and one with more CTAs per SM (split_forms_deep holds the line between them).
+struct SplitForm {
+    int ahead, ctas;  // keys requested ahead; CTAs per SM that the registers are held to
+};
+__host__ __device__ constexpr SplitForm split_form(int dpl, int G, bool q8, bool deep)
+{
+    if (deep) return {q8 ? 3 : 1, dpl == 16 ? (q8 || G == 1 ? 4 : 3) : G == 1 ? (q8 ? 6 : 7) : q8 ? 4 : 5};
+    if (dpl == 16 && G == 1) return q8 ? SplitForm{1, 8} : SplitForm{0, 7};
+    return G == 1 ? SplitForm{1, 9} : SplitForm{0, dpl == 16 ? 4 : 7};
+}
+template <int DPL, int G, bool Q8, bool DEEP>  // DPL = dims per lane = headDim / 8, G = query heads per CTA
+__global__ void __launch_bounds__(SPLIT_THREADS, split_form(DPL, G, Q8, DEEP).ctas) sdpa_decode_split_kernel(
     const float *__restrict__ q, const void *__restrict__ kc_, const void *__restrict__ vc_, const __half *__restrict__ kd,
     const __half *__restrict__ vd, float *part, int heads, int kvHeads, int kvLen, int maxSeq, float scale, int splits,
     float *__restrict__ out, unsigned *tickets, int hshare)
@@ -160,14 +172,9 @@ __global__ void __launch_bounds__(SPLIT_THREADS, Q8 && G <= 2 ? 4 : 1) sdpa_deco
 
     // every lane group runs the same number of iterations so the shuffles below stay converged
     const int iters = k1 > k0 ? (k1 - k0 + ngroups - 1) / ngroups : 0;
-    // A key's K and V pieces are requested AHEAD iterations before they are used: with a few CTAs of four warps per SM the
-    // sweep waited for one key at a time.  The order of the sums is untouched.  Q8_0 rows, three keys ahead, registers capped so that
-    // the launcher's 512 CTAs still run in one wave: 32 sequences over 1501 rows each (8 KV heads of 128, 28 layers, the whole
-    // step) 2870 -> 2642 us.  fp32 rows are four times the bytes a key: one ahead, 1004 -> 993 us a step of the 28-layer shape
-    // and 2220 -> 2186 us of the 8B shape at 2048 positions; two ahead cost 2 % (fewer CTAs per SM), none 1 to 3 %.
-    constexpr int AHEAD = Q8 ? 3 : 1, PIECES = Q8 ? DPL / 4 : DPL;
-    uint32_t kw[AHEAD][PIECES], vw[AHEAD][PIECES];
-    __half kh[AHEAD], vh[AHEAD];  // block scales of the lane's dims (Q8)
+    constexpr int AHEAD = split_form(DPL, G, Q8, DEEP).ahead, SLOTS = AHEAD ? AHEAD : 1, PIECES = Q8 ? DPL / 4 : DPL;
+    uint32_t kw[SLOTS][PIECES], vw[SLOTS][PIECES];
+    __half kh[SLOTS], vh[SLOTS];  // block scales of the lane's dims (Q8)
     auto fetch = [&](int it, int u) {
         const int j = k0 + it * ngroups + gid, jj = j < k1 ? j : k0;
         if (Q8) {
@@ -199,37 +206,50 @@ __global__ void __launch_bounds__(SPLIT_THREADS, Q8 && G <= 2 ? 4 : 1) sdpa_deco
 #pragma unroll
     for (int u = 0; u < AHEAD; ++u)
         if (u < iters) fetch(u, u);
-    for (int it0 = 0; it0 < iters; it0 += AHEAD) {
+    for (int it0 = 0; it0 < iters; it0 += SLOTS) {
 #pragma unroll
-        for (int u = 0; u < AHEAD; ++u) {
+        for (int u = 0; u < SLOTS; ++u) {
             const int it = it0 + u;
             if (it >= iters) break;
+            if (AHEAD == 0) fetch(it, u);
             const bool live = k0 + it * ngroups + gid < k1;
             const float dk = Q8 ? __half2float(kh[u]) : 1.f, dv = Q8 ? __half2float(vh[u]) : 1.f;
-            float dot[G], r[DPL];
-            widen(kw[u], r);
+            auto dot_of = [&](int g, const float (&k)[DPL]) {
+                float dot = 0.f;
 #pragma unroll
-            for (int g = 0; g < G; ++g) {
-                dot[g] = 0.f;
+                for (int d = 0; d < DPL; ++d) dot = fmaf(qr[g][d], k[d], dot);
+                if (Q8) dot *= dk;
+                return smc_group_sum<LPK>(dot);
+            };
+            auto add_key = [&](int g, float dot, const float (&v)[DPL]) {
+                float s = dot * scale;
+                float mn = fmaxf(m[g], s);
+                float alpha = expf(m[g] - mn);  // exp(-inf) = 0 on the first key
+                float p = expf(s - mn);
+                l[g] = fmaf(l[g], alpha, p);
+                const float pv = Q8 ? p * dv : p;
 #pragma unroll
-                for (int d = 0; d < DPL; ++d) dot[g] = fmaf(qr[g][d], r[d], dot[g]);
-                if (Q8) dot[g] *= dk;
-                dot[g] = smc_group_sum<LPK>(dot[g]);
-            }
-            widen(vw[u], r);
-            if (it + AHEAD < iters) fetch(it + AHEAD, u);
-            if (live) {
+                for (int d = 0; d < DPL; ++d) o[g][d] = fmaf(pv, v[d], o[g][d] * alpha);
+                m[g] = mn;
+            };
+            if constexpr (AHEAD == 0) {
+                float kr[DPL], vr[DPL];
+                widen(kw[u], kr), widen(vw[u], vr);
 #pragma unroll
                 for (int g = 0; g < G; ++g) {
-                    float s = dot[g] * scale;
-                    float mn = fmaxf(m[g], s);
-                    float alpha = expf(m[g] - mn);  // exp(-inf) = 0 on the first key
-                    float p = expf(s - mn);
-                    l[g] = fmaf(l[g], alpha, p);
-                    const float pv = Q8 ? p * dv : p;
+                    const float dot = dot_of(g, kr);
+                    if (live) add_key(g, dot, vr);
+                }
+            } else {  // all dots first: K's registers are free for a later key while the weights are formed
+                float dot[G], r[DPL];
+                widen(kw[u], r);
 #pragma unroll
-                    for (int d = 0; d < DPL; ++d) o[g][d] = fmaf(pv, r[d], o[g][d] * alpha);
-                    m[g] = mn;
+                for (int g = 0; g < G; ++g) dot[g] = dot_of(g, r);
+                widen(vw[u], r);
+                if (it + AHEAD < iters) fetch(it + AHEAD, u);
+                if (live) {
+#pragma unroll
+                    for (int g = 0; g < G; ++g) add_key(g, dot[g], r);
                 }
             }
         }
@@ -346,26 +366,42 @@ __global__ void kv_append_kernel(const float *__restrict__ k, const float *__res
     vc[dst] = v[t];
 }
 
+// Which form a grid takes.  Full SMs run at one rate whichever form fills them, so a form costs its waves times the CTAs it keeps on
+// an SM, and fp32 rows take the cheaper one.  Q8_0 rows with look-ahead gain only while one wave holds the grid.  Measured, 2048
+// positions, us a call, deep / other form (no look-ahead and 4 to 11 CTAs per SM before there were two):
+//   fp32, heads of 128, two per CTA (3 / 4 CTAs per SM): 432 CTAs 60 / 65 (65), 448 CTAs 124 / 97 (97), 512 139 / 101 (101),
+//         608 240 / 274 (274), 768 289 / 355 (355), 1024 362 / 323 (322)
+//   fp32, heads of 128, one per CTA (4 / 7): 576 CTAs 190 / 240 (253), 896 329 / 311 (313), 1216 465 / 566 (566), 2048 691 / 663 (684)
+//   fp32, heads of 64, two (5 / 7): 608 CTAs 95 / 115 (112), 768 162 / 120 (116); one (7 / 9): 576 107 / 106 (156), 896 144 / 154
+//         (174), 1216 225 / 197 (202), 2048 308 / 343 (377)
+//   Q8_0, heads of 128, one (4 / 8): 576 CTAs 102 / 106 (178), 896 188 / 134 (193), 2048 391 / 256 (432)
+//   Q8_0, heads of 64, two (4 / 7): 512 CTAs 90 / 113 (116), 608 157 / 127 (129), 1536 257 / 228 (236); one (6 / 9): 576 92 / 90 (140),
+//         896 162 / 106 (148)
+// Q8_0 heads of 128, two per CTA, fit four CTAs per SM with look-ahead as they did without it: one form, 512 CTAs 62 us (73).
+template <int DPL, int G, bool Q8>
+bool split_forms_deep(long long ctas, long long sms)
+{
+    const long long deep = split_form(DPL, G, Q8, true).ctas * sms, other = split_form(DPL, G, Q8, false).ctas * sms;
+    if (Q8) return ctas <= deep;
+    return (ctas + deep - 1) / deep * deep < (ctas + other - 1) / other * other;
+}
+
 template <int DPL, bool Q8>
 int launch_split_g(smc_ctx *ctx, int G, dim3 grid, size_t smem, cudaStream_t s, const float *q, const void *k,
                    const void *v, const __half *kd, const __half *vd, float *part, int heads, int kvHeads, int kvLen, int maxSeq,
                    float scale, int splits, float *out, unsigned *tickets, int hshare)
 {
-#define SMC_SPLIT_CASE(GV)                                                                                         \
-    case GV:                                                                                                       \
-        if (smem > 48 * 1024)                                                                                      \
-            cudaFuncSetAttribute(sdpa_decode_split_kernel<DPL, GV, Q8>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
-                                 (int)smem);                                                                       \
-        smc_launch_dep(ctx->use_pdl, sdpa_decode_split_kernel<DPL, GV, Q8>, grid, dim3(SPLIT_THREADS), smem, s, q, k, v, kd, vd, part, heads, \
-                       kvHeads, kvLen, maxSeq, scale, splits, out, tickets, hshare);        \
-        break;
-    switch (G) {
-        SMC_SPLIT_CASE(1)
-        SMC_SPLIT_CASE(2)
-        SMC_SPLIT_CASE(4)
-    default: return smc_fail(ctx, SMC_E_UNSUPPORTED, "sdpa_decode: %d query heads per KV head", G);
+    auto go = [&](auto kernel) {
+        smc_launch_dep(ctx->use_pdl, kernel, grid, dim3(SPLIT_THREADS), smem, s, q, k, v, kd, vd, part, heads, kvHeads, kvLen, maxSeq, scale, splits,
+                       out, tickets, hshare);
+    };
+    const long long ctas = (long long)grid.x * grid.y * grid.z;
+    if (G == 1) {
+        split_forms_deep<DPL, 1, Q8>(ctas, ctx->sm_count) ? go(sdpa_decode_split_kernel<DPL, 1, Q8, true>) : go(sdpa_decode_split_kernel<DPL, 1, Q8, false>);
+    } else {
+        if constexpr (Q8 && DPL == 16) go(sdpa_decode_split_kernel<DPL, 2, Q8, true>);
+        else split_forms_deep<DPL, 2, Q8>(ctas, ctx->sm_count) ? go(sdpa_decode_split_kernel<DPL, 2, Q8, true>) : go(sdpa_decode_split_kernel<DPL, 2, Q8, false>);
     }
-#undef SMC_SPLIT_CASE
     SMC_LAUNCH_CHECK(ctx);
     return SMC_OK;
 }
@@ -591,7 +627,7 @@ int smc_sdpa_decode_any(smc_ctx *ctx, const float *d_q, const void *d_k, const v
     const int hshare = Gall / G;
     const int kvReal = kvHeads;
     kvHeads *= hshare;  // virtual KV heads from here on
-    const bool split_ok = (headDim == 64 || headDim == 128) && (G == 1 || G == 2 || G == 4) &&
+    const bool split_ok = (headDim == 64 || headDim == 128) &&
                           ((reinterpret_cast<uintptr_t>(d_q) | reinterpret_cast<uintptr_t>(d_k) |
                             reinterpret_cast<uintptr_t>(d_v)) & 15) == 0;
     if (!split_ok) {

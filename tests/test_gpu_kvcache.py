@@ -246,3 +246,38 @@ def test_few_rows_over_a_long_cache(cuda, hd, heads, kvh, most, rows, length):
     reach = float(q.norm(dim=-1).max() * k.norm(dim=-1).max()) * scale
     assert (got.double() - exact).abs().max() <= 4 * 2.0 ** -24 * reach * v.abs().max()
     kv.Dispose()
+
+
+@pytest.mark.parametrize("hd,group,resident", [(128, 2, 3), (128, 1, 4), (64, 2, 5), (64, 1, 7)])
+@pytest.mark.parametrize("kind", [ops.KVCache.F32, ops.KVCache.Q8_0])
+@pytest.mark.parametrize("length", [1, 17, 40, 64])
+def test_decode_attention_forms_keep_the_bits(cuda, hd, group, resident, kind, length):
+    """One sequence's decode attention by the number of CTAs that the grid has: with and without keys requested ahead, on both sides of
+    the lines between the forms (`resident` CTAs per SM with look-ahead).  Up to 64 positions a CTA takes a whole cached head whatever
+    the batch, so every batch gives a sequence the same bits, and the ones of small batches are right (float64, a few roundings
+    of weights and sums)."""
+    import torch
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    most = 7 * sms + 1
+    g = torch.Generator(device="cuda").manual_seed(hd + group + length)
+    k, v = (torch.randn((most, length, 1, hd), generator=g, device="cuda") for _ in range(2))
+    q = torch.randn((most, 1, group, hd), generator=g, device="cuda")
+
+    def attend(lo, hi):
+        kv = ops.KVCache(cuda, hi - lo, 1, length, hd, kind)
+        kv.Update(k[lo:hi].contiguous(), v[lo:hi].contiguous())
+        out = kv.attention(q[lo:hi].contiguous(), hd ** -0.5)
+        torch.cuda.synchronize()
+        kv.Dispose()
+        return out
+
+    want = torch.cat([attend(lo, min(lo + 64, most)) for lo in range(0, most, 64)])
+    for n in sorted({resident * sms, resident * sms + 1, 4 * sms + 1, 6 * sms + 1, most}):
+        got = attend(0, n)
+        assert torch.equal(got.view(torch.int32), want[:n].view(torch.int32)), n
+    if kind == ops.KVCache.F32:
+        p = torch.softmax(torch.einsum("bgd,bld->bgl", q[:, 0].double(), k[:, :, 0].double()) * hd ** -0.5, -1)
+        exact = torch.einsum("bgl,bld->bgd", p, v[:, :, 0].double())
+        reach = float(q.norm(dim=-1).max() * k.norm(dim=-1).max()) * hd ** -0.5
+        assert (want[:, 0].double() - exact).abs().max() <= 4 * 2.0 ** -24 * max(reach, 8.0) * v.abs().max()
