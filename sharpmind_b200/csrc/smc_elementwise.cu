@@ -858,23 +858,22 @@ int smc_argmax_dev(smc_ctx *ctx, const float *d_logits, int rows, int n, int *d_
     if (!ctx || !d_logits || !d_out || rows < 0 || n <= 0) return smc_fail(ctx, SMC_E_INVALID, "argmax: bad arguments");
     if (rows == 0) return SMC_OK;
     const int chunks = (n + ARGMAX_CHUNK - 1) / ARGMAX_CHUNK;
-    {
-        // scratch for the chunk results and the per-row tickets, grown on demand (the first call of a larger
-        // shape allocates: make it outside stream capture).  Layout: values [rows x chunks] | indices | tickets.
-        std::lock_guard<std::mutex> lock(ctx->mu);
-        if (rows > ctx->argmax_rows || chunks > ctx->argmax_chunks) {
-            const int big_rows = rows > ctx->argmax_rows ? rows : ctx->argmax_rows;
-            const int big_chunks = chunks > ctx->argmax_chunks ? chunks : ctx->argmax_chunks;
-            if (ctx->d_argmax) {
-                cudaDeviceSynchronize();
-                cudaFree(ctx->d_argmax);
-                ctx->d_argmax = nullptr, ctx->argmax_rows = ctx->argmax_chunks = 0;
-            }
-            const size_t bytes = (size_t)big_rows * big_chunks * 8 + (size_t)big_rows * 4;
-            SMC_CUDA(ctx, cudaMalloc(&ctx->d_argmax, bytes));
-            SMC_CUDA(ctx, cudaMemset(ctx->d_argmax, 0, bytes));
-            ctx->argmax_rows = big_rows, ctx->argmax_chunks = big_chunks;
+    // scratch for the chunk results and the per-row tickets, grown on demand (the first call of a larger
+    // shape allocates: make it outside stream capture).  Layout: values [rows x chunks] | indices | tickets.  The lock is held until
+    // the launch is queued: another thread's larger call frees the buffer.
+    std::lock_guard<std::mutex> lock(ctx->mu);
+    if (rows > ctx->argmax_rows || chunks > ctx->argmax_chunks) {
+        const int big_rows = rows > ctx->argmax_rows ? rows : ctx->argmax_rows;
+        const int big_chunks = chunks > ctx->argmax_chunks ? chunks : ctx->argmax_chunks;
+        if (ctx->d_argmax) {
+            cudaDeviceSynchronize();
+            cudaFree(ctx->d_argmax);
+            ctx->d_argmax = nullptr, ctx->argmax_rows = ctx->argmax_chunks = 0;
         }
+        const size_t bytes = (size_t)big_rows * big_chunks * 8 + (size_t)big_rows * 4;
+        SMC_CUDA(ctx, cudaMalloc(&ctx->d_argmax, bytes));
+        SMC_CUDA(ctx, cudaMemset(ctx->d_argmax, 0, bytes));
+        ctx->argmax_rows = big_rows, ctx->argmax_chunks = big_chunks;
     }
     const size_t cap_cells = (size_t)ctx->argmax_rows * ctx->argmax_chunks;
     float *pv = reinterpret_cast<float *>(ctx->d_argmax);

@@ -204,7 +204,8 @@ def test_host_threads_on_one_context_and_stream(oracle):
             name, mode, xs = cases[i]
             try:
                 for x in xs:
-                    out[i] += [dev.qmatmul(x, w[name], mode) for _ in range(24)]
+                    y = [dev.qmatmul(x, w[name], mode) for _ in range(24)]
+                    out[i] += y + [dev.argmax(t) for t in y[::8]]
             except Exception as e:  # reported below, by the test's own thread
                 failed.append(e)
 
