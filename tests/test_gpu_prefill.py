@@ -38,6 +38,22 @@ def test_tc_matmul_matches_oracle(oracle, cuda, dev, n, k, m):
     cuda.release(w)
 
 
+@pytest.mark.parametrize("size", [1e-37, 1e-40, 3e37])
+def test_tc_matmul_rows_at_the_ends_of_the_range(oracle, cuda, dev, size):
+    """Rows whose scale would have no finite inverse, and very large ones: the bound of the mode at the row's own size, and a few
+    of fp32's smallest numbers where the sums fall below its normal range."""
+    n, k, m = 128, 512, 130
+    raw = oracle.quantize(Q4_K, synth.normal("prefill", "wends", (n, k), 0.02))
+    x = synth.normal("prefill", "xends", (m, k))
+    x[::3] = (x[::3].astype(np.float64) * size).astype(np.float32)
+    w = cuda.register(raw, Q4_K, n, k)
+    got = dev.qmatmul_tc(to_dev(x), w).cpu().numpy()
+    want = x.astype(np.float64) @ oracle.dequantize(Q4_K, raw, n * k).reshape(n, k).astype(np.float64).T
+    bound = row_norm_bound(oracle, Q4_K, raw, n, k, x) + k * 2.0 ** -149
+    assert np.all(np.abs(got - want) <= bound), float(np.max(np.abs(got - want) / bound))
+    cuda.release(w)
+
+
 @pytest.mark.parametrize("n,k", [(28672, 8192), (8192, 28672)])
 def test_tc_matmul_llama70b_shapes_sampled_rows(oracle, cuda, dev, n, k):
     """The benchmarked prefill shapes (Llama-3-70B FFN, 512 tokens): weights drawn and quantised on the device, sampled
@@ -142,10 +158,11 @@ def test_quantised_activations_at_prefill_sizes_run_on_the_tensor_cores(oracle, 
     (8192, 1024, 300),   # two waves of tiles
 ])
 def test_q6k_fp32_rows_on_the_tensor_cores(oracle, cuda, dev, n, k, m):
-    """fp32 rows over Q6_K at 64 rows and more: the weights' integer parts reach 4096 and travel as exact fp16 pairs.  Scales of
-    every size and sign (products above 2048 need the second half of the pair), rows of very different magnitude (one whose
+    """fp32 rows over Q6_K at 64 rows and more: the weights' integer parts reach 4096 and travel as exact bfloat16 pairs.  Scales of
+    every size and sign (products above 256 need the second half of the pair), rows of very different magnitude (one whose
     scale has no finite inverse) and a zero row;
-    against float64 over the dequantised weights at the bound of the mode, and no further off than the digit planes it replaces."""
+    against float64 over the dequantised weights at the bound of the mode, and no further off than the digit planes it replaces.
+    A row has the same bits whatever the batch it travels in, as long as that batch comes this way too."""
     import torch
 
     rs = np.random.default_rng(n + k + m)
@@ -162,11 +179,15 @@ def test_q6k_fp32_rows_on_the_tensor_cores(oracle, cuda, dev, n, k, m):
     assert cuda.device_status() == 0
     want = x.astype(np.float64) @ oracle.dequantize(Q6_K, raw, n * k).reshape(n, k).astype(np.float64).T
     bound = row_norm_bound(oracle, Q6_K, raw, n, k, x)
-    assert np.all(np.abs(got - want) <= bound + 1e-30), float(np.max(np.abs(got - want) / np.maximum(bound, 1e-30)))
+    bound += k * 2.0 ** -149  # sums of the smallest row round at fp32's smallest number
+    assert np.all(np.abs(got - want) <= bound), float(np.max(np.abs(got - want) / bound))
     assert np.all(got[3] == 0.0)
+    more = np.concatenate([x[5:37], x])  # other neighbours, another place in the tile, more rows
+    again = dev.qmatmul(to_dev(more), w, ops.Mode.ACT_F32).cpu().numpy()
+    assert np.array_equal(again[32:].view(np.uint32), got.view(np.uint32)) and np.array_equal(again[:32].view(np.uint32), got[5:37].view(np.uint32))
     # the digit planes take batches below 64 rows
     planes = torch.cat([dev.qmatmul(to_dev(x[i:i + 32]), w, ops.Mode.ACT_F32) for i in range(0, m, 32)]).cpu().numpy()
-    live = [i for i in range(m) if i != 3]
+    live = [i for i in range(m) if i not in (3, 4)]  # row 4: the planes' own scales fall below fp32's normal range
     err = [float(np.linalg.norm(((y - want) / np.linalg.norm(want, axis=1, keepdims=True).clip(1e-30))[live])) for y in (got, planes)]
     print(f"{n}x{k}, {m} rows: error {err[0]:.2e}, digit planes {err[1]:.2e}")
     assert err[0] <= err[1]

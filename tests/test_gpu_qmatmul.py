@@ -75,8 +75,9 @@ def test_qmatmul_modes_against_oracle(oracle, cuda, dev, dtype, n, k, m):
 
 
 def test_results_do_not_depend_on_batch_size(oracle, cuda, dev):
-    """Row r of an M-row call has the same bits for every M >= 2, whatever the other rows hold (both fast modes,
-    all formats); the one-row kernels use a different summation tree and agree within the parity bound."""
+    """Row r of an M-row call has the same bits for every M from 2 to 32, whatever the other rows hold (both fast modes, all
+    formats; larger batches where no tcgen05 kernel takes them: Q4_K leaves at 64 rows, fp32 rows over Q6_K where N and M fill the
+    device); the one-row kernels use a different summation tree and agree within the parity bound."""
     from sharpmind_b200.ops import Mode
 
     for dtype, n, k in ((Q8_0, 512, 1024), (Q4_K, 256, 4096), (Q6_K, 64, 14336)):
