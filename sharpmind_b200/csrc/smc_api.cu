@@ -240,7 +240,6 @@ void smc_destroy(smc_ctx *ctx)
     cudaFree(ctx->d_status);
     if (ctx->h_pin) cudaFreeHost(ctx->h_pin);
     smc_q8act_free(ctx->act);
-    smc_q8act_free(ctx->digits);
     cudaFree(ctx->d_fp32_rows);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -465,33 +464,41 @@ int smc_qmatmul_q8_dev(smc_ctx *ctx, const smc_q8act *a, const smc_weight *w, fl
     return smc_launch_gemv_q8(ctx, a, w, d_out, static_cast<cudaStream_t>(stream));
 }
 
-// Scratch of fp32 rows over M x K activations and N outputs (caller holds mu_scratch): the digit planes, and one block that
-// holds either the planes' products or the activation image of the tcgen05 form of Q6_K.  A call reserves for both forms
-// whichever it takes, so that after a first one no call with at most its values (M K) and outputs (M N) allocates.
+// The three digit planes of M K = `values` activations (3 M rows of one batch), each array on 256 bytes; base may be null.
+static size_t digit_planes(uint8_t *base, size_t values, smc_q8act *a)
+{
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        uint8_t *p = base + at;
+        at += (bytes + 255) & ~(size_t)255;
+        return p;
+    };
+    a->q = reinterpret_cast<int8_t *>(take(3 * values));
+    a->d = reinterpret_cast<float *>(take(3 * values / 32 * sizeof(float)));
+    a->sd = reinterpret_cast<float *>(take(3 * values / 32 * sizeof(float)));
+    a->s16 = reinterpret_cast<int16_t *>(take(3 * values / 16 * sizeof(int16_t)));
+    return at;
+}
+
+// Scratch of fp32 rows over M x K activations and N outputs (caller holds mu_scratch), one block that holds either the digit planes
+// and their products or the activation image of the tcgen05 form of Q6_K.  A call reserves for both whichever it takes, and
+// for the most values (M K) and outputs (M N) of any call before it: one that has no more of either does not allocate.
 static int reserve_fp32_rows(smc_ctx *ctx, const smc_weight *w, int M)
 {
-    const size_t values = (size_t)M * w->K;
-    if (!ctx->digits || ctx->digits_cap < 3 * values) {
-        if (ctx->digits) {  // growing allocates: make the first call of a new size outside stream capture
-            cudaDeviceSynchronize();
-            smc_q8act_free(ctx->digits);
-            ctx->digits = nullptr, ctx->digits_cap = 0;
-        }
-        const int rc = smc_q8act_alloc(ctx, 3 * M, w->K, &ctx->digits);
-        if (rc) return rc;
-        ctx->digits_cap = 3 * values;
-    }
-    size_t block = (size_t)3 * M * w->N * sizeof(float);
-    if (ctx->has_q6k || w->q6u) block = std::max(block, smc_prefill_q6k_scratch(values));  // a context without such weights needs no image
-    if (ctx->fp32_rows_cap < block) {
+    const size_t values = std::max(ctx->fp32_values, (size_t)M * w->K), outputs = std::max(ctx->fp32_outputs, (size_t)M * w->N);
+    smc_q8act a;
+    size_t bytes = digit_planes(nullptr, values, &a) + 3 * outputs * sizeof(float);
+    if (ctx->has_q6k || w->q6u) bytes = std::max(bytes, smc_prefill_q6k_scratch(values));  // a context without such weights needs no image
+    if (bytes > ctx->fp32_rows_cap) {  // growing allocates: make the first call of a new size outside stream capture
         if (ctx->d_fp32_rows) {
             cudaDeviceSynchronize();
             cudaFree(ctx->d_fp32_rows);
-            ctx->d_fp32_rows = nullptr, ctx->fp32_rows_cap = 0;
+            ctx->d_fp32_rows = nullptr, ctx->fp32_rows_cap = ctx->fp32_values = ctx->fp32_outputs = 0;
         }
-        SMC_CUDA(ctx, cudaMalloc(&ctx->d_fp32_rows, block));
-        ctx->fp32_rows_cap = block;
+        SMC_CUDA(ctx, cudaMalloc(&ctx->d_fp32_rows, bytes));
+        ctx->fp32_rows_cap = bytes;
     }
+    ctx->fp32_values = values, ctx->fp32_outputs = outputs;
     return SMC_OK;
 }
 
@@ -506,12 +513,13 @@ static int qmatmul_f32_digits(smc_ctx *ctx, const float *d_in, const smc_weight 
     int rc;
     if ((rc = reserve_fp32_rows(ctx, w, M))) return rc;
     if (smc_prefill_q6k_supported(ctx, w, M)) return smc_launch_prefill_q6k(ctx, d_in, w, d_out, M, ctx->d_fp32_rows, s);
-    smc_q8act *a = ctx->digits;
-    float *products = static_cast<float *>(ctx->d_fp32_rows);
-    a->max_rows = (int)(ctx->digits_cap / w->K), a->max_k = w->K;  // the same allocation (digits_cap values), seen with this K
     // the planes are 3 M rows of one batch: the weights are read once for all three
-    if ((rc = smc_launch_quantize_q8_digits(ctx, d_in, M, w->K, a, s))) return rc;
-    if ((rc = smc_launch_gemv_q8(ctx, a, w, products, s))) return rc;
+    smc_q8act a;
+    uint8_t *base = static_cast<uint8_t *>(ctx->d_fp32_rows);
+    float *products = reinterpret_cast<float *>(base + digit_planes(base, (size_t)M * w->K, &a));
+    a.max_rows = 3 * M, a.max_k = w->K;
+    if ((rc = smc_launch_quantize_q8_digits(ctx, d_in, M, w->K, &a, s))) return rc;
+    if ((rc = smc_launch_gemv_q8(ctx, &a, w, products, s))) return rc;
     return smc_launch_sum3(ctx, products, d_out, (long long)M * w->N, s);
 }
 

@@ -87,10 +87,8 @@ struct smc_ctx {
     const void *pin_seen[4] = {nullptr, nullptr, nullptr, nullptr};  // host buffers lately classified as page-locked or not (under mu)
     bool pin_is[4] = {false, false, false, false};
     unsigned pin_next = 0;
-    smc_q8act *digits = nullptr;       // the three int8 digit planes of fp32 activations, stacked as 3 M rows (SMC_ACT_F32)
-    size_t digits_cap = 0;             // values it holds
-    void *d_fp32_rows = nullptr;       // their products [3 M, N], or the activation image of the tcgen05 form of Q6_K
-    size_t fp32_rows_cap = 0;
+    void *d_fp32_rows = nullptr;       // SMC_ACT_F32: three int8 digit planes (3 M rows) and their products [3 M, N], or the image of Q6_K's tcgen05 form
+    size_t fp32_rows_cap = 0, fp32_values = 0, fp32_outputs = 0;  // its bytes; the most values (M K) and outputs (M N) that it was sized for
     std::atomic<bool> has_q6k{false};  // a repacked Q6_K weight was registered: the block above is also sized for the image
     int f32_digits = 1;                // that path on (0: the CUDA-core kernel at every batch size)
     int f32_digits_row_mb = 32;        // one row: K-quant matrices of at least this many MB take that path too (0: never)
