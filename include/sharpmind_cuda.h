@@ -25,6 +25,10 @@
  * smc_sdpa_decode_dev, smc_argmax_dev, smc_decode_step, smc_forward_last_logits) reuse those buffers in stream
  * order: all such calls on one context must go to ONE stream (or be ordered by events).  Work that is to run
  * concurrently on several streams takes one context per stream.
+ * Such a buffer grows with the first call that needs more of it, after a device-wide synchronisation: make that call outside
+ * stream capture, and capture again what was captured over the old buffer, which is freed.  SMC_ACT_F32 for M > 1 over Q6_K and
+ * Q8_0 needs more when M * K or M * N is larger than in any earlier such call, whichever of its kernels the call takes; Q4_K has
+ * a buffer of its own from 64 rows on (rows rounded up to 128), so its smaller batches need a first call too.
  */
 #ifndef SHARPMIND_CUDA_H
 #define SHARPMIND_CUDA_H
@@ -104,10 +108,13 @@ SMC_API const char *smc_last_error(smc_ctx *ctx);
  *                           activation rows (d * q is exact in its fp16 pairs; same parity bound as the int8 kernels, other
  *                           summation order); 0: the int8 mma.sync kernels at every batch size
  *   "f32_prefill_int8_digits"  1 (default): SMC_ACT_F32 with two rows and more, where no tcgen05 kernel takes the format
- *                           or shape, splits the fp32 rows into three int8 digit planes (fp32 accuracy) and runs the int8
+ *                           or shape (Q4_K with N % 128 == 0 from 64 rows; Q6_K with N % 128 == 0 from 64 rows where N * M fills the
+ *                           device, see smc_prefill.cu), splits the fp32 rows into three int8 digit planes (fp32 accuracy) and runs the int8
  *                           tensor-core kernels once per plane (the planes live in the context's scratch, like the
  *                           SMC_ACT_Q8 activations of a several-row call); 0: the CUDA-core kernel at every batch size;
- *                           a value above 1: the row count to start from
+ *                           a value above 1: the row count to start from.  0 and a larger row count keep Q6_K off its tcgen05
+ *                           kernel too.  The three kernels add in different orders: a row agrees within the mode's bound
+ *                           across them, and bit for bit among the batches that one of them takes
  *   "f32_one_row_digits_min_mb"  one row in SMC_ACT_F32 takes the same path when the K-quant matrix holds at least this many
  *                           MB (default 32: its three digit rows as one small batch then beat the fp32 one-row kernel);
  *                           0: never
@@ -122,7 +129,7 @@ SMC_API const char *smc_last_error(smc_ctx *ctx);
  *                           0 (default) never (then the kernel that fetches its fragments from global memory runs; the
  *                           two add a row's blocks in different orders: results agree within the mode's bound, not
  *                           bit for bit)
- * Results do not depend on any of them.  SMC_E_INVALID for an unknown name. */
+ * No option takes results out of their bounds.  SMC_E_INVALID for an unknown name. */
 SMC_API int smc_set_option(smc_ctx *ctx, const char *name, int value);
 /* QuantizationOps.GetRawTensorByteCount for a [N, K] tensor (QuantizationOps.cs:15-72); -1 if dtype unknown. */
 SMC_API int64_t smc_raw_tensor_bytes(int dtype, int64_t N, int64_t K);

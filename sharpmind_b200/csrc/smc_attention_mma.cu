@@ -296,8 +296,12 @@ __global__ void __launch_bounds__(128 * HPC) sdpa_prefill_mma_kernel(const float
 //      weights from the CTA that made them through distributed shared memory, while the other warps stage V
 // Shared memory stays below half an SM's: with one CTA per SM fewer than 16 clusters of eight were resident at once, and the
 // 16 head pairs of a 32-head model took two waves.  What bounds it: step 1's MMAs and step 3's chain of 12 MMAs per tile.
+// (128 registers, 264 / 280 bytes spilled at head sizes 64 / 128, for two CTAs per SM.)
 // Six rows over 1021 keys, 32 heads on 8 KV heads of 128, one layer: 175 us in the kernel above,
 // 41 us here; the whole 32-layer pass 8.59 -> 4.32 ms.
+// Scores and weights of all of a CTA's tiles are kept in shared memory, which ends at 14 tiles: 3584 keys at head size 128, 1792 at 64.
+// Longer caches go back to the kernel above (3584 keys 109 us, 3585 583 us; 64: 1792 42 us, 1793 160 us), as do Q8_0 caches and
+// groups of an odd number of heads.
 constexpr int FEW_ROWS = 8;  // per cluster: rows 8 .. 15 of the MMAs are not used
 template <int HD>
 struct FewShape {
