@@ -267,6 +267,29 @@ def test_add_rmsnorm_q8_equals_separate_launches(dev, rows, n, with_add):
         dev.add_rmsnorm_q8(to_dev(np.zeros((2, 1000), np.float32)), None, to_dev(np.ones(1000, np.float32)), 1e-6, ops.Q8Act(ctx, 2, 1024))
 
 
+@pytest.mark.parametrize("n", [288, 992, 1024, 1056, 2048, 2080, 4064, 4096, 4128])
+def test_add_rmsnorm_q8_at_the_ends_of_its_register_forms(dev, n):
+    """Rows held in registers (up to 1024, 2048 and 4096 elements, whole or ragged) and longer ones: the bits of the separate kernels."""
+    import torch
+
+    from sharpmind_b200 import ops
+
+    ctx, rows = dev.ctx, 3
+    x, y = to_dev(synth.normal("gpue", f"arx{n}", (rows, n))), to_dev(synth.normal("gpue", f"ary{n}", (rows, n)))
+    w = to_dev(synth.normal("gpue", f"arw{n}", (n,), 0.1, 1.0))
+    for add in (y, None):
+        x1, x2, out = x.clone(), x.clone(), torch.empty_like(x)
+        if add is not None:
+            dev.add_(x1, add)
+        normed = dev.rmsnorm(x1, w, 1e-6)
+        want = ops.Q8Act(ctx, rows, n)
+        dev.quantize_q8(normed, want, n)
+        got = dev.add_rmsnorm_q8(x2, add, w, 1e-6, ops.Q8Act(ctx, rows, n), out=out)
+        assert torch.equal(x1, x2) and torch.equal(out, normed)
+        (wq, wd), (gq, gd) = want.read(), got.read()
+        assert np.array_equal(wq, gq) and np.array_equal(wd, gd)
+
+
 @pytest.mark.parametrize("rows,F", [(1, 3072), (5, 1024), (33, 14336), (300, 3072), (2, 32)])
 def test_swiglu_quantize_q8_equals_separate_launches(dev, rows, F):
     """SiLU(gate) * up and the Q8_0 row quantiser in one pass (16-byte accesses for batches, one lane per value for a
