@@ -123,8 +123,8 @@ SMC_API const char *smc_last_error(smc_ctx *ctx);
  *                           runs the gate as a launch of its own.  Same bits either way
  *   "prompt_attention_mma"  causal attention of a prompt chunk: 1 (default) bf16 tensor-core MMAs on operands split three
  *                           ways (fp32-grade accuracy), 0 the fp32 CUDA-core kernel
- *   "prompt_attention_heads_per_cta"  0 (default): a CTA of that kernel takes two query heads that share a KV head where
- *                           the model has them; 1: always one
+ *   "prompt_attention_heads_per_cta"  0 (default): the tcgen05 kernel, or the mma.sync kernel with two query heads that
+ *                           share a KV head per CTA; 1: the mma.sync kernel with one.  Same bits either way
  *   "small_batch_ring"      2..32 rows in SMC_ACT_Q8: weights through the bulk-copy ring for 1 Q4_K, 2 every format,
  *                           0 (default) never (then the kernel that fetches its fragments from global memory runs; the
  *                           two add a row's blocks in different orders: results agree within the mode's bound, not

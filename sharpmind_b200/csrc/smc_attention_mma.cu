@@ -11,7 +11,8 @@
 // while they are staged (rows padded to an odd multiple of 16 bytes: every ldmatrix is conflict free); Q is split
 // the same way once per CTA.  The score tile's accumulator layout is the A-operand layout of the next MMA for
 // 16-bit types, so P goes from registers to registers.  Online softmax per row as in the scalar kernel.
-// sm_100a runs mma.sync on its legacy tensor path; a tcgen05 version would keep S and O in tensor memory.
+// sm_100a runs mma.sync on its legacy tensor path.  smc_attention_tc.cu is the tcgen05 form, with the same bits; this kernel stays for calls of
+// one key tile, outputs off 16 bytes, one head per CTA (an option) and calls that find no room for the other's planes.
 #include <cuda_bf16.h>
 
 #include "smc_common.cuh"
@@ -516,6 +517,7 @@ static int launch_prefill_mma(smc_ctx *ctx, const float *q, const void *kc, cons
                               int T, int nh, int nkv, int hd, int pos0, int maxSeq, float scale, cudaStream_t s)
 {
     const int G = nh / nkv;
+    // the order matters: a few rows over a long fp32 cache, then the tcgen05 kernel; all of them give the same bits
     auto go = [&](auto kernel, int hpc) {
         const dim3 grid(nh / hpc, (T + QROWS - 1) / QROWS);
         const size_t ldb = (size_t)hd * 2 + 16;
@@ -536,6 +538,12 @@ static int launch_prefill_mma(smc_ctx *ctx, const float *q, const void *kc, cons
         else few(sdpa_few_rows_kernel<64>, FewShape<64>::CS, FewShape<64>::SMEM);
         SMC_LAUNCH_CHECK(ctx);
         return SMC_OK;
+    }
+    // More than one tile of keys: tcgen05, two launches.  16 heads of 128: 20 rows (one tile) 10.8 us here, 13.1 there; 33 rows of 4 heads
+    // 16.0 / 13.8; 64 rows of 32 heads 18.0 / 14.3; 100 rows behind 1900 keys of a Q8_0 cache 398 / 149; 2048 rows 362 / 164.
+    if (tiles > 1 && ctx->attn_hpc != 1 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+        const int rc = smc_launch_sdpa_prefill_tc(ctx, q, kc, vc, kd, vd, out, T, nh, nkv, hd, pos0, maxSeq, scale, s);
+        if (rc != SMC_E_UNSUPPORTED) return rc;  // else there is no room for the planes (a first call under capture, a very long cache)
     }
     if (kd) {
         if (hd == 128) two ? go(sdpa_prefill_mma_kernel<128, 2, true>, 2) : go(sdpa_prefill_mma_kernel<128, 1, true>, 1);

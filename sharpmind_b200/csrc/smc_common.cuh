@@ -105,6 +105,9 @@ struct smc_ctx {
     int mt_ring = 0;                              // 2..32 rows, weights through the bulk-copy ring: 0 never, 1 Q4_K, 2 every format
     void *d_argmax = nullptr;          // chunk results and tickets of the argmax
     int argmax_rows = 0, argmax_chunks = 0;
+    std::mutex mu_attn;                // guards d_attn_planes, until the launches that use it are queued
+    void *d_attn_planes = nullptr;     // keys and values of a prompt's attention as bfloat16 planes
+    size_t attn_planes_cap = 0;
     void *d_prefill = nullptr;         // activation image of the tensor-core matmul
     size_t prefill_cap = 0;
     float *d_attn_part = nullptr;      // split-KV partial results
@@ -165,6 +168,8 @@ int smc_launch_prefill_q4k_q8(smc_ctx *, const smc_q8act *a, const smc_weight *,
 bool smc_mma_supported(const smc_weight *, int M);
 bool smc_mt_supported(const smc_weight *, int M);
 bool smc_sdpa_prefill_mma_supported(int nh, int nkv, int hd);
+int smc_launch_sdpa_prefill_tc(smc_ctx *, const float *q, const void *kc, const void *vc, const __half *kd, const __half *vd, float *out, int T, int nh, int nkv,
+                               int hd, int pos0, int maxSeq, float scale, cudaStream_t s);
 int smc_launch_sdpa_prefill_mma(smc_ctx *, const float *q, const float *kc, const float *vc, float *out, int T, int nh, int nkv, int hd,
                                 int pos0, int maxSeq, float scale, cudaStream_t s);
 int smc_launch_sdpa_prefill_mma_q8(smc_ctx *ctx, const float *q, const int8_t *kq, const __half *kd, const int8_t *vq, const __half *vd,

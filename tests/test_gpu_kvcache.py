@@ -281,3 +281,53 @@ def test_decode_attention_forms_keep_the_bits(cuda, hd, group, resident, kind, l
         exact = torch.einsum("bgl,bld->bgd", p, v[:, :, 0].double())
         reach = float(q.norm(dim=-1).max() * k.norm(dim=-1).max()) * hd ** -0.5
         assert (want[:, 0].double() - exact).abs().max() <= 4 * 2.0 ** -24 * max(reach, 8.0) * v.abs().max()
+
+
+@pytest.mark.parametrize("kind", ["f32", "q8_0"])
+@pytest.mark.parametrize("hd,heads,kvh", [(128, 4, 2), (64, 3, 1)])
+def test_prompt_attention_on_tcgen05_gives_the_bits_of_mma_sync(cuda, kind, hd, heads, kvh):
+    """The tcgen05 kernel against the mma.sync kernel (one head per CTA selects it), bit for bit: lengths at the borders of its key tiles
+    (32), chunks (64) and row tiles (128), starts that are no multiple of any, enough chunks for every barrier to go round, and scores that
+    keep raising the running maximum."""
+    import torch
+
+    scale = 1.0 / np.sqrt(hd)
+    for n0, s in ((0, 33), (0, 64), (31, 34), (0, 127), (0, 128), (0, 129), (17, 175), (70, 58), (500, 260), (1003, 18)):
+        kv = ops.KVCache(cuda, 1, kvh, n0 + s, hd, ops.KVCache.Q8_0 if kind == "q8_0" else ops.KVCache.F32)
+        ramp = np.linspace(0.2, 4.0, n0 + s, dtype=np.float32)[None, :, None, None]
+        k = to_dev(synth.normal("kvtc", f"k{hd}{n0}{s}", (1, n0 + s, kvh, hd)) * ramp)
+        v = to_dev(synth.normal("kvtc", f"v{hd}{n0}{s}", (1, n0 + s, kvh, hd)))
+        if n0:
+            kv.Update(k[:, :n0].contiguous(), v[:, :n0].contiguous())
+        kv.Update(k[:, n0:].contiguous(), v[:, n0:].contiguous())
+        q = to_dev(synth.normal("kvtc", f"q{hd}{n0}{s}", (1, s, heads, hd)) * 2.0)
+        got = kv.attention(q, scale)
+        cuda.set_option("prompt_attention_heads_per_cta", 1)
+        try:
+            want = kv.attention(q, scale)
+        finally:
+            cuda.set_option("prompt_attention_heads_per_cta", 0)
+        assert torch.equal(got.view(torch.int32), want.view(torch.int32)), (n0, s)
+        kv.Dispose()
+    assert cuda.device_status() == 0
+
+
+def test_prompt_attention_first_called_under_capture():
+    """Without room for its planes, and none to be had under capture, the call takes the mma.sync kernel: same bits."""
+    import torch
+
+    ctx = ops.CudaContext(0)
+    kv = ops.KVCache(ctx, 1, 2, 200, 128, ops.KVCache.F32)
+    kv.Update(*(to_dev(synth.normal("kvcap", n, (1, 200, 2, 128))) for n in "kv"))
+    q = to_dev(synth.normal("kvcap", "q", (1, 150, 4, 128)))
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = kv.attention(q, 128 ** -0.5)
+    graph.replay()
+    torch.cuda.synchronize()
+    want = kv.attention(q, 128 ** -0.5)
+    assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+    assert ctx.device_status() == 0
+    kv.Dispose()
+    ctx.close()
