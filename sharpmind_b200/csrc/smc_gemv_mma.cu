@@ -150,113 +150,6 @@ gemv_mma_q8_0_kernel(const int8_t *__restrict__ wq, const __half *__restrict__ w
     }
 }
 
-// Prompt-sized batches (hundreds of rows): the same sums with no shared-memory reduction.  The kernel above splits K
-// over the eight warps of a CTA (warp w takes the groups w, w + 8, ...) and adds the eight partial tiles in warp order;
-// with this many tokens there is parallelism enough without that split, so here one warp owns a 32 x 64 output tile and
-// walks the eight group classes one after the other, adding each finished class to its running total: the same
-// partial sums added in the same order, hence the same bits, without the barriers, the 64 KB of partial tiles and the
-// 8-way re-read that cost the split kernel a quarter of its instructions on K = 1024.  A CTA = eight token tiles of
-// one 32-row strip, which share the weight fragments through L1.
-__global__ void __launch_bounds__(256, 1)
-gemv_mma_q8_0_tile_kernel(const int8_t *__restrict__ wq, const __half *__restrict__ wd, const int8_t *__restrict__ xq,
-                          const float *__restrict__ xd, float *__restrict__ out, int N, int K, int M)
-{
-    constexpr int NT = 8;
-    smc_grid_dep_sync();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tg = lane & 3;
-    const int r0 = blockIdx.x * MMA_ROWS;
-    const int t0 = (blockIdx.y * (blockDim.x >> 5) + warp) * 8 * NT;  // the launcher picks 1..8 warps (token tiles) per CTA
-    if (t0 >= M) return;  // no barrier below
-    const int nb = K / 32, ngroups = nb / 4;
-    const int8_t *abase = wq + 8 * tg;
-    uint32_t aoff[4];  // 32-bit offsets (the launcher keeps N * K and M * K below 2^32): pointers would not fit the register file
-#pragma unroll
-    for (int j = 0; j < 4; ++j) aoff[j] = (uint32_t)min(r0 + (j >> 1) * 16 + g + (j & 1) * 8, N - 1) * (uint32_t)K;
-    const __half *drow = wd + (size_t)min(r0 + lane, N - 1) * nb;
-    const int8_t *bbase = xq + 8 * tg;
-    uint32_t boff[NT];  // rows past the end are clamped for loads and masked at the store
-#pragma unroll
-    for (int t = 0; t < NT; ++t) boff[t] = (uint32_t)min(t0 + 8 * t + g, M - 1) * (uint32_t)K;
-    const float *xrow[2] = {xd + (size_t)min(t0 + lane, M - 1) * nb, xd + (size_t)min(t0 + 32 + lane, M - 1) * nb};
-    float total[2][NT][4];
-#pragma unroll 1
-    for (int cls = 0; cls < MMA_WARPS; ++cls) {
-        float acc[2][NT][4];
-#pragma unroll
-        for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-            for (int t = 0; t < NT; ++t)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) acc[mt][t][i] = 0.f;
-#pragma unroll 1
-        for (int gi = cls; gi < ngroups; gi += MMA_WARPS) {
-            uint2 aq[4][4];
-#pragma unroll
-            for (int kb = 0; kb < 4; ++kb)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) aq[kb][j] = ldg8(abase + aoff[j] + (uint32_t)(gi * 4 + kb) * 32u);
-            const uint2 dwp = *reinterpret_cast<const uint2 *>(drow + gi * 4);
-            const float4 dxp[2] = {*reinterpret_cast<const float4 *>(xrow[0] + gi * 4), *reinterpret_cast<const float4 *>(xrow[1] + gi * 4)};
-            // the activation fragments of block kb + 1 are requested before block kb is multiplied (those of block 0 go
-            // out with the weight fragments above): one exposed load latency per group instead of five
-            uint2 bn[NT];
-#pragma unroll
-            for (int t = 0; t < NT; ++t) bn[t] = ldg8(bbase + boff[t] + (uint32_t)(gi * 4) * 32u);
-#pragma unroll
-            for (int kb = 0; kb < 4; ++kb) {
-                uint2 b[NT];
-                const uint2 (&a)[4] = aq[kb];
-#pragma unroll
-                for (int t = 0; t < NT; ++t) b[t] = bn[t];
-                if (kb < 3) {
-#pragma unroll
-                    for (int t = 0; t < NT; ++t) bn[t] = ldg8(bbase + boff[t] + (uint32_t)(gi * 4 + kb + 1) * 32u);
-                }
-                const uint32_t dword = (kb & 2) ? dwp.y : dwp.x;
-                float dxl[2];
-#pragma unroll
-                for (int x = 0; x < 2; ++x) dxl[x] = kb == 0 ? dxp[x].x : kb == 1 ? dxp[x].y : kb == 2 ? dxp[x].z : dxp[x].w;
-                float dw[2][2];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const uint32_t wv = __shfl_sync(0xffffffffu, dword, (j >> 1) * 16 + g + (j & 1) * 8);
-                    dw[j >> 1][j & 1] = smc_h2f((uint16_t)((kb & 1) ? (wv >> 16) : (wv & 0xFFFFu)));
-                }
-#pragma unroll
-                for (int t = 0; t < NT; ++t) {
-                    const float dx0 = __shfl_sync(0xffffffffu, dxl[t >> 2], 8 * (t & 3) + 2 * tg);
-                    const float dx1 = __shfl_sync(0xffffffffu, dxl[t >> 2], 8 * (t & 3) + 2 * tg + 1);
-#pragma unroll
-                    for (int mt = 0; mt < 2; ++mt) {
-                        int c[4];
-                        mma_s8(c, a[2 * mt].x, a[2 * mt + 1].x, a[2 * mt].y, a[2 * mt + 1].y, b[t].x, b[t].y);
-                        acc[mt][t][0] = fmaf((float)c[0], dw[mt][0] * dx0, acc[mt][t][0]);
-                        acc[mt][t][1] = fmaf((float)c[1], dw[mt][0] * dx1, acc[mt][t][1]);
-                        acc[mt][t][2] = fmaf((float)c[2], dw[mt][1] * dx0, acc[mt][t][2]);
-                        acc[mt][t][3] = fmaf((float)c[3], dw[mt][1] * dx1, acc[mt][t][3]);
-                    }
-                }
-            }
-        }
-        // the split kernel's fold: s = partial of warp 0; s += partial of warp 1; ...
-#pragma unroll
-        for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-            for (int t = 0; t < NT; ++t)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) total[mt][t][i] = cls == 0 ? acc[mt][t][i] : total[mt][t][i] + acc[mt][t][i];
-    }
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-        for (int t = 0; t < NT; ++t)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int tok = t0 + 8 * t + 2 * tg + (i & 1), row = r0 + mt * 16 + g + ((i >> 1) << 3);
-                if (row < N && tok < M) out[(size_t)tok * N + row] = total[mt][t][i];
-            }
-}
-
 // ------------------------------------------------------------------------------------------ Q4_K
 // GGUF blocks of 144 bytes: d, dmin (fp16), 12 packed scale / min bytes, 128 nibble bytes; the 32 bytes of
 // group gq hold sub-block 2*gq in the low nibbles and 2*gq + 1 in the high ones.  K % 256 == 0; a warp works
@@ -479,6 +372,291 @@ gemv_mma_q6_K_kernel(const uint8_t *__restrict__ q6u, const int8_t *__restrict__
     }
 }
 
+// ------------------------------------------------------------------------------------------ prompt sizes, Q8_0 and Q6_K
+// The same sums with no split over warps: with hundreds of tokens a warp owns an output tile of 32 rows x 8 NT tokens, walks the classes of
+// groups that the kernels above give to their eight (sixteen) warps one after the other, and adds each finished class to a running
+// total: the same partial sums added in the same order, hence the same bits.
+//
+// A CTA is two row warps x two token warps: 64 rows x 16 NT tokens.  Weights, activations and scales of a group (128 elements of Q8_0, 256
+// of Q6_K) come to shared memory by asynchronous copies, S groups in flight; a weight row or token takes an odd multiple of 16 bytes there,
+// so that an ldmatrix of eight of them is free of conflicts.  The tokens' scales are stored so that the 2 NT of a lane lie side by side:
+// a 16-byte load brings four.  Products of scales and fused multiply-adds are done two at a time (each half rounds as the scalar one).
+// (The first form fetched fragments and scales from global memory and handed scales round by shuffles, which the four schedulers of an SM
+// share at one per clock: Q8_0 6144 x 1024 with 2048 tokens spent 55 clocks per scheduler on an MMA and its 12 scaling operations.)
+// What bounds it: 15 instructions per MMA at half the issue rate; mma.sync and the fp32 pipe exclude each other (an MMA with its conversions
+// and scaling alone takes 25 clocks, the kernel 28).  The sums from tcgen05.mma kind::f16 (exact in its fp32 accumulators) were no faster:
+// two drain warps per scheduler took 24 clocks per MMA's worth.
+// Measured, us (before): Q8_0 6144 x 1024, 2048 tokens 155 -> 103, 4096 x 1024 105 -> 69, 1024 x 3072 67 -> 52, 1024 x 2048 48 -> 38, 4096 x 1024
+// with 333 25 -> 19; Q6_K 4096 x 14336, 777 tokens 833 -> 615.
+__device__ __forceinline__ uint32_t smem_at(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+template <int B>
+__device__ __forceinline__ void copy_async(uint32_t dst, const void *src)
+{
+    if constexpr (B == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(B) : "memory");
+}
+__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t &a, uint32_t &b, uint32_t &c, uint32_t &d)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm2(uint32_t addr, uint32_t &a, uint32_t &b)
+{
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(a), "=r"(b) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ uint2 lds8(uint32_t a)
+{
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a) : "memory");
+    return v;
+}
+typedef unsigned long long f32x2;  // two floats in a register pair
+__device__ __forceinline__ f32x2 pair_x2(float a, float b)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpair_x2(f32x2 v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 add_x2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul_x2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma_x2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+constexpr int TILE_ROWS = 64, TILE_THREADS = 128;
+template <bool Q6, int NT>
+struct TileShape {
+    static constexpr int TOK = 16 * NT, KG = Q6 ? 256 : 128, NB = KG / 32, S = 2;  // tokens; elements and 32-element blocks of a group; groups in flight
+    static constexpr int WROW = Q6 ? 208 : 144, XROW = KG + 16;                     // bytes of a weight row (Q8_0: 128 and its four scales) and of a token
+    static constexpr int DXS = NT == 8 ? 20 : NT == 6 ? 12 : 2 * NT;               // floats between the lanes' token scales: off each other's banks
+    static constexpr int OFF_X = TILE_ROWS * WROW, OFF_DX = OFF_X + TOK * XROW, OFF_D = OFF_DX + 2 * NB * 4 * DXS * 4;
+    static constexpr int STAGE = OFF_D + (Q6 ? TILE_ROWS * 4 : 0), SMEM = S * STAGE;
+    static_assert(STAGE % 16 == 0 && NT % 2 == 0, "alignment");
+};
+
+template <bool Q6, int NT, int CTAS>
+__global__ void __launch_bounds__(TILE_THREADS, CTAS)
+gemv_mma_tile_kernel(const uint8_t *__restrict__ w, const __half *__restrict__ wd, const int8_t *__restrict__ xq, const float *__restrict__ xd,
+                     float *__restrict__ out, int N, int K, int M, int ncls)
+{
+    using P = TileShape<Q6, NT>;
+    extern __shared__ __align__(16) uint8_t sm_tile[];
+    const uint32_t base = smem_at(sm_tile);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tg = lane & 3, wr = warp >> 1, wt = warp & 1;
+    const int r0 = blockIdx.x * TILE_ROWS, t0 = blockIdx.y * P::TOK, nb = K / 32, ngroups = K / P::KG;
+
+    int a_cls = 0, a_gi = 0;  // the group to be requested next: classes in turn, groups cls, cls + ncls, ... of each
+    auto request = [&](int slot) {
+        if (a_cls < ncls && a_gi < ngroups) {
+            const uint32_t st = base + (uint32_t)slot * P::STAGE;
+            constexpr int PIECES = Q6 ? 13 : 8, XP = P::KG / 16;
+#pragma unroll
+            for (int i = 0; i < (TILE_ROWS * PIECES + TILE_THREADS - 1) / TILE_THREADS; ++i) {
+                const int e = threadIdx.x + i * TILE_THREADS;
+                if (TILE_ROWS * PIECES % TILE_THREADS && e >= TILE_ROWS * PIECES) break;
+                const int r = e / PIECES, c = e % PIECES;
+                // What lies past the last row or token is not loaded (nor stored: outputs do not mix).  Clamped to the last token, a ragged tile
+                // of every CTA asked the same L2 lines for it: 6144 x 1024 Q8_0 with 300 tokens took 52 us, with 256 21.
+                if (r0 + r >= N) break;
+                const size_t row = (size_t)(r0 + r);
+                const uint8_t *src;
+                if (Q6) {
+                    const size_t blk = row * ngroups + a_gi;
+                    src = c < 12 ? w + smc_q6u_slot(blk, 0, 0) + 512 * (c >> 2) + 16 * (c & 3) : w + smc_q6u_scales(blk);
+                } else src = w + row * K + a_gi * 128 + 16 * c;
+                copy_async<16>(st + (uint32_t)(r * P::WROW + 16 * c), src);
+            }
+            if (threadIdx.x < TILE_ROWS && r0 + (int)threadIdx.x < N) {  // Q8_0: four scales behind the row's codes; Q6_K: the aligned four bytes that hold the block's d
+                const size_t row = (size_t)(r0 + (int)threadIdx.x);
+                if (Q6) copy_async<4>(st + (uint32_t)(P::OFF_D + 4 * threadIdx.x), w + (smc_q6u_d(row * ngroups + a_gi) & ~(size_t)3));
+                else copy_async<8>(st + (uint32_t)(threadIdx.x * P::WROW + 128), wd + row * nb + a_gi * 4);
+            }
+#pragma unroll
+            for (int i = 0; i < P::TOK * XP / TILE_THREADS; ++i) {
+                const int e = threadIdx.x + i * TILE_THREADS, t = e / XP, c = e % XP;
+                if (t0 + t < M) copy_async<16>(st + (uint32_t)(P::OFF_X + t * P::XROW + 16 * c), xq + (size_t)(t0 + t) * K + a_gi * P::KG + 16 * c);
+            }
+#pragma unroll
+            for (int i = 0; i < P::TOK * P::NB / TILE_THREADS; ++i) {
+                const int e = threadIdx.x + i * TILE_THREADS, t = e / P::NB, b = e % P::NB, u = t % (8 * NT);
+                if (t0 + t < M)
+                    copy_async<4>(st + (uint32_t)(P::OFF_DX + 4 * ((((t / (8 * NT)) * P::NB + b) * 4 + ((u & 7) >> 1)) * P::DXS + 2 * (u >> 3) + (u & 1))),
+                                  xd + (size_t)(t0 + t) * nb + a_gi * P::NB + b);
+            }
+            a_gi += ncls;
+            while (a_gi >= ngroups && a_cls < ncls) a_gi = ++a_cls;
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    static_assert(P::TOK * (P::KG / 16) % TILE_THREADS == 0 && P::TOK * P::NB % TILE_THREADS == 0, "copies per thread");
+    smc_grid_dep_sync();
+#pragma unroll
+    for (int i = 0; i < P::S - 1; ++i) request(i);
+
+    // this lane's ldmatrix rows
+    const uint32_t a_off = (uint32_t)((wr * 32 + (lane & 7) + 8 * ((lane >> 3) & 1)) * P::WROW + 16 * (lane >> 4));
+    const uint32_t b_off = (uint32_t)(P::OFF_X + wt * 8 * NT * P::XROW), dx_off = (uint32_t)(P::OFF_DX + (wt * P::NB * 4 + tg) * P::DXS * 4);
+    f32x2 acc[2][NT][2], total[2][NT][2];  // [16-row tile][token tile][rows g, g + 8]: tokens 2 tg, 2 tg + 1
+    auto scale_add = [&](f32x2 (&a)[2], const int (&c)[4], const f32x2 (&ws)[2], f32x2 dx) {
+        a[0] = fma_x2(pair_x2((float)c[0], (float)c[1]), mul_x2(ws[0], dx), a[0]);
+        a[1] = fma_x2(pair_x2((float)c[2], (float)c[3]), mul_x2(ws[1], dx), a[1]);
+    };
+    auto token_scales = [&](uint32_t at, f32x2 (&v)[NT]) {
+#pragma unroll
+        for (int t = 0; t < NT; t += 2) asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(v[t]), "=l"(v[t + 1]) : "r"(at + 8u * t) : "memory");
+    };
+    auto group_q8 = [&](uint32_t st) {
+        uint2 dw[2][2];
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) dw[mt][h] = lds8(st + (uint32_t)((wr * 32 + 16 * mt + 8 * h + g) * P::WROW + 128));
+#pragma unroll
+        for (int kb = 0; kb < 4; ++kb) {
+            uint32_t a[2][4], b[NT][2];
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt) ldsm4(st + a_off + (uint32_t)(16 * mt * P::WROW + 32 * kb), a[mt][0], a[mt][1], a[mt][2], a[mt][3]);
+#pragma unroll
+            for (int t = 0; t < NT; t += 2)
+                ldsm4(st + b_off + (uint32_t)((8 * t + (lane & 7) + 8 * (lane >> 4)) * P::XROW + 32 * kb + 16 * ((lane >> 3) & 1)), b[t][0], b[t][1], b[t + 1][0], b[t + 1][1]);
+            f32x2 dx[NT], ws[2][2];
+            token_scales(st + dx_off + (uint32_t)(kb * 16 * P::DXS), dx);
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const uint32_t two = (kb & 2) ? dw[mt][h].y : dw[mt][h].x;
+                    const float d = smc_h2f((uint16_t)((kb & 1) ? (two >> 16) : (two & 0xFFFFu)));
+                    ws[mt][h] = pair_x2(d, d);
+                }
+#pragma unroll
+            for (int t = 0; t < NT; ++t)
+#pragma unroll
+                for (int mt = 0; mt < 2; ++mt) {
+                    int c[4];
+                    mma_s8(c, a[mt][0], a[mt][1], a[mt][2], a[mt][3], b[t][0], b[t][1]);
+                    scale_add(acc[mt][t], c, ws[mt], dx[t]);
+                }
+        }
+    };
+    auto group_q6 = [&](uint32_t st, int gi) {
+        float d[2][2];
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int r = wr * 32 + 16 * mt + 8 * u + g;
+                uint32_t two;
+                asm volatile("ld.shared.u32 %0, [%1];" : "=r"(two) : "r"(st + (uint32_t)(P::OFF_D + 4 * r)) : "memory");
+                const bool odd = ((uint32_t)(r0 + r) * (uint32_t)ngroups + (uint32_t)gi) & 1u;  // of the block's number
+                d[mt][u] = smc_h2f((uint16_t)(odd ? two >> 16 : two & 0xFFFFu));
+            }
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+            uint2 sc[2][2];  // this half's scale bytes: is + 2 c
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+                for (int u = 0; u < 2; ++u) sc[mt][u] = lds8(st + (uint32_t)((wr * 32 + 16 * mt + 8 * u + g) * P::WROW + 192 + 8 * h));
+#pragma unroll
+            for (int is = 0; is < 2; ++is) {
+                uint32_t X[2][2], Y[2][2], Z[2][2];  // matrix i of an ldmatrix: rows 8 i .. 8 i + 7 of the warp's 32
+                const uint32_t at = st + (uint32_t)((wr * 32 + lane) * P::WROW + 32 * h + 16 * is);
+                ldsm4(at, X[0][0], X[0][1], X[1][0], X[1][1]);
+                ldsm4(at + 64, Y[0][0], Y[0][1], Y[1][0], Y[1][1]);
+                ldsm4(at + 128, Z[0][0], Z[0][1], Z[1][0], Z[1][1]);
+#pragma unroll
+                for (int c4 = 0; c4 < 4; ++c4) {
+                    uint32_t b[NT], a[2][2];
+                    const uint32_t kh = 128u * h + 32u * c4 + 16u * is;
+#pragma unroll
+                    for (int t = 0; t < NT; t += 4) {
+                        if (NT - t >= 4) ldsm4(st + b_off + (uint32_t)((8 * t + lane) * P::XROW) + kh, b[t], b[t + 1], b[t + 2], b[t + 3]);
+                        else ldsm2(st + b_off + (uint32_t)((8 * t + (lane & 15)) * P::XROW) + kh, b[t], b[t + 1]);
+                    }
+                    f32x2 dx[NT], ws[2][2];
+                    token_scales(st + dx_off + (uint32_t)((4 * h + c4) * 16 * P::DXS), dx);
+#pragma unroll
+                    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            const uint32_t wx = X[mt][u], wy = Y[mt][u], wz = Z[mt][u];
+                            uint32_t q;  // codes 0 .. 63, then 32 taken off bytewise: 0x80 keeps the borrow inside a byte
+                            if (c4 == 0) q = wx & 0x3F3F3F3Fu;
+                            else if (c4 == 1) q = wy & 0x3F3F3F3Fu;
+                            else if (c4 == 2) q = wz & 0x3F3F3F3Fu;
+                            else q = ((wx >> 6) & 0x03030303u) | ((wy >> 4) & 0x0C0C0C0Cu) | ((wz >> 2) & 0x30303030u);
+                            a[mt][u] = ((q | 0x80808080u) - 0x20202020u) ^ 0x80808080u;
+                            const int si = is + 2 * c4;
+                            const uint32_t word = si < 4 ? sc[mt][u].x : sc[mt][u].y;
+                            const float s = d[mt][u] * (float)(int)(int8_t)((word >> (8 * (si & 3))) & 0xFFu);
+                            ws[mt][u] = pair_x2(s, s);
+                        }
+#pragma unroll
+                    for (int t = 0; t < NT; ++t)
+#pragma unroll
+                        for (int mt = 0; mt < 2; ++mt) {
+                            int c[4];
+                            mma_s8_k16(c, a[mt][0], a[mt][1], b[t]);
+                            scale_add(acc[mt][t], c, ws[mt], dx[t]);
+                        }
+                }
+            }
+        }
+    };
+    int slot = 0;
+#pragma unroll 1
+    for (int cls = 0; cls < ncls; ++cls) {
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int t = 0; t < NT; ++t) acc[mt][t][0] = acc[mt][t][1] = 0ull;
+#pragma unroll 1
+        for (int gi = cls; gi < ngroups; gi += ncls) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(P::S - 2) : "memory");
+            __syncthreads();  // the group has landed for everybody, and everybody is through with the slot that is refilled
+            request(slot == 0 ? P::S - 1 : slot - 1);
+            const uint32_t st = base + (uint32_t)slot * P::STAGE;
+            if constexpr (Q6) group_q6(st, gi);
+            else group_q8(st);
+            if (++slot == P::S) slot = 0;
+        }
+        // the split kernels' fold: s = partial of warp 0; s += partial of warp 1; ...
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int t = 0; t < NT; ++t)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) total[mt][t][h] = cls == 0 ? acc[mt][t][h] : add_x2(total[mt][t][h], acc[mt][t][h]);
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float v[2];
+                unpair_x2(total[mt][t][h], v[0], v[1]);
+                const int row = r0 + wr * 32 + 16 * mt + 8 * h + g, tok = t0 + wt * 8 * NT + 8 * t + 2 * tg;
+                if (row < N && tok < M) out[(size_t)tok * N + row] = v[0];
+                if (row < N && tok + 1 < M) out[(size_t)(tok + 1) * N + row] = v[1];
+            }
+}
+
 }  // namespace
 
 bool smc_mma_supported(const smc_weight *w, int M)
@@ -490,12 +668,49 @@ bool smc_mma_supported(const smc_weight *w, int M)
     return false;
 }
 
+// Tokens per tile / 16 of the prompt-sized kernel for a call, 0: the kernels that split K over warps are the faster ones.
+// Both run in rounds: a CTA of a kernel takes so many us per 1024 elements of K, more if others share its SM.  Measured at K = 1024 .. 28672,
+// for one, two (and three) tiles on an SM; a CTA of the split kernels 2.7, and 1.8 whatever K of Q8_0 (its fold).  The estimates are within
+// a tenth of these measurements (us, split kernel -> the tile chosen): Q8_0 6144 x 1024, 64 tokens 12.5 -> 10.5, 400 48 -> 29, 700 72 -> 41; 1024 x
+// 3072, 256 14.3 (tiles 22.8), 512 24.5 -> 22.8, 1200 54 -> 43; Q6_K 4096 x 14336, 160 195 (213), 300 342 -> 312, 777 834 -> 615; 1024 x 4096, 600
+// 58 (64), 1200 101 -> 95.
+static int prompt_tile(const smc_ctx *ctx, const smc_weight *w, int M)
+{
+    const bool q6 = w->dtype == SMC_Q6_K;
+    if (M < 64 || (w->dtype != SMC_Q8_0 && !q6)) return 0;
+    const long long sms = ctx->sm_count, k = w->K;
+    auto per_sm = [&](long long ctas) { return (ctas + sms - 1) / sms; };
+    const long long strips = (w->N + MMA_ROWS - 1) / MMA_ROWS;
+    double best = q6 ? per_sm(strips * ((M + 31) / 32)) * 2.7 * k : per_sm(strips * ((M + 63) / 64)) * (1.8 * 1024 + 2.75 * k);
+    int nt = 0;
+    auto offer = [&](int n, int fit, const double (&us)[3]) {  // `fit` tiles share an SM
+        const long long c = per_sm(((long long)w->N + TILE_ROWS - 1) / TILE_ROWS * ((M + 16 * n - 1) / (16 * n)));
+        const double t = ((c / fit) * us[fit - 1] + (c % fit ? us[c % fit - 1] : 0.0)) * k;
+        if (t < best) best = t, nt = n;
+    };
+    if (q6) offer(4, 2, {12.6, 17.4, 0.0}), offer(6, 2, {15.2, 22.0, 0.0});
+    else offer(4, 3, {6.25, 10.0, 13.75}), offer(6, 2, {8.3, 13.0, 0.0}), offer(8, 2, {10.0, 15.8, 0.0});
+    return nt;
+}
+
 int smc_launch_gemv_mma(smc_ctx *ctx, const smc_q8act *a, const smc_weight *w, float *out, cudaStream_t s)
 {
     const int N = w->N, K = w->K, M = a->M;
     const int nt = M <= 8 ? 1 : (M <= 16 ? 2 : 4);
     const dim3 grid((N + MMA_ROWS - 1) / MMA_ROWS, (M + 8 * nt - 1) / (8 * nt));
-    if (w->dtype == SMC_Q8_0) {
+    if (const int pt = prompt_tile(ctx, w, M)) {
+        auto go = [&](auto kernel, size_t smem, int ncls) {
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            smc_launch_dep(ctx->use_pdl, kernel, dim3((N + TILE_ROWS - 1) / TILE_ROWS, (M + 16 * pt - 1) / (16 * pt)), dim3(TILE_THREADS), smem, s,
+                           w->dtype == SMC_Q6_K ? (const uint8_t *)w->q6u : (const uint8_t *)w->q8_qs, (const __half *)w->q8_d, (const int8_t *)a->q, (const float *)a->d,
+                           out, N, K, M, ncls);
+        };
+        if (w->dtype == SMC_Q6_K) {
+            const int ncls = K >= 8192 ? 16 : 8;
+            pt == 6 ? go(gemv_mma_tile_kernel<true, 6, 2>, TileShape<true, 6>::SMEM, ncls) : go(gemv_mma_tile_kernel<true, 4, 2>, TileShape<true, 4>::SMEM, ncls);
+        } else if (pt == 8) go(gemv_mma_tile_kernel<false, 8, 2>, TileShape<false, 8>::SMEM, 8);
+        else pt == 6 ? go(gemv_mma_tile_kernel<false, 6, 2>, TileShape<false, 6>::SMEM, 8) : go(gemv_mma_tile_kernel<false, 4, 3>, TileShape<false, 4>::SMEM, 8);
+    } else if (w->dtype == SMC_Q8_0) {
         // prompt-sized batches: passes of 64 tokens
         const int nt8 = M >= 64 ? 8 : nt;
         const dim3 g8((N + MMA_ROWS - 1) / MMA_ROWS, (M + 8 * nt8 - 1) / (8 * nt8));
@@ -505,15 +720,7 @@ int smc_launch_gemv_mma(smc_ctx *ctx, const smc_q8act *a, const smc_weight *w, f
             smc_launch_dep(ctx->use_pdl, kernel, g8, dim3(256), smem, s, (const int8_t *)w->q8_qs, (const __half *)w->q8_d,
                            (const int8_t *)a->q, (const float *)a->d, out, N, K, M);
         };
-        if (M >= 256 && (size_t)N * K < (1ull << 32) && (size_t)M * K < (1ull << 32)) {  // enough token tiles for a warp to own one: no K split, no shared memory
-            // eight token tiles of a 32-row strip per CTA share its weight fragments through L1; matrices of few rows
-            // take fewer per CTA so that the grid still covers the SMs twice (a warp's bits do not depend on this)
-            const int strips = (N + MMA_ROWS - 1) / MMA_ROWS, tiles = (M + 63) / 64;
-            int wpc = 8;
-            while (wpc > 1 && strips * ((tiles + wpc - 1) / wpc) < 2 * ctx->sm_count) wpc >>= 1;
-            smc_launch_dep(ctx->use_pdl, gemv_mma_q8_0_tile_kernel, dim3(strips, (tiles + wpc - 1) / wpc), dim3(32 * wpc), 0, s,
-                           (const int8_t *)w->q8_qs, (const __half *)w->q8_d, (const int8_t *)a->q, (const float *)a->d, out, N, K, M);
-        } else if (nt8 == 1) go8(gemv_mma_q8_0_kernel<1>, 32);
+        if (nt8 == 1) go8(gemv_mma_q8_0_kernel<1>, 32);
         else if (nt8 == 2) go8(gemv_mma_q8_0_kernel<2>, 32);
         else if (nt8 == 4) go8(gemv_mma_q8_0_kernel<4>, 32);
         else go8(gemv_mma_q8_0_kernel<8>, 64);

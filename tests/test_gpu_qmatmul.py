@@ -126,6 +126,26 @@ def test_q8_0_prompt_sized_batches_keep_the_small_batch_bits(oracle, cuda, dev, 
     cuda.release(w)
 
 
+@pytest.mark.parametrize("dtype,n,m,ks", [(Q8_0, 4100, 100, (384, 1152)), (Q8_0, 4700, 190, (384, 1024)), (Q8_0, 4700, 500, (384, 1152)),
+                                          (Q6_K, 9400, 128, (768, 2304)), (Q6_K, 4700, 190, (768, 8448))])
+def test_prompt_tiles_keep_the_small_batch_bits(cuda, dev, dtype, n, m, ks):
+    """The tile kernel of prompt-sized batches (64, 96 and 128 tokens a tile; ragged last rows and tokens; classes without groups, with one, with
+    several; eight and sixteen of them): every row has the bits that the kernels which split K give it in a batch of sixteen."""
+    import torch
+
+    from sharpmind_b200.ops import Mode
+
+    for k in ks:
+        g = torch.Generator(device="cuda").manual_seed(n + k)
+        w = cuda.register_dev(dev.quantize_weights(dtype, torch.randn((n, k), generator=g, device="cuda") * 0.02), dtype, n, k)
+        x = torch.randn((m, k), generator=g, device="cuda")
+        got = dev.qmatmul(x, w, Mode.ACT_Q8)
+        for lo in (0, 57, m - 16):
+            want = dev.qmatmul(x[lo:lo + 16].contiguous(), w, Mode.ACT_Q8)
+            assert torch.equal(got[lo:lo + 16].view(torch.int32), want.view(torch.int32)), (k, lo)
+        cuda.release(w)
+
+
 @pytest.mark.parametrize("dtype,n,k", [(Q6_K, 64, 2048), (Q8_0, 96, 1024), (Q4_K, 96, 4096), (Q6_K, 40, 14336)])
 @pytest.mark.parametrize("m", [2, 7, 64, 100])
 def test_fp32_activations_as_int8_digit_planes(oracle, cuda, dev, dtype, n, k, m):
