@@ -61,15 +61,18 @@ constexpr uint32_t COL_ACC_D = 0;    // 2 x 128
 constexpr uint32_t COL_ACC_M = 256;  // 128
 constexpr uint32_t COL_A = 384;      // NA x 32
 
-// barrier slots (8 bytes each) inside the last 256 bytes
+// Barrier slots (8 bytes each) inside the last 256 bytes.  The thread that issues the MMAs is what both kernels of this file ran at:
+// a wait, even for a barrier that has long completed, and a commit cost it 100 to 250 clocks each.  So it waits once per stage, for the
+// weights (the expanding warps see to it that the activations are there before they report theirs), and commits once, to
+// one barrier that all who wait for the stage's end look at.  Before: two waits and two commits, in the Q6_K kernel three of each.
+// Measured with the weights' copies (see the expansion): Q4_K 28672 x 4096, 777 tokens 667 -> 503 us, 4096 x 4096, 2048 tokens 283 -> 224;
+// Q6_K 4096 x 14336, 500 rows of fp32 404 -> 371, 8192 x 28672, 100 rows 748 -> 677.
+static_assert(NA == NB, "one barrier releases an A and a B stage");
 enum {
     BAR_FULL_B = 0,
-    BAR_EMPTY_B = BAR_FULL_B + NB,
-    BAR_FULL_A = BAR_EMPTY_B + NB,
+    BAR_FULL_A = BAR_FULL_B + NB,
     BAR_EMPTY_A = BAR_FULL_A + NA,
-    BAR_FULL_W = BAR_EMPTY_A + NA,
-    BAR_EMPTY_W = BAR_FULL_W + NW,
-    BAR_ACC_FULL = BAR_EMPTY_W + NW,
+    BAR_ACC_FULL = BAR_EMPTY_A + NA,
     BAR_ACC_EMPTY = BAR_ACC_FULL + 2,
     BAR_COUNT = BAR_ACC_EMPTY + 2
 };
@@ -117,10 +120,11 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, volatil
     *abort_flag = 1;
     atomicExch(status, 3);
 }
-// One lane polls, the warp follows: 128 or 256 threads polling (and arriving on) one barrier word made the
-// handshakes themselves the slowest part of the pipeline.
+// All lanes look once (mostly the phase is over), then one polls and the warp follows: 128 or 256 threads polling (and arriving on) one
+// barrier word made the handshakes themselves the slowest part of the pipeline.
 __device__ __forceinline__ void warp_wait(uint32_t bar, uint32_t parity, volatile uint32_t *abort_flag, int *status)
 {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return;
     if ((threadIdx.x & 31) == 0) mbar_wait(bar, parity, abort_flag, status);
     __syncwarp();
 }
@@ -306,17 +310,10 @@ prefill_q4k_kernel(const uint8_t *__restrict__ raw, const __half *__restrict__ i
     auto bar = [&](int i) { return sbase + OFF_BAR + 8u * (uint32_t)i; };
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < NB; ++i) {
-            mbar_init(bar(BAR_FULL_B + i), 1);
-            mbar_init(bar(BAR_EMPTY_B + i), 1);
-        }
+        for (int i = 0; i < NB; ++i) mbar_init(bar(BAR_FULL_B + i), 1);
         for (int i = 0; i < NA; ++i) {
             mbar_init(bar(BAR_FULL_A + i), EXPAND_WARPS);  // one arrival per expansion warp
             mbar_init(bar(BAR_EMPTY_A + i), 1);
-        }
-        for (int i = 0; i < NW; ++i) {
-            mbar_init(bar(BAR_FULL_W + i), 1);             // the expect_tx arrival; the 128 row copies add bytes
-            mbar_init(bar(BAR_EMPTY_W + i), EXPAND_WARPS);
         }
         for (int i = 0; i < 2; ++i) {
             mbar_init(bar(BAR_ACC_FULL + i), 1);
@@ -341,21 +338,18 @@ prefill_q4k_kernel(const uint8_t *__restrict__ raw, const __half *__restrict__ i
         if (lane == 0) {
             const __half *src = img + (size_t)tt * (K / KS) * 2 * (TN * KS);
             const __half *msrc = mimg + (size_t)tt * nsb * (2 * TN * 16);
-            int slot = 0;
-            uint32_t phase = 1;  // a fresh barrier passes a wait on the phase before its first
             for (int sb = 0; sb < nsb; ++sb) {
 #pragma unroll
                 for (int g = 0; g < NA; ++g) {
-                    mbar_wait(bar(BAR_EMPTY_B + slot), phase, abort_flag, status);
-                    const uint32_t fb = bar(BAR_FULL_B + slot);
+                    mbar_wait(bar(BAR_EMPTY_A + g), (uint32_t)((sb & 1) ^ 1), abort_flag, status);  // a fresh barrier passes a wait on the phase before its first
+                    const uint32_t fb = bar(BAR_FULL_B + g);
                     mbar_expect_tx(fb, 2 * B_BYTES + (g == 0 ? BM_BYTES : 0u));
-                    bulk_g2s(sbase + (uint32_t)slot * SLOT_BYTES, src + (size_t)(sb * NA + g) * 2 * (TN * KS), 2 * B_BYTES, fb);
+                    bulk_g2s(sbase + (uint32_t)g * SLOT_BYTES, src + (size_t)(sb * NA + g) * 2 * (TN * KS), 2 * B_BYTES, fb);
                     // the aux buffer sb & 1 was last read by the MMAs of block sb - 2, which completed before the
                     // MMAs whose commit released this B slot (a stage of block sb - 1) were even issued
                     if (g == 0)
                         bulk_g2s(sbase + OFF_AUX + (uint32_t)(sb & 1) * AUX_BYTES + AM_BYTES, msrc + (size_t)sb * (2 * TN * 16),
                                  BM_BYTES, fb);
-                    if (++slot == NB) slot = 0, phase ^= 1;
                 }
             }
         }
@@ -369,19 +363,15 @@ prefill_q4k_kernel(const uint8_t *__restrict__ raw, const __half *__restrict__ i
             const uint64_t aux_desc0 = smem_desc(sbase + OFF_AUX, 128, 256);  // aux buffer 0, A''
             constexpr uint64_t U_SLOT = SLOT_BYTES >> 4, U_LO = B_BYTES >> 4, U_KK = 256 >> 4;
             constexpr uint64_t U_AUX = AUX_BYTES >> 4, U_BM = AM_BYTES >> 4, U_BM2 = (AM_BYTES + TN * 16 * 2) >> 4;
-            int slot = 0;
-            uint32_t b_phase = 0;
             for (int sb = 0; sb < nsb; ++sb) {
                 const int buf = sb & 1;
                 mbar_wait(bar(BAR_ACC_EMPTY + buf), (uint32_t)(((sb >> 1) & 1) ^ 1), abort_flag, status);
-                tc_fence_after();
                 const uint32_t acc_d = tmem_base + COL_ACC_D + (uint32_t)buf * 128u;
 #pragma unroll
                 for (int g = 0; g < NA; ++g) {
-                    mbar_wait(bar(BAR_FULL_B + slot), b_phase, abort_flag, status);
                     mbar_wait(bar(BAR_FULL_A + g), (uint32_t)(sb & 1), abort_flag, status);
                     tc_fence_after();
-                    const uint64_t bh = b_desc0 + (uint64_t)slot * U_SLOT;
+                    const uint64_t bh = b_desc0 + (uint64_t)g * U_SLOT;
                     const uint32_t a0 = tmem_base + COL_A + (uint32_t)g * 32u;
                     if (g == 0) {
                         const uint64_t am = aux_desc0 + (uint64_t)buf * U_AUX;
@@ -393,10 +383,7 @@ prefill_q4k_kernel(const uint8_t *__restrict__ raw, const __half *__restrict__ i
                         tc_mma_f16_ta(acc_d, a0 + kk * 8, bh + kk * U_KK, IDESC, (g | kk) != 0 ? 1u : 0u);
 #pragma unroll
                     for (int kk = 0; kk < KS / 16; ++kk) tc_mma_f16_ta(acc_d, a0 + kk * 8, bh + U_LO + kk * U_KK, IDESC, 1u);
-                    // both arrive when the MMAs above have read their operands
-                    tc_commit(bar(BAR_EMPTY_B + slot));
-                    tc_commit(bar(BAR_EMPTY_A + g));
-                    if (++slot == NB) slot = 0, b_phase ^= 1;
+                    tc_commit(bar(BAR_EMPTY_A + g));  // arrives when the MMAs above have read their operands
                 }
                 tc_commit(bar(BAR_ACC_FULL + buf));
             }
@@ -404,33 +391,37 @@ prefill_q4k_kernel(const uint8_t *__restrict__ raw, const __half *__restrict__ i
     } else if (warp < WARP_DRAIN0) {
         // ---------------- weight expansion.  A warp may only touch the TMEM lanes of its quarter (warp % 4); the
         // two warps of a quarter split a stage: plane 0 expands the low nibbles (sub-block 2g, columns 0..15),
-        // plane 1 the high nibbles (sub-block 2g + 1, columns 16..31).  The raw 144-byte blocks arrive through a
-        // ring of bulk copies, one copy per row and block, issued NW - 1 blocks ahead by the plane-0 thread of
-        // the row: register prefetch of one block was not enough to cover the latency of these scattered reads.
+        // plane 1 the high nibbles (sub-block 2g + 1, columns 16..31).  The raw 144-byte blocks come by 16-byte asynchronous copies,
+        // NW - 1 blocks ahead (as one bulk copy per row and block they took the issuing lanes 2400 clocks of a block's 5900).
         const int quarter = warp & 3, plane = (warp - WARP_EXPAND0) >> 2;
         const int r = quarter * 32 + lane;
-        const uint8_t *rowp = raw + (size_t)(row0 + r) * row_bytes;
         const uint32_t am_row = (uint32_t)(r >> 3) * 256u + (uint32_t)(r & 7) * 16u;
         const uint32_t a_lane = tmem_base + ((uint32_t)(quarter * 32) << 16) + COL_A + (uint32_t)plane * 16u;
-        const uint32_t w_row = sbase + OFF_W + (uint32_t)r * 144u;
-        auto fetch_block = [&](int p) {  // plane-0 threads: request block p of this thread's row
-            const int ws = p % NW;
-            warp_wait(bar(BAR_EMPTY_W + ws), (uint32_t)(((p / NW) & 1) ^ 1), abort_flag, status);
-            const uint32_t fw = bar(BAR_FULL_W + ws);
-            if (warp == WARP_EXPAND0 && lane == 0) mbar_expect_tx(fw, W_BYTES);
-            asm volatile("bar.sync 1, 128;" ::: "memory");  // the four plane-0 warps: bytes are expected before any copy lands
-            bulk_g2s(w_row + (uint32_t)ws * W_BYTES, rowp + (size_t)p * 144, 144u, fw);
+        const uint32_t w_quarter = sbase + OFF_W + (uint32_t)(quarter * 32) * 144u, meet = 1u + (uint32_t)quarter;  // named barrier of the quarter's two warps
+        auto fetch_block = [&](int p) {  // plane 0: block p of the quarter's 32 rows, nine pieces a row, neighbouring lanes on one row
+            if (p < nsb) {
+                const uint32_t dst = w_quarter + (uint32_t)(p % NW) * W_BYTES;
+#pragma unroll
+                for (int i = 0; i < 9; ++i) {
+                    const int idx = i * 32 + lane, rr = idx / 9, c = idx % 9;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * (uint32_t)idx),
+                                 "l"(raw + (size_t)(row0 + quarter * 32 + rr) * row_bytes + (size_t)p * 144 + 16 * c)
+                                 : "memory");
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
         };
         if (plane == 0)
-            for (int p = 0; p < NW - 1 && p < nsb; ++p) fetch_block(p);
+            for (int p = 0; p < NW - 1; ++p) fetch_block(p);
         for (int sb = 0; sb < nsb; ++sb) {
-            const int ws = sb % NW;
-            if (plane == 0 && sb + NW - 1 < nsb) fetch_block(sb + NW - 1);
-            warp_wait(bar(BAR_FULL_W + ws), (uint32_t)((sb / NW) & 1), abort_flag, status);
+            if (plane == 0) asm volatile("cp.async.wait_group %0;" ::"n"(NW - 2) : "memory");
+            // block sb has landed; and both warps are through with block sb - 1, whose slot is refilled next
+            asm volatile("bar.sync %0, 64;" ::"r"(meet) : "memory");
+            if (plane == 0) fetch_block(sb + NW - 1);
+            const uint32_t w_row = w_quarter + (uint32_t)(sb % NW) * W_BYTES + (uint32_t)lane * 144u;
             uint4 cur[9];
 #pragma unroll
-            for (int i = 0; i < 9; ++i) cur[i] = lds128(w_row + (uint32_t)ws * W_BYTES + 16u * i);
-            warp_arrive(bar(BAR_EMPTY_W + ws));  // the bytes are in registers: the slot may be refilled
+            for (int i = 0; i < 9; ++i) cur[i] = lds128(w_row + 16u * i);
             const uint32_t s0 = cur[0].y, s1 = cur[0].z, s2 = cur[0].w;  // the 12 packed scale / min bytes
 #pragma unroll
             for (int g = 0; g < NA; ++g) {
@@ -475,9 +466,11 @@ prefill_q4k_kernel(const uint8_t *__restrict__ raw, const __half *__restrict__ i
                 tc_st16(a_lane + (uint32_t)g * 32u, col);
                 tc_wait_st();
                 tc_fence_before();
+                warp_wait(bar(BAR_FULL_B + g), (uint32_t)(sb & 1), abort_flag, status);
                 warp_arrive(bar(BAR_FULL_A + g));
             }
         }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
     } else {
         // ---------------- drain: thread = (TMEM lane = weight row, 64 of the 128 token columns)
         const int quarter = warp & 3, half = (warp - WARP_DRAIN0) >> 2;
@@ -487,9 +480,11 @@ prefill_q4k_kernel(const uint8_t *__restrict__ raw, const __half *__restrict__ i
         float acc[64];
 #pragma unroll
         for (int i = 0; i < 64; ++i) acc[i] = 0.f;
+        uint16_t d_next = smc_ldg_stream2(rowp);
         for (int sb = 0; sb < nsb; ++sb) {
             const int buf = sb & 1;
-            const float d = smc_h2f(smc_ldg_stream2(rowp + (size_t)sb * 144));
+            const float d = smc_h2f(d_next);
+            if (sb + 1 < nsb) d_next = smc_ldg_stream2(rowp + (size_t)(sb + 1) * 144);
             warp_wait(bar(BAR_ACC_FULL + buf), (uint32_t)((sb >> 1) & 1), abort_flag, status);
             tc_fence_after();
             const uint32_t td = lane_base + COL_ACC_D + (uint32_t)buf * 128u;
@@ -543,10 +538,10 @@ prefill_q4k_kernel(const uint8_t *__restrict__ raw, const __half *__restrict__ i
 // five places of its unit, so they come by 16-byte asynchronous copies: a warp of the first four (plane 0) fetches the rows of its
 // quarter for both warps of the quarter and the pair meets at a named barrier; plane 0 unpacks the first 32 elements of each
 // stage, plane 1 the second 32.
-// What bounds it: the hand-overs.  The tensor pipe is active 38 % of the time; of 1.8 us per 64 elements of K about 1 us stays whichever of
-// drain, fold, unpacking and copies is left out (24 MMAs a stage 447 us, 20 420 us, 12 366 us, before the fold's change).  Before, fp32 rows went through mma.sync as three int8 digit planes, one scaling on
-// the CUDA cores per output, plane and 16 elements.
-// 4096 x 14336 with 500 rows: 1595 -> 404 us (145 useful TFLOP/s); distance from 64 bits 1.84e-7 -> 1.33e-7, 8192 x 28672
+// What bounds it: the hand-overs.  The tensor pipe is active 40 % of the time; of 1.65 us per 64 elements of K about 1 us stays whichever of
+// drain, fold, unpacking and copies is left out (24 MMAs a stage 447 us, 20 420 us, 12 366 us, before the fold's and the issuing thread's
+// changes).  Before, fp32 rows went through mma.sync as three int8 digit planes, one scaling on the CUDA cores per output, plane and 16 elements.
+// 4096 x 14336 with 500 rows: 1595 -> 371 us (158 useful TFLOP/s); distance from 64 bits 1.84e-7 -> 1.33e-7, 8192 x 28672
 // 2.26e-7 -> 1.42e-7, 1024 x 4096 1.50e-7 -> 1.26e-7.
 constexpr int Q6_RAW = 208;                        // bytes of a row and block in shared memory: X, Y, Z (64 each), 16 scales: an odd multiple of 16
 constexpr int Q6_NW = 3;                           // blocks in flight
@@ -556,8 +551,7 @@ constexpr uint32_t Q6_SLOT = 3 * B_BYTES;          // x0, x1, x2
 constexpr uint32_t Q6_OFF_W = Q6_NB * Q6_SLOT, Q6_OFF_BAR = Q6_OFF_W + Q6_NW * Q6_W_BYTES, Q6_SMEM = Q6_OFF_BAR + 256;
 static_assert(Q6_SMEM <= 227 * 1024, "shared memory budget");
 constexpr uint32_t Q6_COL_A = 256;                 // NA x 64 columns: 32 of v_hi, 32 of v_lo
-enum { Q6_FULL_B = 0, Q6_EMPTY_B = Q6_FULL_B + Q6_NB, Q6_FULL_A = Q6_EMPTY_B + Q6_NB, Q6_EMPTY_A = Q6_FULL_A + NA, Q6_ACC_FULL = Q6_EMPTY_A + NA,
-       Q6_ACC_EMPTY = Q6_ACC_FULL + 2, Q6_BARS = Q6_ACC_EMPTY + 2 };
+enum { Q6_FULL_B = 0, Q6_FULL_A = Q6_FULL_B + Q6_NB, Q6_DONE = Q6_FULL_A + NA, Q6_ACC_EMPTY = Q6_DONE + NA, Q6_BARS = Q6_ACC_EMPTY + 2 };  // DONE: a stage's MMAs
 static_assert(Q6_BARS * 8 + 8 <= 256, "barrier area");
 
 constexpr uint32_t Q6_IDESC = IDESC | (1u << 7) | (1u << 10);  // bfloat16 A and B
@@ -617,9 +611,9 @@ prefill_q6k_kernel(const uint8_t *__restrict__ q6u, const __nv_bfloat16 *__restr
     auto bar = [&](int i) { return sbase + Q6_OFF_BAR + 8u * (uint32_t)i; };
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < Q6_NB; ++i) mbar_init(bar(Q6_FULL_B + i), 1), mbar_init(bar(Q6_EMPTY_B + i), 1);
-        for (int i = 0; i < NA; ++i) mbar_init(bar(Q6_FULL_A + i), EXPAND_WARPS), mbar_init(bar(Q6_EMPTY_A + i), 1);
-        for (int i = 0; i < 2; ++i) mbar_init(bar(Q6_ACC_FULL + i), 1), mbar_init(bar(Q6_ACC_EMPTY + i), DRAIN_WARPS);
+        for (int i = 0; i < Q6_NB; ++i) mbar_init(bar(Q6_FULL_B + i), 1);
+        for (int i = 0; i < NA; ++i) mbar_init(bar(Q6_FULL_A + i), EXPAND_WARPS), mbar_init(bar(Q6_DONE + i), 1);
+        for (int i = 0; i < 2; ++i) mbar_init(bar(Q6_ACC_EMPTY + i), DRAIN_WARPS);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_proxy_async();
@@ -638,12 +632,11 @@ prefill_q6k_kernel(const uint8_t *__restrict__ q6u, const __nv_bfloat16 *__restr
         if (lane == 0) {
             const __nv_bfloat16 *src = img + (size_t)tt * (K / KS) * 3 * (TN * KS);
             int slot = 0;
-            uint32_t phase = 1;
             for (int st = 0; st < nsb * NA; ++st) {
-                mbar_wait(bar(Q6_EMPTY_B + slot), phase, abort_flag, status);
+                if (st >= Q6_NB) mbar_wait(bar(Q6_DONE + (st - Q6_NB) % NA), (uint32_t)((st - Q6_NB) / NA) & 1u, abort_flag, status);
                 mbar_expect_tx(bar(Q6_FULL_B + slot), Q6_SLOT);
                 bulk_g2s(sbase + (uint32_t)slot * Q6_SLOT, src + (size_t)st * 3 * (TN * KS), Q6_SLOT, bar(Q6_FULL_B + slot));
-                if (++slot == Q6_NB) slot = 0, phase ^= 1;
+                if (++slot == Q6_NB) slot = 0;
             }
         }
     } else if (warp == 1) {
@@ -651,14 +644,12 @@ prefill_q6k_kernel(const uint8_t *__restrict__ q6u, const __nv_bfloat16 *__restr
             const uint64_t b_desc0 = smem_desc(sbase, 128, 1024);
             constexpr uint64_t U_SLOT = Q6_SLOT >> 4, U_X = B_BYTES >> 4, U_KK = 256 >> 4;
             int slot = 0;
-            uint32_t b_phase = 0;
             for (int sb = 0; sb < nsb; ++sb) {
 #pragma unroll
                 for (int g = 0; g < NA; ++g) {
                     const int buf = g & 1, use = 2 * sb + (g >> 1);  // which time this accumulator is filled
                     const uint32_t acc_d = tmem_base + (uint32_t)buf * 128u;
                     mbar_wait(bar(Q6_ACC_EMPTY + buf), (uint32_t)((use & 1) ^ 1), abort_flag, status);
-                    mbar_wait(bar(Q6_FULL_B + slot), b_phase, abort_flag, status);
                     mbar_wait(bar(Q6_FULL_A + g), (uint32_t)(sb & 1), abort_flag, status);
                     tc_fence_after();
                     const uint64_t x0 = b_desc0 + (uint64_t)slot * U_SLOT, x1 = x0 + U_X, x2 = x1 + U_X;
@@ -670,10 +661,8 @@ prefill_q6k_kernel(const uint8_t *__restrict__ q6u, const __nv_bfloat16 *__restr
                     products(v_lo, x1, true), products(v_hi, x2, false);
                     products(v_lo, x0, false), products(v_hi, x1, false);
                     products(v_hi, x0, false);
-                    tc_commit(bar(Q6_EMPTY_B + slot));
-                    tc_commit(bar(Q6_EMPTY_A + g));
-                    tc_commit(bar(Q6_ACC_FULL + buf));
-                    if (++slot == Q6_NB) slot = 0, b_phase ^= 1;
+                    tc_commit(bar(Q6_DONE + g));  // frees both operands' stages and hands the accumulator over
+                    if (++slot == Q6_NB) slot = 0;
                 }
             }
         }
@@ -697,6 +686,8 @@ prefill_q6k_kernel(const uint8_t *__restrict__ q6u, const __nv_bfloat16 *__restr
         };
         if (plane == 0)
             for (int p = 0; p < Q6_NW - 1; ++p) fetch_block(p);
+        int b_slot = 0;
+        uint32_t b_phase = 0;
         for (int sb = 0; sb < nsb; ++sb) {
             if (plane == 0) asm volatile("cp.async.wait_group %0;" ::"n"(Q6_NW - 2) : "memory");
             // block sb has landed; and both warps are through with block sb - 1, whose slot is refilled next
@@ -730,12 +721,14 @@ prefill_q6k_kernel(const uint8_t *__restrict__ q6u, const __nv_bfloat16 *__restr
                             hi[8 * o + 2 * j] = eh[0], hi[8 * o + 2 * j + 1] = eh[1], lo[8 * o + 2 * j] = el[0], lo[8 * o + 2 * j + 1] = el[1];
                         }
                     }
-                    warp_wait(bar(Q6_EMPTY_A + g), (uint32_t)((sb & 1) ^ 1), abort_flag, status);
+                    warp_wait(bar(Q6_DONE + g), (uint32_t)((sb & 1) ^ 1), abort_flag, status);
                     tc_fence_after();
                     tc_st16(a_lane + (uint32_t)g * 64u, hi);
                     tc_st16(a_lane + (uint32_t)g * 64u + 32u, lo);
                     tc_wait_st();
                     tc_fence_before();
+                    warp_wait(bar(Q6_FULL_B + b_slot), b_phase, abort_flag, status);
+                    if (++b_slot == Q6_NB) b_slot = 0, b_phase ^= 1;
                     warp_arrive(bar(Q6_FULL_A + g));
                 }
             }
@@ -751,12 +744,14 @@ prefill_q6k_kernel(const uint8_t *__restrict__ q6u, const __nv_bfloat16 *__restr
 #pragma unroll
         for (int i = 0; i < 64; ++i) acc[i] = 0.f;
         bool folded = false;
+        __half d_next = *reinterpret_cast<const __half *>(q6u + smc_q6u_d(blk0));
         for (int sb = 0; sb < nsb; ++sb) {
-            const float d = __half2float(*reinterpret_cast<const __half *>(q6u + smc_q6u_d(blk0 + sb)));
+            const float d = __half2float(d_next);
+            if (sb + 1 < nsb) d_next = *reinterpret_cast<const __half *>(q6u + smc_q6u_d(blk0 + sb + 1));
 #pragma unroll 1
             for (int g = 0; g < NA; ++g) {
-                const int buf = g & 1, use = 2 * sb + (g >> 1);
-                warp_wait(bar(Q6_ACC_FULL + buf), (uint32_t)(use & 1), abort_flag, status);
+                const int buf = g & 1;
+                warp_wait(bar(Q6_DONE + g), (uint32_t)(sb & 1), abort_flag, status);
                 tc_fence_after();
                 const uint32_t td = lane_base + (uint32_t)buf * 128u;
 #pragma unroll
@@ -891,7 +886,8 @@ int smc_launch_prefill_q4k_q8(smc_ctx *ctx, const smc_q8act *a, const smc_weight
 // digit planes on mma.sync take 5.5e-5 ns per element of K, weight row and activation row, in steps of 16 rows: the lines cross at
 // about 500 000 outputs per wave.  Measured, digit planes -> here, us: 3584 x 4096 with 137 rows 121 -> 129, 143 rows 130 -> 129, 168
 // rows 152 -> 128; 1024 x 4096 with 479 rows 125 -> 130, 499 rows 135 -> 130; 3584 x 14336 with 143 rows 428 -> 382; 8192 x 28672
-// with 65 rows 942 -> 757, 600 rows (three waves) 7397 -> 2120.
+// with 65 rows 942 -> 757, 600 rows (three waves) 7397 -> 2120.  (Both sides have become about a tenth to a quarter faster since; the line
+// stays, for moving it would change the bits of the calls between.)
 bool smc_prefill_q6k_supported(const smc_ctx *ctx, const smc_weight *w, int M)
 {
     if (w->dtype != SMC_Q6_K || w->N % TM || w->K % 256 || M < 64 || !w->q6u) return false;
