@@ -106,6 +106,26 @@ def test_dense_matmul_tile_widths_of_short_prompts(cuda, dev, n):
     cuda.release(h)
 
 
+@pytest.mark.parametrize("m,n,k", [(33, 40, 512), (96, 1024, 1024), (128, 1184, 1016), (65, 1184, 1080), (96, 2336, 3072), (100, 2400, 520), (300, 200, 4100 // 4 * 8)])
+def test_dense_matmul_with_k_shared_by_a_cluster(cuda, dev, m, n, k):
+    """Few tiles over a long K: two or four CTAs share a tile and K, in whole and ragged steps of 64.  fp32 sums of exact products: against
+    64 bits, 1e-5 of the norms."""
+    import torch
+
+    from sharpmind_b200 import ops
+
+    g = torch.Generator(device="cuda").manual_seed(m + n + k)
+    w = torch.randn((n, k), generator=g, device="cuda").to(torch.bfloat16)
+    x = torch.randn((m, k), generator=g, device="cuda")
+    h = cuda.register_dev(w.view(torch.uint8).reshape(-1), ops.QuantDType.BF16, n, k, repack=False)
+    got = dev.qmatmul(x, h, ops.Mode.ACT_BF16).double()
+    x16 = x.to(torch.bfloat16).double()
+    bound = 1e-5 * x16.norm(dim=1)[:, None] * w.double().norm(dim=1)[None]
+    assert bool(((got - x16 @ w.double().T).abs() <= bound).all())
+    cuda.release(h)
+    assert cuda.device_status() == 0
+
+
 @pytest.mark.parametrize("n", [8, 96, 1000])
 @pytest.mark.parametrize("offset", [0.0, 1.0])
 def test_scaled_add_rmsnorm(dev, n, offset):
