@@ -349,11 +349,13 @@ sdpa_prefill_tc_kernel(const float *__restrict__ q, const uint8_t *__restrict__ 
         constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(ROWS >> 4) << 24);
         constexpr uint32_t ID_S = IDESC | ((uint32_t)(CHUNK >> 3) << 17), ID_O = IDESC | ((uint32_t)(HD >> 3) << 17);
         constexpr int A_PART[6] = {1, 0, 2, 0, 1, 0}, B_PART[6] = {1, 2, 0, 1, 0, 0};  // smallest products first
+        bool k_there = false, v_there = false;  // the next chunk's planes, as far as is known
         auto scores = [&](int c) {
             const int st = c % STAGES;
-            smc_tc_wait(bar(FULL_K + st), (uint32_t)(c / STAGES) & 1u, abort_flag, status);
+            if (!k_there) smc_tc_wait(bar(FULL_K + st), (uint32_t)(c / STAGES) & 1u, abort_flag, status);
             smc_tc_wait(bar(S_FREE), (uint32_t)(c & 1) ^ 1u, abort_flag, status);
             smc_tc_fence_after();
+            k_there = smc_mbar_test(bar(FULL_K + (c + 1) % STAGES), (uint32_t)((c + 1) / STAGES) & 1u);
             const uint64_t k0 = desc(sbase + (uint32_t)st * S::STAGE, 128, HD / 8 * 128);
 #pragma unroll
             for (int ks = 0; ks < HD / 16; ++ks) {
@@ -371,9 +373,10 @@ sdpa_prefill_tc_kernel(const float *__restrict__ q, const uint8_t *__restrict__ 
         scores(0);
 #pragma unroll 1
         for (int c = 0; c < chunks; ++c) {
-            if (c + 1 < chunks) scores(c + 1);
             const int st = c % STAGES;
-            smc_tc_wait(bar(FULL_V + st), (uint32_t)(c / STAGES) & 1u, abort_flag, status);
+            v_there = smc_mbar_test(bar(FULL_V + st), (uint32_t)(c / STAGES) & 1u);
+            if (c + 1 < chunks) scores(c + 1);
+            if (!v_there) smc_tc_wait(bar(FULL_V + st), (uint32_t)(c / STAGES) & 1u, abort_flag, status);
 #pragma unroll 1
             for (int u = 0; u < 2; ++u) {
                 smc_tc_wait(bar(P_FULL), (uint32_t)u, abort_flag, status);

@@ -421,14 +421,17 @@ __global__ void __launch_bounds__(192, 1) dense_tc_kernel(const __grid_constant_
         if (lane == 0) {
             int st = 0;
             uint32_t ph = 1;
+            bool free = true;  // the slot, as far as is known
             for (int t = tile0; t < tiles; t += tstep) {
                 const int m0 = (t % mt) * TC_M, n0 = (t / mt) * BN;
                 for (int k = k0; k < k1; ++k) {
-                    smc_tc_wait(empty(st), ph, abort_flag, status);
-                    smc_mbar_expect_tx(full(st), S::STAGE);
-                    smc_tma_2d(sbase + (uint32_t)st * S::STAGE, &map_x, k * TC_K, m0, full(st));
-                    smc_tma_2d(sbase + (uint32_t)st * S::STAGE + S::A_BYTES, &map_w, k * TC_K, n0, full(st));
+                    if (!free) smc_tc_wait(empty(st), ph, abort_flag, status);
+                    const uint32_t at = sbase + (uint32_t)st * S::STAGE, bar = full(st);
                     if (++st == S::STAGES) st = 0, ph ^= 1;
+                    free = smc_mbar_test(empty(st), ph);
+                    smc_mbar_expect_tx(bar, S::STAGE);
+                    smc_tma_2d(at, &map_x, k * TC_K, m0, bar);
+                    smc_tma_2d(at + S::A_BYTES, &map_w, k * TC_K, n0, bar);
                 }
             }
         }
@@ -437,19 +440,21 @@ __global__ void __launch_bounds__(192, 1) dense_tc_kernel(const __grid_constant_
             constexpr uint32_t IDESC = smc_tc_idesc_bf16(TC_M, BN);
             int st = 0, n = 0;
             uint32_t ph = 0;
+            bool there = false;  // the stage, as far as is known
             for (int t = tile0; t < tiles; t += tstep, ++n) {
                 const int buf = n & 1;
                 smc_tc_wait(acc_empty(buf), (uint32_t)(((n >> 1) & 1) ^ 1), abort_flag, status);
-                smc_tc_fence_after();
                 const uint32_t d = tmem + (uint32_t)(buf * BN);
                 for (int k = k0; k < k1; ++k) {
-                    smc_tc_wait(full(st), ph, abort_flag, status);
+                    if (!there) smc_tc_wait(full(st), ph, abort_flag, status);
                     smc_tc_fence_after();
                     const uint64_t da = smc_tc_desc_sw128(sbase + (uint32_t)st * S::STAGE), db = smc_tc_desc_sw128(sbase + (uint32_t)st * S::STAGE + S::A_BYTES);
+                    const uint32_t done = empty(st);
+                    if (++st == S::STAGES) st = 0, ph ^= 1;
+                    there = smc_mbar_test(full(st), ph);
 #pragma unroll
                     for (int kk = 0; kk < TC_K / 16; ++kk) smc_tc_mma(d, da + 2 * kk, db + 2 * kk, IDESC, k > k0 || kk > 0 ? 1u : 0u);
-                    smc_tc_commit(empty(st));
-                    if (++st == S::STAGES) st = 0, ph ^= 1;
+                    smc_tc_commit(done);
                 }
                 smc_tc_commit(acc_full(buf));
             }

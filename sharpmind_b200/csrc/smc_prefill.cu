@@ -32,6 +32,7 @@
 #include <stdlib.h>
 
 #include "smc_common.cuh"
+#include "smc_tc.cuh"
 
 namespace {
 
@@ -363,14 +364,17 @@ prefill_q4k_kernel(const uint8_t *__restrict__ raw, const __half *__restrict__ i
             const uint64_t aux_desc0 = smem_desc(sbase + OFF_AUX, 128, 256);  // aux buffer 0, A''
             constexpr uint64_t U_SLOT = SLOT_BYTES >> 4, U_LO = B_BYTES >> 4, U_KK = 256 >> 4;
             constexpr uint64_t U_AUX = AUX_BYTES >> 4, U_BM = AM_BYTES >> 4, U_BM2 = (AM_BYTES + TN * 16 * 2) >> 4;
+            bool there = false, free = true;  // the next stage's weights, the next block's accumulator, as far as is known
             for (int sb = 0; sb < nsb; ++sb) {
                 const int buf = sb & 1;
-                mbar_wait(bar(BAR_ACC_EMPTY + buf), (uint32_t)(((sb >> 1) & 1) ^ 1), abort_flag, status);
+                if (!free) mbar_wait(bar(BAR_ACC_EMPTY + buf), (uint32_t)(((sb >> 1) & 1) ^ 1), abort_flag, status);
                 const uint32_t acc_d = tmem_base + COL_ACC_D + (uint32_t)buf * 128u;
 #pragma unroll
                 for (int g = 0; g < NA; ++g) {
-                    mbar_wait(bar(BAR_FULL_A + g), (uint32_t)(sb & 1), abort_flag, status);
+                    if (!there) mbar_wait(bar(BAR_FULL_A + g), (uint32_t)(sb & 1), abort_flag, status);
                     tc_fence_after();
+                    there = smc_mbar_test(bar(BAR_FULL_A + (g + 1) % NA), (uint32_t)((sb + (g + 1) / NA) & 1));
+                    if (g == NA - 1) free = smc_mbar_test(bar(BAR_ACC_EMPTY + (buf ^ 1)), (uint32_t)((((sb + 1) >> 1) & 1) ^ 1));
                     const uint64_t bh = b_desc0 + (uint64_t)g * U_SLOT;
                     const uint32_t a0 = tmem_base + COL_A + (uint32_t)g * 32u;
                     if (g == 0) {
@@ -644,14 +648,17 @@ prefill_q6k_kernel(const uint8_t *__restrict__ q6u, const __nv_bfloat16 *__restr
             const uint64_t b_desc0 = smem_desc(sbase, 128, 1024);
             constexpr uint64_t U_SLOT = Q6_SLOT >> 4, U_X = B_BYTES >> 4, U_KK = 256 >> 4;
             int slot = 0;
+            bool there = false, free = true;  // the next stage's weights and accumulator, as far as is known
             for (int sb = 0; sb < nsb; ++sb) {
 #pragma unroll
                 for (int g = 0; g < NA; ++g) {
                     const int buf = g & 1, use = 2 * sb + (g >> 1);  // which time this accumulator is filled
                     const uint32_t acc_d = tmem_base + (uint32_t)buf * 128u;
-                    mbar_wait(bar(Q6_ACC_EMPTY + buf), (uint32_t)((use & 1) ^ 1), abort_flag, status);
-                    mbar_wait(bar(Q6_FULL_A + g), (uint32_t)(sb & 1), abort_flag, status);
+                    if (!free) mbar_wait(bar(Q6_ACC_EMPTY + buf), (uint32_t)((use & 1) ^ 1), abort_flag, status);
+                    if (!there) mbar_wait(bar(Q6_FULL_A + g), (uint32_t)(sb & 1), abort_flag, status);
                     tc_fence_after();
+                    there = smc_mbar_test(bar(Q6_FULL_A + (g + 1) % NA), (uint32_t)((sb + (g + 1) / NA) & 1));
+                    free = smc_mbar_test(bar(Q6_ACC_EMPTY + (buf ^ 1)), (uint32_t)(((2 * sb + ((g + 1) >> 1)) & 1) ^ 1));
                     const uint64_t x0 = b_desc0 + (uint64_t)slot * U_SLOT, x1 = x0 + U_X, x2 = x1 + U_X;
                     const uint32_t v_hi = tmem_base + Q6_COL_A + (uint32_t)g * 64u, v_lo = v_hi + 32;
                     auto products = [&](uint32_t v, uint64_t x, bool first) {

@@ -18,6 +18,18 @@ __device__ __forceinline__ void smc_tc_wait(uint32_t bar, uint32_t parity, volat
     *abort_flag = 1;
     atomicExch(status, 4);
 }
+// Has the phase completed?  Never blocks.  The answer takes some 280 clocks to come back on a busy SM, so a thread that feeds the tensor cores
+// asks for its next stage before it issues this one's MMAs and waits (smc_tc_wait) only where the answer was no.
+__device__ __forceinline__ bool smc_mbar_test(uint32_t bar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 __device__ __forceinline__ void smc_tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void smc_tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void smc_tc_commit(uint32_t bar)
