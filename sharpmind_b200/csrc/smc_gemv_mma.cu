@@ -10,12 +10,14 @@
 // split K) are added in warp order: the result of a row does not depend on the batch size or on the other
 // rows (for any batch >= 2; the one-row kernels use a different summation tree).
 //
-// Layout choices.  A CTA owns 32 weight rows (two m16 tiles) and all tokens; its 8 warps take interleaved
-// k groups and meet in shared memory at the end.  Fragments are loaded straight from global memory as 8-byte
-// words: the dot product does not care about the order of k inside a block, so MMA k index 4*tg + i is bound to
-// byte 8*tg + i and 16 + 4*tg + i to byte 8*tg + 4 + i of the block, for weights and activations alike; a
-// quad of lanes then reads one whole 32-byte sector per row.  Scales are loaded once per lane (lane = row for
-// the weights, lane = token for the activations) and handed round with shuffles.
+// Three kinds of kernel share these sums, bit for bit:
+//   split   Q6_K below 64 rows, and Q8_0 / Q4_K where no other has a better form: a CTA owns 32 weight rows (two m16 tiles) and a pass of tokens, its 8 (16) warps take
+//           interleaved k groups and meet in shared memory.  Fragments come straight from global memory as 8-byte words: the dot product does not care
+//           about the order of k inside a block, so MMA k index 4*tg + i is bound to byte 8*tg + i and 16 + 4*tg + i to byte 8*tg + 4 + i of the
+//           block, for weights and activations alike; a quad of lanes then reads one whole 32-byte sector per row.  Scales are loaded once per
+//           lane (lane = row for the weights, lane = token for the activations) and handed round with shuffles.
+//   tile    prompt-sized batches of Q8_0 and Q6_K: no split, operands staged in shared memory.
+//   staged  2 to 63 rows of Q8_0, small batches of Q4_K: the split, operands staged in shared memory.
 #include "smc_common.cuh"
 
 #include <type_traits>
@@ -68,14 +70,13 @@ __device__ __forceinline__ void reduce_and_store(float (*red)[TOK][RED_LD], cons
 
 // ------------------------------------------------------------------------------------------ Q8_0
 // Planes: quants [N][K] int8, scales [N][K/32] fp16.  K % 128 == 0; a warp works on groups of four blocks.
-template <int NT>
-__global__ void __launch_bounds__(256, NT > 4 ? 1 : 2)
+// Batches of 64 rows and more that the tile kernel (below) does not take, in passes of 64 tokens that share every weight fragment and scale.
+constexpr int Q8_PASS = 64;
+__global__ void __launch_bounds__(256, 1)
 gemv_mma_q8_0_kernel(const int8_t *__restrict__ wq, const __half *__restrict__ wd, const int8_t *__restrict__ xq,
                      const float *__restrict__ xd, float *__restrict__ out, int N, int K, int M)
 {
-    // NT token tiles of 8 per pass: 1, 2, 4 for up to 32 rows; 8 for prompt-sized batches (64 tokens share every weight
-    // fragment and scale, which halves the passes over the matrix)
-    constexpr int TOK = NT > 4 ? 64 : 32, XR = TOK / 32;
+    constexpr int TOK = Q8_PASS, NT = TOK / 8, XR = TOK / 32;
     extern __shared__ __align__(16) float red_q8[];
     float (*red)[TOK][RED_LD] = reinterpret_cast<float (*)[TOK][RED_LD]>(red_q8);
     smc_grid_dep_sync();
@@ -154,11 +155,12 @@ gemv_mma_q8_0_kernel(const int8_t *__restrict__ wq, const __half *__restrict__ w
 // GGUF blocks of 144 bytes: d, dmin (fp16), 12 packed scale / min bytes, 128 nibble bytes; the 32 bytes of
 // group gq hold sub-block 2*gq in the low nibbles and 2*gq + 1 in the high ones.  K % 256 == 0; a warp works
 // on whole 256-element blocks.  out += d*sc_j * dx * isum  -  dmin*m_j * (dx * sum(xq))  per sub-block.
-template <int NT>
-__global__ void __launch_bounds__(256, NT > 2 ? 1 : 2)
+// Batches of 17 rows and more, in passes of 32, where the staged kernel (below) has no better form.
+__global__ void __launch_bounds__(256, 1)
 gemv_mma_q4_K_kernel(const uint8_t *__restrict__ raw, const int8_t *__restrict__ xq, const float *__restrict__ xd,
                      const float *__restrict__ xsd, float *__restrict__ out, int N, int K, int M)
 {
+    constexpr int NT = 4;
     __shared__ float red[MMA_WARPS][32][RED_LD];
     smc_grid_dep_sync();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tg = lane & 3;
@@ -290,7 +292,7 @@ gemv_mma_q6_K_kernel(const uint8_t *__restrict__ q6u, const int8_t *__restrict__
 {
     // NW warps split K: 8 (two CTAs per SM), or 16 in one CTA per SM for rows of 8192 elements and more
     extern __shared__ __align__(16) float red_dyn[];
-    float (*red)[32][RED_LD] = reinterpret_cast<float (*)[32][RED_LD]>(red_dyn);
+    float (*red)[8 * NT][RED_LD] = reinterpret_cast<float (*)[8 * NT][RED_LD]>(red_dyn);
     smc_grid_dep_sync();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tg = lane & 3;
     const int r0 = blockIdx.x * MMA_ROWS;
@@ -368,7 +370,7 @@ gemv_mma_q6_K_kernel(const uint8_t *__restrict__ q6u, const int8_t *__restrict__
                 }
             }
         }
-        reduce_and_store<NT, NW>(red, acc, out, N, M, r0, t0);
+        reduce_and_store<NT, NW, 8 * NT>(red, acc, out, N, M, r0, t0);
     }
 }
 
@@ -657,6 +659,286 @@ gemv_mma_tile_kernel(const uint8_t *__restrict__ w, const __half *__restrict__ w
             }
 }
 
+// ------------------------------------------------------------------------------------------ 2 .. 63 rows, Q8_0 and Q4_K, staged
+// The same sums again, for batches that the tiles above are too large for.  A CTA takes jobs of 32 WR weight rows x 8 NT tokens; its 8 / WR groups of WR warps
+// take the classes of K groups as the warps of the split kernels do (a group of fewer than eight takes several, one after the other)
+// and meet in shared memory, where each output is added up in class order: the same bits.  Each group of warps has its own ring of S stages (a
+// stage: a class's next 128 elements of Q8_0 or 256 of Q4_K, of all rows and tokens of the job), filled by asynchronous copies, and with one warp to a
+// group it waits for nobody else's.  A CTA is one per SM and goes from job to job with its copies running ahead; the first weights are asked
+// for before the predecessor is waited for.  Layout in a stage, scales and products are the tile kernel's.  Q4_K: a warp writes its rows'
+// d * sc and dmin * m of a 256-block to a table once, instead of handing them round by shuffles.
+// What bounds it: the MMAs with their scaling are 24 of 57 us (Q4_K 28672 x 4096, 32 rows, 25 - 30 clocks each) and 6 of 29 with 6 rows, the weights' bytes 10; the
+// rest is a warp's own chain of copy, wait, fragments and sums, with one or two steps in flight and eight warps to an SM.
+// The split kernels that ran here had their fragments as 8-byte loads from global memory, just in time, and 8 shuffles per MMA's tokens.
+// Measured, us (before): Q4_K 28672 x 4096 with 6 rows 33.5 -> 28.8, 16 45.2 -> 40.5, 32 70.9 -> 57.5; 4096 x 14336, 6 20.5 -> 14.5; 6144 x 4096, 32
+// 22.7 -> 18.6; 1024 x 4096, 32 12.4 -> 6.5; Q8_0 1024 x 3072, 32 10.4 -> 6.1; 4096 x 14336, 6 24.7 -> 16.5, 16 27.1 -> 20.7, 32 37.1 -> 25.3; 6144 x
+// 1024, 32 8.7 -> 8.3.
+template <bool Q4, int WR, int NT, int S>
+struct StageShape {
+    static constexpr int WK = MMA_WARPS / WR, GROUP = 32 * WR;
+    static constexpr int ROWS = 32 * WR, TOK = 8 * NT, KG = Q4 ? 256 : 128, NB = KG / 32;
+    static constexpr int WROW = 144, XROW = KG + 16, DXS = 2 * NT;  // Q8_0: 128 codes and their four scales; Q4_K: a block
+    static constexpr int DXB = NB * 4 * DXS * 4;
+    static constexpr int OFF_X = ROWS * WROW, OFF_DX = OFF_X + TOK * XROW, OFF_SX = OFF_DX + DXB, STAGE = OFF_SX + (Q4 ? DXB : 0);
+    static constexpr int TAB = Q4 ? 32 * 80 : 0;  // a warp's rows' eight (d sc, dmin m), 64 bytes on 80
+    static constexpr int OFF_TAB = WK * S * STAGE, OFF_RED = OFF_TAB + MMA_WARPS * TAB;
+    static constexpr int RLD = ROWS + 4, RED = WK * TOK * RLD * 4;
+    static constexpr int REDS = OFF_RED + 2 * RED <= 227 * 1024 ? 2 : 1;  // two: the next round's partial sums need not wait for this one's readers
+    static constexpr int SMEM = OFF_RED + REDS * RED;
+    static_assert(STAGE % 16 == 0 && OFF_TAB % 16 == 0 && SMEM <= 227 * 1024, "shared memory");
+};
+
+template <bool Q4, int WR, int NT, int S>
+__global__ void __launch_bounds__(32 * MMA_WARPS, 1)
+gemv_mma_staged_kernel(const uint8_t *__restrict__ w, const __half *__restrict__ wd, const int8_t *__restrict__ xq, const float *__restrict__ xd,
+                       const float *__restrict__ xsd, float *__restrict__ out, int N, int K, int M, int passes, int jobs)
+{
+    using P = StageShape<Q4, WR, NT, S>;
+    constexpr int WK = P::WK;
+    extern __shared__ __align__(16) uint8_t sm_staged[];
+    const uint32_t base = smem_at(sm_staged);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tg = lane & 3;
+    const int wk = warp / WR, wr = warp % WR, gt = threadIdx.x % P::GROUP;
+    const int nb = K / 32, ngroups = K / P::KG;
+    const uint32_t ring = base + (uint32_t)(wk * S) * P::STAGE;
+
+    // the step whose bytes are asked for next: job, class, K group
+    int a_job = blockIdx.x, a_cls = wk, a_gi = wk;
+    auto settle = [&]() {  // over classes that have no (more) steps
+        while (a_job < jobs && a_gi >= ngroups) {
+            a_cls += WK;
+            if (a_cls >= MMA_WARPS) a_cls = wk, a_job += gridDim.x;
+            a_gi = a_cls;
+            if (wk >= ngroups) a_job = jobs;  // none of this group's classes has any
+        }
+    };
+    // What lies past the last row or token is not loaded (nor stored: outputs do not mix).
+    auto request_weights = [&](int slot) {
+        const uint32_t st = ring + (uint32_t)slot * P::STAGE;
+        const int r0 = a_job / passes * P::ROWS;
+        constexpr int PIECES = Q4 ? 9 : 8;
+#pragma unroll
+        for (int i = 0; i < P::ROWS * PIECES / P::GROUP; ++i) {
+            const int e = gt + i * P::GROUP, r = e / PIECES, c = e % PIECES;
+            if (r0 + r >= N) break;
+            const size_t row = (size_t)(r0 + r);
+            copy_async<16>(st + (uint32_t)(r * P::WROW + 16 * c), Q4 ? w + (row * ngroups + a_gi) * 144 + 16 * c : w + row * K + a_gi * 128 + 16 * c);
+        }
+        if (!Q4 && r0 + gt < N) copy_async<8>(st + (uint32_t)(gt * P::WROW + 128), wd + (size_t)(r0 + gt) * nb + a_gi * 4);
+    };
+    auto request_tokens = [&](int slot) {
+        const uint32_t st = ring + (uint32_t)slot * P::STAGE;
+        const int t0 = a_job % passes * P::TOK;
+        constexpr int XP = P::KG / 16;
+#pragma unroll
+        for (int i = 0; i < P::TOK * XP / P::GROUP; ++i) {
+            const int e = gt + i * P::GROUP, t = e / XP, c = e % XP;
+            if (t0 + t < M) copy_async<16>(st + (uint32_t)(P::OFF_X + t * P::XROW + 16 * c), xq + (size_t)(t0 + t) * K + a_gi * P::KG + 16 * c);
+        }
+#pragma unroll
+        for (int i = 0; i < (P::TOK * P::NB + P::GROUP - 1) / P::GROUP; ++i) {
+            const int e = gt + i * P::GROUP, t = e / P::NB, b = e % P::NB;
+            if (t < P::TOK && t0 + t < M) {
+                const uint32_t at = 4u * (uint32_t)((b * 4 + ((t & 7) >> 1)) * P::DXS + 2 * (t >> 3) + (t & 1));
+                const size_t from = (size_t)(t0 + t) * nb + a_gi * P::NB + b;
+                copy_async<4>(st + P::OFF_DX + at, xd + from);
+                if (Q4) copy_async<4>(st + P::OFF_SX + at, xsd + from);
+            }
+        }
+    };
+    auto advance = [&]() { a_gi += MMA_WARPS, settle(); };
+    static_assert(P::ROWS == P::GROUP && P::ROWS * (Q4 ? 9 : 8) % P::GROUP == 0 && P::TOK * (P::KG / 16) % P::GROUP == 0, "copies per thread");
+
+    settle();
+    const int f_job = a_job, f_cls = a_cls, f_gi = a_gi;
+#pragma unroll
+    for (int i = 0; i < S - 1; ++i)
+        if (a_job < jobs) request_weights(i), advance();
+    a_job = f_job, a_cls = f_cls, a_gi = f_gi;
+    smc_grid_dep_sync();
+#pragma unroll
+    for (int i = 0; i < S - 1; ++i) {  // (the first of these groups holds all the weights)
+        if (a_job < jobs) request_tokens(i), advance();
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+
+    // this lane's ldmatrix rows
+    const uint32_t a_off = (uint32_t)((wr * 32 + (lane & 7) + 8 * ((lane >> 3) & 1)) * P::WROW + 16 * (lane >> 4));
+    const uint32_t dx_off = (uint32_t)(P::OFF_DX + tg * P::DXS * 4);
+    const uint32_t tab = base + P::OFF_TAB + (uint32_t)warp * P::TAB;
+    f32x2 acc[2][NT][2];  // [16-row tile][token tile][rows g, g + 8]: tokens 2 tg, 2 tg + 1
+    auto scale_add = [&](f32x2 (&a)[2], const int (&c)[4], const f32x2 (&ws)[2], f32x2 dx) {
+        a[0] = fma_x2(pair_x2((float)c[0], (float)c[1]), mul_x2(ws[0], dx), a[0]);
+        a[1] = fma_x2(pair_x2((float)c[2], (float)c[3]), mul_x2(ws[1], dx), a[1]);
+    };
+    auto token_scales = [&](uint32_t at, f32x2 (&v)[NT]) {
+        if constexpr (NT == 1) asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v[0]) : "r"(at) : "memory");
+        else {
+#pragma unroll
+            for (int t = 0; t < NT; t += 2) asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(v[t]), "=l"(v[t + 1]) : "r"(at + 8u * t) : "memory");
+        }
+    };
+    auto token_codes = [&](uint32_t st, int k, uint32_t (&b)[NT][2]) {  // of the 32-element block at byte k of the stage's token rows
+        const uint32_t at = st + P::OFF_X + (uint32_t)((lane & 7) * P::XROW + k + 16 * ((lane >> 3) & 1));
+        if constexpr (NT == 1) ldsm2(at, b[0][0], b[0][1]);
+        else {
+#pragma unroll
+            for (int t = 0; t < NT; t += 2) ldsm4(at + (uint32_t)((8 * t + 8 * (lane >> 4)) * P::XROW), b[t][0], b[t][1], b[t + 1][0], b[t + 1][1]);
+        }
+    };
+    auto step_q8 = [&](uint32_t st) {
+        uint2 dw[2][2];
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) dw[mt][h] = lds8(st + (uint32_t)((wr * 32 + 16 * mt + 8 * h + g) * P::WROW + 128));
+#pragma unroll
+        for (int kb = 0; kb < 4; ++kb) {
+            uint32_t a[2][4], b[NT][2];
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt) ldsm4(st + a_off + (uint32_t)(16 * mt * P::WROW + 32 * kb), a[mt][0], a[mt][1], a[mt][2], a[mt][3]);
+            token_codes(st, 32 * kb, b);
+            f32x2 dx[NT], ws[2][2];
+            token_scales(st + dx_off + (uint32_t)(kb * 16 * P::DXS), dx);
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const uint32_t two = (kb & 2) ? dw[mt][h].y : dw[mt][h].x;
+                    const float d = smc_h2f((uint16_t)((kb & 1) ? (two >> 16) : (two & 0xFFFFu)));
+                    ws[mt][h] = pair_x2(d, d);
+                }
+#pragma unroll
+            for (int t = 0; t < NT; ++t)
+#pragma unroll
+                for (int mt = 0; mt < 2; ++mt) {
+                    int c[4];
+                    mma_s8(c, a[mt][0], a[mt][1], a[mt][2], a[mt][3], b[t][0], b[t][1]);
+                    scale_add(acc[mt][t], c, ws[mt], dx[t]);
+                }
+        }
+    };
+    auto step_q4 = [&](uint32_t st) {
+        {
+            uint4 hdr;
+            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(hdr.x), "=r"(hdr.y), "=r"(hdr.z), "=r"(hdr.w) : "r"(st + (uint32_t)((wr * 32 + lane) * P::WROW)) : "memory");
+            const float d = smc_h2f((uint16_t)(hdr.x & 0xFFFFu)), dmin = smc_h2f((uint16_t)(hdr.x >> 16));
+            __syncwarp();  // the previous step's table has been read
+#pragma unroll
+            for (int i = 0; i < 8; i += 2) {
+                int s0, m0, s1, m1;
+                smc_k4_scale_min(hdr.y, hdr.z, hdr.w, i, s0, m0), smc_k4_scale_min(hdr.y, hdr.z, hdr.w, i + 1, s1, m1);
+                asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(tab + (uint32_t)(lane * 80 + 8 * i)), "f"(d * (float)s0), "f"(dmin * (float)m0), "f"(d * (float)s1),
+                             "f"(dmin * (float)m1)
+                             : "memory");
+            }
+            __syncwarp();
+        }
+#pragma unroll
+        for (int gq = 0; gq < 4; ++gq) {
+            uint32_t raw[2][4];
+            float4 sm[2][2];
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt) {
+                ldsm4(st + a_off + (uint32_t)(16 * mt * P::WROW + 16 + 32 * gq), raw[mt][0], raw[mt][1], raw[mt][2], raw[mt][3]);
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];"
+                                 : "=f"(sm[mt][h].x), "=f"(sm[mt][h].y), "=f"(sm[mt][h].z), "=f"(sm[mt][h].w)
+                                 : "r"(tab + (uint32_t)((16 * mt + 8 * h + g) * 80 + 16 * gq))
+                                 : "memory");
+            }
+#pragma unroll
+            for (int hi = 0; hi < 2; ++hi) {
+                const int j = 2 * gq + hi;  // sub-block
+                uint32_t b[NT][2];
+                token_codes(st, 32 * j, b);
+                f32x2 dx[NT], sx[NT], ws[2][2], wm[2][2];
+                token_scales(st + dx_off + (uint32_t)(j * 16 * P::DXS), dx);
+                token_scales(st + dx_off + (uint32_t)(P::DXB + j * 16 * P::DXS), sx);
+#pragma unroll
+                for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const float s = hi ? sm[mt][h].z : sm[mt][h].x, m = -(hi ? sm[mt][h].w : sm[mt][h].y);
+                        ws[mt][h] = pair_x2(s, s), wm[mt][h] = pair_x2(m, m);
+                    }
+#pragma unroll
+                for (int t = 0; t < NT; ++t)
+#pragma unroll
+                    for (int mt = 0; mt < 2; ++mt) {
+                        uint32_t a[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) a[i] = (hi ? raw[mt][i] >> 4 : raw[mt][i]) & 0x0F0F0F0Fu;
+                        int c[4];
+                        mma_s8(c, a[0], a[1], a[2], a[3], b[t][0], b[t][1]);
+                        scale_add(acc[mt][t], c, ws[mt], dx[t]);
+                        acc[mt][t][0] = fma_x2(wm[mt][0], sx[t], acc[mt][t][0]), acc[mt][t][1] = fma_x2(wm[mt][1], sx[t], acc[mt][t][1]);
+                    }
+            }
+        }
+    };
+
+    constexpr int OWN = P::ROWS * P::TOK / (32 * MMA_WARPS);  // outputs of a thread
+    static_assert(OWN * 32 * MMA_WARPS == P::ROWS * P::TOK, "outputs per thread");
+    int slot = 0, round = 0;
+#pragma unroll 1
+    for (int job = blockIdx.x; job < jobs; job += gridDim.x) {
+        float own[OWN];
+#pragma unroll 1
+        for (int cls = wk; cls < MMA_WARPS; cls += WK) {
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+                for (int t = 0; t < NT; ++t) acc[mt][t][0] = acc[mt][t][1] = 0ull;
+#pragma unroll 1
+            for (int gi = cls; gi < ngroups; gi += MMA_WARPS) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(S - 2) : "memory");
+                // the step has landed for the whole group of warps, and all of it is through with the slot that is refilled
+                if constexpr (WR == 1) __syncwarp();
+                else asm volatile("bar.sync %0, %1;" ::"r"(1 + wk), "n"(P::GROUP) : "memory");
+                if (a_job < jobs) {
+                    const int next = slot == 0 ? S - 1 : slot - 1;
+                    request_weights(next), request_tokens(next), advance();
+                }
+                asm volatile("cp.async.commit_group;" ::: "memory");
+                const uint32_t st = ring + (uint32_t)slot * P::STAGE;
+                if constexpr (Q4) step_q4(st);
+                else step_q8(st);
+                if (++slot == S) slot = 0;
+            }
+            float *red = reinterpret_cast<float *>(sm_staged + P::OFF_RED + (P::REDS == 2 ? (round & 1) * P::RED : 0));
+            if (P::REDS == 1 && round) __syncthreads();
+            ++round;
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+                for (int t = 0; t < NT; ++t)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        float *at = red + (wk * P::TOK + 8 * t + 2 * tg) * P::RLD + wr * 32 + 16 * mt + 8 * h + g;
+                        unpair_x2(acc[mt][t][h], at[0], at[P::RLD]);
+                    }
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < OWN; ++i) {
+                const int e = threadIdx.x + i * 32 * MMA_WARPS, row = e % P::ROWS, tok = e / P::ROWS;
+                float s = cls == wk ? red[tok * P::RLD + row] : own[i] + red[tok * P::RLD + row];
+#pragma unroll
+                for (int c = 1; c < WK; ++c) s += red[(c * P::TOK + tok) * P::RLD + row];
+                own[i] = s;
+            }
+        }
+        const int r0 = job / passes * P::ROWS, t0 = job % passes * P::TOK;
+#pragma unroll
+        for (int i = 0; i < OWN; ++i) {
+            const int e = threadIdx.x + i * 32 * MMA_WARPS, row = r0 + e % P::ROWS, tok = t0 + e / P::ROWS;
+            if (row < N && tok < M) out[(size_t)tok * N + row] = own[i];
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
 }  // namespace
 
 bool smc_mma_supported(const smc_weight *w, int M)
@@ -693,6 +975,53 @@ static int prompt_tile(const smc_ctx *ctx, const smc_weight *w, int M)
     return nt;
 }
 
+// The form of the staged kernel for a call; wr = 0: the Q4_K kernel that splits K over warps.
+// A CTA per SM takes its jobs in rounds, each so many us per 1024 elements of K (and some 4 us a launch, the same for all): measured with one job per SM and
+// with many at K = 1024 .. 28672 and 2 .. 63 rows, where the choice by these rates was never slower than the kernels it replaces.  Up to 8 tokens there is the one
+// form; 9 .. 16 in one tile or two; more in tiles of 8, 16 or 32.  Narrow tiles win where weight rows are few (Q8_0 1024 x 3072, 32 tokens: 6.1 us in
+// tiles of 8, 8.3 of 32; 4096 x 14336: 48 and 25).  Q4_K at 32 tokens has no room for 32 rows' rings: 64 or 128 rows to a CTA pay where they come out
+// even (us, split kernel / 64 / 128 rows: 28672 x 4096 70.9 / 61.7 / 57.5, 6144 x 4096 22.7 / 18.6 / 30, 4096 x 4096 14.2 / 18.6 / 30).
+struct StagedForm {
+    int wr, nt;
+};
+static StagedForm staged_form(const smc_ctx *ctx, const smc_weight *w, int M)
+{
+    const bool q4 = w->dtype == SMC_Q4_K;
+    double best = 1e30;
+    StagedForm form{0, 0};
+    auto offer = [&](int wr, int nt, double us) {
+        const long long jobs = (long long)((w->N + 32 * (wr ? wr : 1) - 1) / (32 * (wr ? wr : 1))) * ((M + 8 * nt - 1) / (8 * nt));
+        const double t = (double)((jobs + ctx->sm_count - 1) / ctx->sm_count) * us;
+        if (t < best) best = t, form = {wr, wr ? nt : 0};
+    };
+    if (M > 16) q4 ? (offer(0, 4, 2.0), offer(4, 4, 6.6), offer(2, 4, 3.6)) : offer(1, 4, 1.5);
+    if (M > 8) offer(1, 2, 1.2);
+    offer(1, 1, q4 ? 0.75 : 0.85);
+    return form;
+}
+
+// The split kernels live on L1: a lane's words are pieces of lines that its neighbours ask for.  An SM that a kernel with a large ring has left keeps its division
+// into L1 and shared memory unless the next kernel asks for another, so these ask for no more shared memory than their CTAs take.  With the
+// staged kernel around them and without this, a Q4_K / Q6_K decoder of 32 layers took 4322 us for 6 rows and 6376 for 32 (3547 and 5257 with it; before the staged kernel
+// 4160 and 5921).  The same request from the kernels between the matmuls cost 6 % of the 6 rows.
+template <class Kernel>
+static void keep_l1(Kernel kernel, size_t smem, int ctas)
+{
+    cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)((ctas * (smem + 1024) * 100 + 228 * 1024 - 1) / (228 * 1024)));
+}
+
+template <bool Q4, int WR, int NT, int S>
+static void launch_staged(smc_ctx *ctx, const smc_q8act *a, const smc_weight *w, float *out, cudaStream_t s)
+{
+    using P = StageShape<Q4, WR, NT, S>;
+    const auto kernel = gemv_mma_staged_kernel<Q4, WR, NT, S>;
+    const int passes = (a->M + P::TOK - 1) / P::TOK, jobs = (w->N + P::ROWS - 1) / P::ROWS * passes;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, P::SMEM);
+    smc_launch_dep(ctx->use_pdl, kernel, dim3(jobs < ctx->sm_count ? jobs : ctx->sm_count), dim3(32 * MMA_WARPS), P::SMEM, s,
+                   Q4 ? (const uint8_t *)w->d_raw : (const uint8_t *)w->q8_qs, (const __half *)w->q8_d, (const int8_t *)a->q, (const float *)a->d, (const float *)a->sd, out,
+                   w->N, w->K, a->M, passes, jobs);
+}
+
 int smc_launch_gemv_mma(smc_ctx *ctx, const smc_q8act *a, const smc_weight *w, float *out, cudaStream_t s)
 {
     const int N = w->N, K = w->K, M = a->M;
@@ -710,27 +1039,24 @@ int smc_launch_gemv_mma(smc_ctx *ctx, const smc_q8act *a, const smc_weight *w, f
             pt == 6 ? go(gemv_mma_tile_kernel<true, 6, 2>, TileShape<true, 6>::SMEM, ncls) : go(gemv_mma_tile_kernel<true, 4, 2>, TileShape<true, 4>::SMEM, ncls);
         } else if (pt == 8) go(gemv_mma_tile_kernel<false, 8, 2>, TileShape<false, 8>::SMEM, 8);
         else pt == 6 ? go(gemv_mma_tile_kernel<false, 6, 2>, TileShape<false, 6>::SMEM, 8) : go(gemv_mma_tile_kernel<false, 4, 3>, TileShape<false, 4>::SMEM, 8);
+    } else if (w->dtype == SMC_Q8_0 && M >= 64) {
+        const size_t smem = (size_t)MMA_WARPS * Q8_PASS * RED_LD * sizeof(float);
+        cudaFuncSetAttribute(gemv_mma_q8_0_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        keep_l1(gemv_mma_q8_0_kernel, smem, 1);
+        smc_launch_dep(ctx->use_pdl, gemv_mma_q8_0_kernel, dim3((N + MMA_ROWS - 1) / MMA_ROWS, (M + Q8_PASS - 1) / Q8_PASS), dim3(256), smem, s, (const int8_t *)w->q8_qs,
+                       (const __half *)w->q8_d, (const int8_t *)a->q, (const float *)a->d, out, N, K, M);
     } else if (w->dtype == SMC_Q8_0) {
-        // prompt-sized batches: passes of 64 tokens
-        const int nt8 = M >= 64 ? 8 : nt;
-        const dim3 g8((N + MMA_ROWS - 1) / MMA_ROWS, (M + 8 * nt8 - 1) / (8 * nt8));
-        auto go8 = [&](auto kernel, int tok) {
-            const size_t smem = (size_t)MMA_WARPS * tok * RED_LD * sizeof(float);
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            smc_launch_dep(ctx->use_pdl, kernel, g8, dim3(256), smem, s, (const int8_t *)w->q8_qs, (const __half *)w->q8_d,
-                           (const int8_t *)a->q, (const float *)a->d, out, N, K, M);
-        };
-        if (nt8 == 1) go8(gemv_mma_q8_0_kernel<1>, 32);
-        else if (nt8 == 2) go8(gemv_mma_q8_0_kernel<2>, 32);
-        else if (nt8 == 4) go8(gemv_mma_q8_0_kernel<4>, 32);
-        else go8(gemv_mma_q8_0_kernel<8>, 64);
+        const StagedForm f = staged_form(ctx, w, M);
+        f.nt == 1 ? launch_staged<false, 1, 1, 3>(ctx, a, w, out, s)
+                  : f.nt == 2 ? launch_staged<false, 1, 2, 2>(ctx, a, w, out, s) : launch_staged<false, 1, 4, 2>(ctx, a, w, out, s);
     } else if (w->dtype == SMC_Q6_K) {
         // the warp count follows from K alone, so a row's bits depend neither on the batch nor on how the rows are
         // split across GPUs; long rows are where matrices of few rows (FFN down) need the extra warps per SM
         const bool wide = K >= 8192;
         auto go = [&](auto kernel, int nw) {
-            const size_t smem = (size_t)nw * 32 * RED_LD * sizeof(float);
+            const size_t smem = (size_t)nw * 8 * nt * RED_LD * sizeof(float);
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            keep_l1(kernel, smem, nw == 8 ? 2 : 1);
             smc_launch_dep(ctx->use_pdl, kernel, grid, dim3(nw * 32), smem, s, (const uint8_t *)w->q6u, (const int8_t *)a->q,
                            (const float *)a->d, out, N, K, M);
         };
@@ -744,12 +1070,12 @@ int smc_launch_gemv_mma(smc_ctx *ctx, const smc_q8act *a, const smc_weight *w, f
             else go(gemv_mma_q6_K_kernel<4, 8>, 8);
         }
     } else {
-        if (nt == 1) smc_launch_dep(ctx->use_pdl, gemv_mma_q4_K_kernel<1>, grid, dim3(256), 0, s, (const uint8_t *)w->d_raw, (const int8_t *)a->q,
-                           (const float *)a->d, (const float *)a->sd, out, N, K, M);
-        else if (nt == 2) smc_launch_dep(ctx->use_pdl, gemv_mma_q4_K_kernel<2>, grid, dim3(256), 0, s, (const uint8_t *)w->d_raw, (const int8_t *)a->q,
-                           (const float *)a->d, (const float *)a->sd, out, N, K, M);
-        else smc_launch_dep(ctx->use_pdl, gemv_mma_q4_K_kernel<4>, grid, dim3(256), 0, s, (const uint8_t *)w->d_raw, (const int8_t *)a->q,
-                           (const float *)a->d, (const float *)a->sd, out, N, K, M);
+        const StagedForm f = staged_form(ctx, w, M);
+        if (f.wr == 0) keep_l1(gemv_mma_q4_K_kernel, sizeof(float) * MMA_WARPS * 32 * RED_LD, 1), smc_launch_dep(ctx->use_pdl, gemv_mma_q4_K_kernel, grid, dim3(256), 0, s, (const uint8_t *)w->d_raw, (const int8_t *)a->q, (const float *)a->d,
+                                      (const float *)a->sd, out, N, K, M);
+        else if (f.wr == 4) launch_staged<true, 4, 4, 2>(ctx, a, w, out, s);
+        else if (f.wr == 2) launch_staged<true, 2, 4, 2>(ctx, a, w, out, s);
+        else f.nt == 2 ? launch_staged<true, 1, 2, 2>(ctx, a, w, out, s) : launch_staged<true, 1, 1, 3>(ctx, a, w, out, s);
     }
     SMC_LAUNCH_CHECK(ctx);
     return SMC_OK;

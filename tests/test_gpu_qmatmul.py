@@ -146,6 +146,33 @@ def test_prompt_tiles_keep_the_small_batch_bits(cuda, dev, dtype, n, m, ks):
         cuda.release(w)
 
 
+@pytest.mark.parametrize("dtype,n,ref_n,ref_m", [(Q8_0, 4700, 1000, 64), (Q8_0, 1000, 1000, 64), (Q4_K, 4700, 4000, 32), (Q4_K, 6100, 4000, 32), (Q4_K, 18900, 4000, 32),
+                                                 (Q4_K, 700, 700, 32)])
+@pytest.mark.parametrize("k", [256, 2304, 4352])
+def test_staged_forms_keep_the_split_kernels_bits(cuda, dev, dtype, n, ref_n, ref_m, k):
+    """The staged kernel of 2 to 63 rows (tiles of 8, 16 and 32 tokens; 32, 64 and 128 weight rows a CTA; ragged last rows and tokens; classes without
+    groups, with one, with two and three; several jobs a CTA): every row has the bits that the kernels which split K over warps give it.  Those run where
+    few weight rows meet 64 tokens (Q8_0), or 4000 meet 32 (Q4_K), so the reference takes the first rows of the same matrix."""
+    import torch
+
+    from sharpmind_b200.ops import Mode
+
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    raw = dev.quantize_weights(dtype, torch.randn((max(n, ref_n), k), generator=g, device="cuda") * 0.02)
+    x = torch.randn((ref_m, k), generator=g, device="cuda")
+    few = raw.reshape(max(n, ref_n), -1)
+    w, ref = cuda.register_dev(few[:n].contiguous(), dtype, n, k), cuda.register_dev(few[:ref_n].contiguous(), dtype, ref_n, k)
+    want = dev.qmatmul(x, ref, Mode.ACT_Q8)
+    cols = min(n, ref_n)
+    for lo, hi in ((0, 2), (3, 11), (1, 13), (0, 16), (7, 24), (3, 32), (0, 32), (0, 33), (1, 64)):
+        if hi <= ref_m:
+            got = dev.qmatmul(x[lo:hi].contiguous(), w, Mode.ACT_Q8)
+            assert torch.equal(got[:, :cols].contiguous().view(torch.int32), want[lo:hi, :cols].contiguous().view(torch.int32)), (lo, hi)
+            assert torch.isfinite(got).all()
+    cuda.release(w)
+    cuda.release(ref)
+
+
 @pytest.mark.parametrize("dtype,n,k", [(Q6_K, 64, 2048), (Q8_0, 96, 1024), (Q4_K, 96, 4096), (Q6_K, 40, 14336)])
 @pytest.mark.parametrize("m", [2, 7, 64, 100])
 def test_fp32_activations_as_int8_digit_planes(oracle, cuda, dev, dtype, n, k, m):
