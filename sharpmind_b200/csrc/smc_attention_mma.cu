@@ -17,6 +17,8 @@
 
 #include "smc_common.cuh"
 
+#include <type_traits>
+
 namespace {
 
 constexpr int QROWS = 64, KT = 32;
@@ -293,30 +295,35 @@ __global__ void __launch_bounds__(128 * HPC) sdpa_prefill_mma_kernel(const float
 //   1. scores and tile maxima: tiles are independent; CTA r takes tiles r, r + CS, ..., a warp per head and half tile
 //   2. with all tile maxima known (they go to every CTA of the cluster) the running maximum before and after a tile is a
 //      maximum over earlier tiles: weights, corrections and row sums of all tiles at once
-//   3. only O += P V and l follow the tiles in order; CTA r does it for its 16 output dims (a warp per head), reading the
-//      weights from the CTA that made them through distributed shared memory, while the other warps stage V
+//   3. only O += P V and l follow the tiles in order; CTA r does it for one head and 32 output dims, a warp for 8 of them, while the other four warps
+//      bring V and the weights, those from the CTA that made them through distributed shared memory
 // Shared memory stays below half an SM's: with one CTA per SM fewer than 16 clusters of eight were resident at once, and the
-// 16 head pairs of a 32-head model took two waves.  What bounds it: step 1's MMAs and step 3's chain of 12 MMAs per tile.
-// (128 registers, 264 / 280 bytes spilled at head sizes 64 / 128, for two CTAs per SM.)
-// Six rows over 1021 keys, 32 heads on 8 KV heads of 128, one layer: 175 us in the kernel above,
-// 41 us here; the whole 32-layer pass 8.59 -> 4.32 ms.
+// 16 head pairs of a 32-head model took two waves.  What bounds it: step 1's MMAs, and in step 3 bringing three tiles (2200 clocks; their 36 dependent
+// MMAs take less).  When a CTA did 16 dims of both heads and its MMA warps read the weights themselves, every CTA of the cluster read all weights of both, tile by tile from
+// the same CTA, and half of the registers on their way were spilled: 1360 clocks a tile, 740 now.
+// Six rows over 1021 keys, 32 heads on 8 KV heads of 128, one layer: 175 us in the kernel above, 43 -> 33 us here (101 keys 16 -> 13, 2200 keys 78 -> 55);
+// a 32-layer pass of six rows 3557 -> 3241 us, of a small model's 28 layers 1601 -> 1334.  (The request into L2 ahead of the predecessor's end is 0.5 and 5 % of that.)
 // Scores and weights of all of a CTA's tiles are kept in shared memory, which ends at 14 tiles: 3584 keys at head size 128, 1792 at 64.
-// Longer caches go back to the kernel above (3584 keys 109 us, 3585 583 us; 64: 1792 42 us, 1793 160 us), as do Q8_0 caches and
-// groups of an odd number of heads.
+// Longer caches go to the tcgen05 prompt kernel, as do Q8_0 caches and groups of an odd number of heads.
 constexpr int FEW_ROWS = 8;  // per cluster: rows 8 .. 15 of the MMAs are not used
 template <int HD>
 struct FewShape {
     static constexpr int CS = HD / 16, LDB = HD * 2 + 16;
     static constexpr int LOCAL = 14, TILES = LOCAL * CS;  // key tiles of one CTA, and in all
     static constexpr int QPLANE = 2 * FEW_ROWS * LDB, KPLANE = 2 * KT * LDB, S_JOB = 1024, P_JOB = 3 * 512;
-    static constexpr int V_LD = 48, V_TILES = 5, V_KEYS = V_TILES * KT, VPLANE = V_KEYS * V_LD;  // 16 dims of a key: 32 bytes, padded to an odd multiple of 16
-    // Q and K, then scores; later weights where Q and K were, then two stages of V over the rest and the scores
+    static constexpr int V_LD = 80, V_TILES = 3, V_KEYS = V_TILES * KT, VPLANE = V_KEYS * V_LD;  // 32 dims of a key: 64 bytes, padded to an odd multiple of 16
+    // Q and K, then scores; later weights where Q and K were, then two stages of V and of the weights it meets over the rest and the scores
     static constexpr int QK = 3 * (QPLANE + KPLANE) > 2 * LOCAL * P_JOB ? 3 * (QPLANE + KPLANE) : 2 * LOCAL * P_JOB;
-    static constexpr int OFF_K = 3 * QPLANE, OFF_S = QK, OFF_P = 0, OFF_V = 2 * LOCAL * P_JOB;
-    static constexpr int END = OFF_S + 2 * LOCAL * S_JOB > OFF_V + 2 * 3 * VPLANE ? OFF_S + 2 * LOCAL * S_JOB : OFF_V + 2 * 3 * VPLANE;
-    static constexpr int OFF_TM = END, OFF_CP = OFF_TM + 2 * 2 * TILES * FEW_ROWS * 4, SMEM = OFF_CP + 2 * LOCAL * FEW_ROWS * 8;
+    static constexpr int OFF_K = 3 * QPLANE, OFF_S = QK, OFF_P = 0, OFF_V = 2 * LOCAL * P_JOB, OFF_W = OFF_V + 2 * 3 * VPLANE, W_END = OFF_W + 2 * V_TILES * P_JOB;
+    static constexpr int END = OFF_S + 2 * LOCAL * S_JOB > W_END ? OFF_S + 2 * LOCAL * S_JOB : W_END;
+    static constexpr int OFF_TM = END, OFF_CP = OFF_TM + 2 * 2 * TILES * FEW_ROWS * 4, OFF_WC = OFF_CP + 2 * LOCAL * FEW_ROWS * 8;
+    static constexpr int SMEM = OFF_WC + 2 * V_TILES * FEW_ROWS * 8;
     static_assert(SMEM <= 113 * 1024, "two CTAs per SM");
 };
+__device__ __forceinline__ void prefetch_l2(const void *src, uint32_t bytes)
+{
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t cta)
 {
     uint32_t v;
@@ -340,11 +347,16 @@ __global__ void __launch_bounds__(256, 2) sdpa_few_rows_kernel(const float *__re
     uint4 *sp = reinterpret_cast<uint4 *>(sm_raw + S::OFF_P);                // weights of row g [job][plane][lane]
     const float *tmx = reinterpret_cast<const float *>(sm_raw + S::OFF_TM);  // maxima [head][half tile][row]
     float2 *cp = reinterpret_cast<float2 *>(sm_raw + S::OFF_CP);             // (correction, row sum) [job][row]
-    smc_grid_dep_sync();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, tg = lane & 3;
     const int hg = blockIdx.x / CS, rank = blockIdx.x % CS, kvh = hg * 2 / (nh / nkv), t0 = (int)blockIdx.y * FEW_ROWS;
     const int len = pos0 + T, tiles = (len + KT - 1) / KT, local = tiles > rank ? (tiles - rank + CS - 1) / CS : 0;
     const float *kbase = kc + (size_t)kvh * maxSeq * HD, *vbase = vc + (size_t)kvh * maxSeq * HD;
+    // The keys and values that are there already are asked for, into L2, before the predecessor is waited for (it writes the newest rows, to L2).
+    if (threadIdx.x == 0) {
+        const int part = (pos0 + CS - 1) / CS, k0 = rank * part, n = min(pos0, k0 + part) - k0;
+        if (n > 0) prefetch_l2(kbase + (size_t)k0 * HD, (uint32_t)n * HD * 4), prefetch_l2(vbase + (size_t)k0 * HD, (uint32_t)n * HD * 4);
+    }
+    smc_grid_dep_sync();
 
     constexpr int PF = 2 * KT * (HD / 4) / 256;  // K: two tiles at a time, requested before the previous two are multiplied
     float4 pk[PF];
@@ -419,91 +431,112 @@ __global__ void __launch_bounds__(256, 2) sdpa_few_rows_kernel(const float *__re
         dst[64] = make_uint4(pl[0][0], pl[0][2], pl[1][0], pl[1][2]);
         if (tg == 0) cp[job * FEW_ROWS + g] = make_float2(c0, ps0);
     }
-    cluster_sync();  // and nobody needs its scores any more: V goes there
-    // ---- 3: O and l in tile order, 16 dims per CTA
-    auto stage_v = [&](int chunk, int t, int threads) {  // V_KEYS keys x 16 dims
-        uint8_t *dst = sm_raw + S::OFF_V + (chunk & 1) * 3 * S::VPLANE;
-        for (int e0 = t; e0 < S::V_KEYS * 4; e0 += 4 * threads) {
-            float4 v[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int e = e0 + i * threads, key = chunk * S::V_KEYS + e / 4;
-                v[i] = e < S::V_KEYS * 4 && key < len ? *reinterpret_cast<const float4 *>(vbase + (size_t)key * HD + rank * 16 + 4 * (e & 3))
-                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int e = e0 + i * threads;
-                if (e < S::V_KEYS * 4) split_store(v[i], dst + (e / 4) * S::V_LD + 8 * (e & 3), S::VPLANE);
-            }
-        }
+    // ---- 3: O and l in tile order, one head and 32 dims per CTA: four warps of 8 dims multiply, the other four bring V and the weights, a chunk of
+    // V_TILES tiles ahead in shared memory and another in registers
+    const int hl3 = rank / (CS / 2), d3 = rank % (CS / 2) * 32;
+    constexpr int PIECES = S::V_KEYS * 8, WORDS = S::V_TILES * (S::P_JOB / 16), ROWS3 = S::V_TILES * FEW_ROWS;
+    auto load_v = [&](int e, int chunk) {  // four dims of a key
+        const int key = chunk * S::V_KEYS + e / 8;
+        return e < PIECES && key < len ? *reinterpret_cast<const float4 *>(vbase + (size_t)key * HD + d3 + 4 * (e & 7)) : make_float4(0.f, 0.f, 0.f, 0.f);
     };
-    stage_v(0, threadIdx.x, 256);
-    const int chunks = (tiles + S::V_TILES - 1) / S::V_TILES;
-    if (warp >= 2) {
-        for (int chunk = 0; chunk < chunks; ++chunk) {
-            __syncthreads();  // this chunk is staged and the other buffer has been read
-            if (chunk + 1 < chunks) stage_v(chunk + 1, threadIdx.x - 64, 192);
-        }
-    } else {
-        const int hl = warp;
-        constexpr int AHEAD = 4;  // tiles whose weights are on their way
-        uint4 wp[AHEAD][3];
-        float2 wr[AHEAD];
-        auto fetch = [&](int tile, int u) {
-            const uint32_t job = (uint32_t)(hl * S::LOCAL + tile / CS);
-            const uint32_t at = cluster_map(base + S::OFF_P, (uint32_t)(tile % CS)) + job * S::P_JOB + 16u * (uint32_t)lane;
-            const uint32_t ac = cluster_map(base + S::OFF_CP, (uint32_t)(tile % CS)) + 8u * (job * FEW_ROWS + (uint32_t)g);
+    auto store_v = [&](int e, int chunk, const float4 &v) {
+        if (e < PIECES) split_store(v, sm_raw + S::OFF_V + (chunk & 1) * 3 * S::VPLANE + (e / 8) * S::V_LD + 8 * (e & 7), S::VPLANE);
+    };
+    auto load_w = [&](int e, int chunk, uint4 &v) {  // 16 bytes of a tile's weights, from the CTA that made them
+        const int tile = chunk * S::V_TILES + e / (S::P_JOB / 16);
+        if (e >= WORDS || tile >= tiles) return;
+        const uint32_t at = cluster_map(base + S::OFF_P, (uint32_t)(tile % CS)) + (uint32_t)((hl3 * S::LOCAL + tile / CS) * S::P_JOB + 16 * (e % (S::P_JOB / 16)));
+        asm volatile("ld.shared::cluster.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at) : "memory");
+    };
+    auto store_w = [&](int e, int chunk, const uint4 &v) {
+        if (e < WORDS) *reinterpret_cast<uint4 *>(sm_raw + S::OFF_W + (chunk & 1) * S::V_TILES * S::P_JOB + 16 * e) = v;
+    };
+    auto load_c = [&](int e, int chunk, float2 &v) {  // (correction, row sum) of a tile's row
+        const int tile = chunk * S::V_TILES + e / FEW_ROWS;
+        if (e >= ROWS3 || tile >= tiles) return;
+        const uint32_t at = cluster_map(base + S::OFF_CP, (uint32_t)(tile % CS)) + 8u * (uint32_t)((hl3 * S::LOCAL + tile / CS) * FEW_ROWS + e % FEW_ROWS);
+        asm volatile("ld.shared::cluster.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(at) : "memory");
+    };
+    auto store_c = [&](int e, int chunk, const float2 &v) {
+        if (e < ROWS3) *reinterpret_cast<float2 *>(sm_raw + S::OFF_WC + 8 * ((chunk & 1) * ROWS3 + e)) = v;
+    };
+    auto bring = [&](auto threads, int t, auto request, auto keep) {
+        constexpr int TH = decltype(threads)::value, NV = (PIECES + TH - 1) / TH, NW = (WORDS + TH - 1) / TH;
+        float4 v[NV];
+        uint4 w[NW];
+        float2 c = make_float2(0.f, 0.f);
 #pragma unroll
-            for (int i = 0; i < 3; ++i)
-                asm volatile("ld.shared::cluster.v4.u32 {%0,%1,%2,%3}, [%4];"
-                             : "=r"(wp[u][i].x), "=r"(wp[u][i].y), "=r"(wp[u][i].z), "=r"(wp[u][i].w)
-                             : "r"(at + 512u * i)
-                             : "memory");
-            asm volatile("ld.shared::cluster.v2.f32 {%0,%1}, [%2];" : "=f"(wr[u].x), "=f"(wr[u].y) : "r"(ac) : "memory");
+        for (int i = 0; i < NW; ++i) w[i] = make_uint4(0u, 0u, 0u, 0u);
+        auto load = [&](int chunk) {
+#pragma unroll
+            for (int i = 0; i < NV; ++i) v[i] = load_v(t + i * TH, chunk);
+            request();
+#pragma unroll
+            for (int i = 0; i < NW; ++i) load_w(t + i * TH, chunk, w[i]);
+            load_c(t, chunk, c);
         };
+        auto store = [&](int chunk) {
 #pragma unroll
-        for (int u = 0; u < AHEAD; ++u)
-            if (u < tiles) fetch(u, u);
-        float o[2][4], l0 = 0.f;
+            for (int i = 0; i < NV; ++i) store_v(t + i * TH, chunk, v[i]);
 #pragma unroll
-        for (int n = 0; n < 2; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
-        const uint32_t va = base + S::OFF_V + (uint32_t)(((lane & 7) + 8 * ((lane >> 3) & 1)) * S::V_LD + 16 * (lane >> 4));
-        int in_chunk = 0, chunk = 0;
-        for (int tile0 = 0; tile0 < tiles; tile0 += AHEAD) {
-#pragma unroll
-            for (int u = 0; u < AHEAD; ++u) {
-                const int tile = tile0 + u;
-                if (tile >= tiles) break;
-                if (in_chunk == 0) __syncthreads();  // the chunk is staged
-                const uint32_t vt = va + (uint32_t)((chunk & 1) * 3 * S::VPLANE + in_chunk * KT * S::V_LD);
-                if (++in_chunk == S::V_TILES) in_chunk = 0, ++chunk;
-                const float c0 = wr[u].x;
-                l0 = fmaf(l0, c0, wr[u].y);
-                const uint4 w[3] = {wp[u][0], wp[u][1], wp[u][2]};
-                if (tile + AHEAD < tiles) fetch(tile + AHEAD, u);
-#pragma unroll
-                for (int n = 0; n < 2; ++n) o[n][0] *= c0, o[n][1] *= c0;
-#pragma unroll
-                for (int j = 0; j < KT / 16; ++j) {
-                    uint32_t b[3][4];
-#pragma unroll
-                    for (int pl = 0; pl < 3; ++pl) ldsm4t(vt + (uint32_t)(pl * S::VPLANE + j * 16 * S::V_LD), b[pl]);
-                    const uint32_t ph[4] = {j ? w[0].z : w[0].x, 0u, j ? w[0].w : w[0].y, 0u}, pm[4] = {j ? w[1].z : w[1].x, 0u, j ? w[1].w : w[1].y, 0u},
-                                   pl[4] = {j ? w[2].z : w[2].x, 0u, j ? w[2].w : w[2].y, 0u};
-                    const uint32_t b0a[3] = {b[0][0], b[1][0], b[2][0]}, b1a[3] = {b[0][1], b[1][1], b[2][1]};
-                    const uint32_t b0b[3] = {b[0][2], b[1][2], b[2][2]}, b1b[3] = {b[0][3], b[1][3], b[2][3]};
-                    mma6(o[0], ph, pm, pl, b0a, b1a);
-                    mma6(o[1], ph, pm, pl, b0b, b1b);
-                }
+            for (int i = 0; i < NW; ++i) store_w(t + i * TH, chunk, w[i]);
+            store_c(t, chunk, c);
+        };
+        keep(load, store);
+    };
+    const int chunks = (tiles + S::V_TILES - 1) / S::V_TILES;
+    // all warps: chunk 0.  Between its two requests the weights are waited for; nobody needs its scores any more then, and V goes there.
+    bring(std::integral_constant<int, 256>{}, threadIdx.x, [] { cluster_sync(); }, [&](auto &load, auto &store) { load(0), store(0); });
+    if (warp >= 4) {
+        bring(std::integral_constant<int, 128>{}, threadIdx.x - 128, [] {}, [&](auto &load, auto &store) {
+            load(1);
+            for (int chunk = 0; chunk < chunks; ++chunk) {
+                __syncthreads();  // this chunk is staged and the other buffers have been read
+                if (chunk + 1 < chunks) store(chunk + 1), load(chunk + 2);
             }
+        });
+    } else {
+        float o[4] = {0.f, 0.f, 0.f, 0.f}, l0 = 0.f;
+        struct Operands {
+            uint32_t v[3][4];  // [plane][8 keys]
+            uint4 w[3];
+            float2 c;
+        } x[2];  // a tile's; the next one's are fetched before this one's MMAs
+        const uint32_t va = base + S::OFF_V + (uint32_t)(lane * S::V_LD + 16 * warp);
+        int next = 0, next_chunk = 0;  // the tile to be fetched: its place in its chunk, and the chunk
+        auto fetch = [&](Operands &d) {
+            if (next == 0) __syncthreads();  // the chunk is staged, and all of the one before it is in registers
+            const int buf = next_chunk & 1;
+#pragma unroll
+            for (int pl = 0; pl < 3; ++pl) {
+                ldsm4t(va + (uint32_t)((buf * 3 + pl) * S::VPLANE + next * KT * S::V_LD), d.v[pl]);
+                d.w[pl] = *reinterpret_cast<const uint4 *>(sm_raw + S::OFF_W + (buf * S::V_TILES + next) * S::P_JOB + 512 * pl + 16 * lane);
+            }
+            d.c = *reinterpret_cast<const float2 *>(sm_raw + S::OFF_WC + 8 * (buf * ROWS3 + next * FEW_ROWS + g));
+            if (++next == S::V_TILES) next = 0, ++next_chunk;
+        };
+        auto add = [&](const Operands &d) {
+            l0 = fmaf(l0, d.c.x, d.c.y);
+            o[0] *= d.c.x, o[1] *= d.c.x;
+#pragma unroll
+            for (int j = 0; j < KT / 16; ++j) {
+                const uint32_t ph[4] = {j ? d.w[0].z : d.w[0].x, 0u, j ? d.w[0].w : d.w[0].y, 0u}, pm[4] = {j ? d.w[1].z : d.w[1].x, 0u, j ? d.w[1].w : d.w[1].y, 0u},
+                               pl[4] = {j ? d.w[2].z : d.w[2].x, 0u, j ? d.w[2].w : d.w[2].y, 0u};
+                const uint32_t b0[3] = {d.v[0][2 * j], d.v[1][2 * j], d.v[2][2 * j]}, b1[3] = {d.v[0][2 * j + 1], d.v[1][2 * j + 1], d.v[2][2 * j + 1]};
+                mma6(o, ph, pm, pl, b0, b1);
+            }
+        };
+        fetch(x[0]);
+        for (int tile = 0; tile < tiles; tile += 2) {
+            if (tile + 1 < tiles) fetch(x[1]);
+            add(x[0]);
+            if (tile + 1 >= tiles) break;
+            if (tile + 2 < tiles) fetch(x[0]);
+            add(x[1]);
         }
         const float i0 = l0 > 0.f ? 1.0f / l0 : 0.f;
-        if (t0 + g < T) {
-            float *dst = out + ((size_t)(t0 + g) * nh + hg * 2 + hl) * HD + rank * 16 + 2 * tg;
-            *reinterpret_cast<float2 *>(dst) = make_float2(o[0][0] * i0, o[0][1] * i0);
-            *reinterpret_cast<float2 *>(dst + 8) = make_float2(o[1][0] * i0, o[1][1] * i0);
-        }
+        if (t0 + g < T)
+            *reinterpret_cast<float2 *>(out + ((size_t)(t0 + g) * nh + hg * 2 + hl3) * HD + d3 + 8 * warp + 2 * tg) = make_float2(o[0] * i0, o[1] * i0);
     }
     cluster_sync();  // nobody leaves while its weights are read
 }
