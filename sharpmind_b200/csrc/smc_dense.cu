@@ -415,14 +415,14 @@ __global__ void __launch_bounds__(192, 1) dense_tc_kernel(const __grid_constant_
     float *part = reinterpret_cast<float *>(smem);
 
     const int mt = (M + TC_M - 1) / TC_M, nt = (N + BN - 1) / BN, tiles = mt * nt, ksteps = (K + TC_K - 1) / TC_K;
-    const int rank = CS > 1 ? blockIdx.x % CS : 0, tile0 = blockIdx.x / CS, tstep = gridDim.x / CS;  // a cluster has one tile
-    const int k0 = rank * ksteps / CS, k1 = (rank + 1) * ksteps / CS;
+    const int rank = CS > 1 ? blockIdx.x % CS : 0;  // a cluster has one tile
+    const int k0 = CS > 1 ? rank * ksteps / CS : 0, k1 = CS > 1 ? (rank + 1) * ksteps / CS : ksteps;
     if (warp == 0) {
         if (lane == 0) {
             int st = 0;
             uint32_t ph = 1;
             bool free = true;  // the slot, as far as is known
-            for (int t = tile0; t < tiles; t += tstep) {
+            for (int t = blockIdx.x / CS; t < tiles; t += gridDim.x / CS) {
                 const int m0 = (t % mt) * TC_M, n0 = (t / mt) * BN;
                 for (int k = k0; k < k1; ++k) {
                     if (!free) smc_tc_wait(empty(st), ph, abort_flag, status);
@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(192, 1) dense_tc_kernel(const __grid_constant_
             int st = 0, n = 0;
             uint32_t ph = 0;
             bool there = false;  // the stage, as far as is known
-            for (int t = tile0; t < tiles; t += tstep, ++n) {
+            for (int t = blockIdx.x / CS; t < tiles; t += gridDim.x / CS, ++n) {
                 const int buf = n & 1;
                 smc_tc_wait(acc_empty(buf), (uint32_t)(((n >> 1) & 1) ^ 1), abort_flag, status);
                 const uint32_t d = tmem + (uint32_t)(buf * BN);
@@ -462,7 +462,7 @@ __global__ void __launch_bounds__(192, 1) dense_tc_kernel(const __grid_constant_
     } else {
         const int quarter = warp & 3;
         int n = 0;
-        for (int t = tile0; t < tiles; t += tstep, ++n) {
+        for (int t = blockIdx.x / CS; t < tiles; t += gridDim.x / CS, ++n) {
             const int buf = n & 1, m = (t % mt) * TC_M + quarter * 32 + lane, n0 = (t / mt) * BN;
             if (lane == 0) smc_tc_wait(acc_full(buf), (uint32_t)((n >> 1) & 1), abort_flag, status);
             __syncwarp();
@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(192, 1) dense_tc_kernel(const __grid_constant_
         if (warp >= 2) {  // 128 threads: 128 / CS tokens, CS threads of BN / CS columns per token
             constexpr int W = BN / CS < 16 ? 8 : 16;
             const int e = threadIdx.x - 64, tok = rank * (TC_M / CS) + e / CS, c0 = e % CS * (BN / CS);
-            const int m = (tile0 % mt) * TC_M + tok, n0 = (tile0 / mt) * BN;
+            const int tile0 = blockIdx.x / CS, m = (tile0 % mt) * TC_M + tok, n0 = (tile0 / mt) * BN;
             const uint32_t at = sbase + 4u * (uint32_t)(tok * PLD + c0);
             for (int c = 0; c < BN / CS; c += W) {
                 if (m >= M || n0 + c0 + c >= N) break;
