@@ -15,13 +15,13 @@
 // One CTA computes 128 weight rows x 128 tokens.  Warp roles:
 //   warp 0        lane 0 streams the activation tiles with bulk copies (global -> shared, mbarrier tx count)
 //   warp 1        lane 0 issues tcgen05.mma / tcgen05.commit
-//   warps 2..5    one thread per weight row: reads its 144-byte block, expands the nibbles to fp16 sc*q and
-//                 stores them with tcgen05.st into its own lane of tensor memory: the A operand never touches
+//   warps 2..9    two threads per weight row: copy the rows' 144-byte blocks ahead (cp.async), expand the nibbles to fp16 sc*q and
+//                 store them with tcgen05.st into their own lane of tensor memory: the A operand never touches
 //                 shared memory (a first version that wrote A tiles to shared memory was bound by shared-memory
 //                 bandwidth: 64 KB of stores and 256 KB of MMA operand reads per block and CTA)
-//   warps 6..13   drain: tcgen05.ld of acc_d, scaling by d_b, fp32 running sums in registers (64 tokens per
+//   warps 10..17  drain: tcgen05.ld of acc_d, scaling by d_b, fp32 running sums in registers (64 tokens per
 //                 thread), final store
-// Shared memory: 6 stages of {B_hi 16 KB, B_lo 16 KB} (64 k each) + 2 x {A'' 4 KB, B'' 8 KB} for the min term.
+// Shared memory: 4 stages of {B_hi 16 KB, B_lo 16 KB} (64 k each), 4 blocks of raw weights, 2 x {A'' 4 KB, B'' 8 KB} for the min term.
 // TMEM (512 columns): acc_d x 2 buffers (the drain of one block overlaps the MMAs of the next), acc_m, and four
 // A stages of 32 columns.  Every mbarrier wait is bounded; a wait that runs out raises the context's status
 // word and a CTA-wide abort flag that makes every later wait return at once, so the kernel still ends and
