@@ -275,20 +275,13 @@ __global__ void __launch_bounds__(256) dense_tile_kernel(const bf16 *__restrict_
 
 // ------------------------------------------------------------------------------ prompt sizes: tcgen05
 constexpr int TC_M = 128, TC_K = 64;
-template <int BN, int CS = 1>
+template <int BN>
 struct TcShape {
-    // a cluster's CTA holds half as many: two fit an SM, so clusters need not find whole free SMs side by side
-    static constexpr int STAGES = CS > 1 ? 5 : BN == 256 ? 4 : BN == 128 ? 6 : BN == 64 ? 8 : 10;
+    static constexpr int STAGES = BN == 256 ? 4 : BN == 128 ? 6 : BN == 64 ? 8 : 10;
     static constexpr uint32_t A_BYTES = TC_M * TC_K * 2, B_BYTES = BN * TC_K * 2, STAGE = A_BYTES + B_BYTES;
     static constexpr uint32_t OFF_BAR = STAGES * STAGE, SMEM = OFF_BAR + 256 + 1024;  // + slack to align the base to 1024
     static constexpr uint32_t COLS = 2 * BN;                                       // two accumulators
 };
-
-__device__ __forceinline__ void cluster_meet()
-{
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 // What the epilogue does: store (or sum), SiLU or GELU of woven pairs, or everything `finish` knows.
 enum { EPI_STORE, EPI_SILU_PAIRS, EPI_GELU_PAIRS, EPI_FINISH };
@@ -298,91 +291,12 @@ __device__ __forceinline__ void add4(float *y, float a, float b, float c, float 
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(y), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
-// W neighbouring columns of one token, from column nc < N on
-template <int EPI, int W>
-__device__ __forceinline__ void store_cols(const smc_dense_out &o, int m, int nc, int N, float (&v)[W])
-{
-    constexpr bool PAIRS = EPI == EPI_SILU_PAIRS || EPI == EPI_GELU_PAIRS;
-    if (PAIRS) {
-        float f[W / 2];
-        if (o.y_bf16) {
-#pragma unroll
-            for (int i = 0; i < W / 2; ++i) f[i] = act_pair_fast<EPI == EPI_GELU_PAIRS>(v[2 * i], v[2 * i + 1]);
-        } else {
-#pragma unroll
-            for (int i = 0; i < W / 2; ++i) f[i] = act_pair(EPI == EPI_GELU_PAIRS ? 2 : 1, v[2 * i], v[2 * i + 1]);
-        }
-        const int c2 = nc >> 1;
-        if (o.y_bf16 && nc + W <= N && (o.ldy & 7) == 0) {
-            using Out = std::conditional_t<W == 16, uint4, uint2>;
-            __align__(16) __nv_bfloat162 p[W / 4];
-#pragma unroll
-            for (int i = 0; i < W / 4; ++i) p[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
-            *reinterpret_cast<Out *>(static_cast<bf16 *>(o.y) + (size_t)m * o.ldy + c2) = *reinterpret_cast<Out *>(p);
-        } else {
-#pragma unroll
-            for (int i = 0; i < W / 2; ++i)
-                if (nc + 2 * i + 1 < N) {
-                    if (o.y_bf16) static_cast<bf16 *>(o.y)[(size_t)m * o.ldy + c2 + i] = __float2bfloat16_rn(f[i]);
-                    else static_cast<float *>(o.y)[(size_t)m * o.ldy + c2 + i] = f[i];
-                }
-        }
-    } else if (nc + W <= N && (o.split == 0 || nc + W <= o.split) && (o.ldy & 7) == 0) {
-        if (EPI == EPI_FINISH) {
-            if (o.bias) {
-#pragma unroll
-                for (int i = 0; i < W / 4; ++i) {
-                    const float4 b = __ldg(reinterpret_cast<const float4 *>(o.bias + nc) + i);
-                    v[4 * i] += b.x, v[4 * i + 1] += b.y, v[4 * i + 2] += b.z, v[4 * i + 3] += b.w;
-                }
-            }
-            if (nc >= o.silu_from && nc + W <= o.silu_to && o.y_bf16) {
-#pragma unroll
-                for (int i = 0; i < W; ++i) v[i] = silu_for<bf16>(v[i]);
-            } else if (nc < o.silu_to && nc + W > o.silu_from) {
-#pragma unroll
-                for (int i = 0; i < W; ++i) v[i] = nc + i >= o.silu_from && nc + i < o.silu_to ? silu(v[i]) : v[i];
-            }
-            if (o.softcap > 0.f) {
-#pragma unroll
-                for (int i = 0; i < W; ++i) v[i] = o.softcap * tanhf(__fdiv_rn(v[i], o.softcap));
-            }
-        }
-        if (o.y_bf16) {
-            __align__(16) __nv_bfloat162 p[W / 2];
-#pragma unroll
-            for (int i = 0; i < W / 2; ++i) p[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-            uint4 *dst = reinterpret_cast<uint4 *>(static_cast<bf16 *>(o.y) + (size_t)m * o.ldy + nc);
-#pragma unroll
-            for (int i = 0; i < W / 8; ++i) dst[i] = reinterpret_cast<uint4 *>(p)[i];
-        } else {
-            float4 *dst = reinterpret_cast<float4 *>(static_cast<float *>(o.y) + (size_t)m * o.ldy + nc);
-#pragma unroll
-            for (int i = 0; i < W / 4; ++i) {
-                if (o.accumulate) add4(reinterpret_cast<float *>(dst + i), v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-                else dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-            }
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < W; ++i)
-            if (nc + i < N) put(o, m, nc + i, v[i]);
-    }
-}
-
 // Warp 0: TMA loads; warp 1: MMA issue; warps 2 .. 5: epilogue (one TMEM lane = one token per thread).
-// CS > 1: a cluster of CS CTAs shares one tile and each takes a part of K, for matrices whose tiles leave most SMs idle while the
-// few that work are bound by what one SM pulls from L2.  The parts meet in shared memory: every CTA adds all of them, in rank
-// order, for its share of the tile's tokens.
-// Measured: 96 rows of 1024 outputs over K = 3072 on 32 CTAs 16.4 us (cold); eight prompts of 96 rows and eight steps of a 16-layer decoder of
-// width 1024: 15.35 -> 13.87 ms.  (Another order of fp32 sums, in shorter chains of the tensor
-// cores' cut-off additions: 96 rows of 1024 outputs are 9.9e-7 -> 2.3e-7 from 64 bits at K = 1024, 3.2e-6 -> 7.3e-7 at 3072.  Behind the rounding to bfloat16 a
-// whole 16-layer model shows no difference: 0.0160 and 0.0164 over 40 draws, standard error of the difference 0.0002; 0.0166 and 0.0166 over 16 others.)
-template <int BN, int EPI, int CS>
+template <int BN, int EPI>
 __global__ void __launch_bounds__(192, 1) dense_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, int M,
                                                           int N, int K, smc_dense_out o, int *status)
 {
-    using S = TcShape<BN, CS>;
+    using S = TcShape<BN>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smc_smem_u32(smem_raw), sbase = (raw + 1023u) & ~1023u;
     uint8_t *smem = smem_raw + (sbase - raw);
@@ -412,20 +326,16 @@ __global__ void __launch_bounds__(192, 1) dense_tc_kernel(const __grid_constant_
     smc_tc_fence_after();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(smem + OFF_PTR);
-    constexpr int PLD = BN + 4;  // floats per token of a part: 16-byte pieces of neighbouring tokens on other banks
-    float *part = reinterpret_cast<float *>(smem);
 
     const int mt = (M + TC_M - 1) / TC_M, nt = (N + BN - 1) / BN, tiles = mt * nt, ksteps = (K + TC_K - 1) / TC_K;
-    const int rank = CS > 1 ? blockIdx.x % CS : 0;  // a cluster has one tile
-    const int k0 = CS > 1 ? rank * ksteps / CS : 0, k1 = CS > 1 ? (rank + 1) * ksteps / CS : ksteps;
     if (warp == 0) {
         if (lane == 0) {
             int st = 0;
             uint32_t ph = 1;
             bool free = true;  // the slot, as far as is known
-            for (int t = blockIdx.x / CS; t < tiles; t += gridDim.x / CS) {
+            for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
                 const int m0 = (t % mt) * TC_M, n0 = (t / mt) * BN;
-                for (int k = k0; k < k1; ++k) {
+                for (int k = 0; k < ksteps; ++k) {
                     if (!free) smc_tc_wait(empty(st), ph, abort_flag, status);
                     const uint32_t at = sbase + (uint32_t)st * S::STAGE, bar = full(st);
                     if (++st == S::STAGES) st = 0, ph ^= 1;
@@ -442,11 +352,11 @@ __global__ void __launch_bounds__(192, 1) dense_tc_kernel(const __grid_constant_
             int st = 0, n = 0;
             uint32_t ph = 0;
             bool there = false;  // the stage, as far as is known
-            for (int t = blockIdx.x / CS; t < tiles; t += gridDim.x / CS, ++n) {
+            for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++n) {
                 const int buf = n & 1;
                 smc_tc_wait(acc_empty(buf), (uint32_t)(((n >> 1) & 1) ^ 1), abort_flag, status);
                 const uint32_t d = tmem + (uint32_t)(buf * BN);
-                for (int k = k0; k < k1; ++k) {
+                for (int k = 0; k < ksteps; ++k) {
                     if (!there) smc_tc_wait(full(st), ph, abort_flag, status);
                     smc_tc_fence_after();
                     const uint64_t da = smc_tc_desc_sw128(sbase + (uint32_t)st * S::STAGE), db = smc_tc_desc_sw128(sbase + (uint32_t)st * S::STAGE + S::A_BYTES);
@@ -454,7 +364,7 @@ __global__ void __launch_bounds__(192, 1) dense_tc_kernel(const __grid_constant_
                     if (++st == S::STAGES) st = 0, ph ^= 1;
                     there = smc_mbar_test(full(st), ph);
 #pragma unroll
-                    for (int kk = 0; kk < TC_K / 16; ++kk) smc_tc_mma(d, da + 2 * kk, db + 2 * kk, IDESC, k > k0 || kk > 0 ? 1u : 0u);
+                    for (int kk = 0; kk < TC_K / 16; ++kk) smc_tc_mma(d, da + 2 * kk, db + 2 * kk, IDESC, (k | kk) != 0 ? 1u : 0u);
                     smc_tc_commit(done);
                 }
                 smc_tc_commit(acc_full(buf));
@@ -463,7 +373,7 @@ __global__ void __launch_bounds__(192, 1) dense_tc_kernel(const __grid_constant_
     } else {
         const int quarter = warp & 3;
         int n = 0;
-        for (int t = blockIdx.x / CS; t < tiles; t += gridDim.x / CS, ++n) {
+        for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++n) {
             const int buf = n & 1, m = (t % mt) * TC_M + quarter * 32 + lane, n0 = (t / mt) * BN;
             if (lane == 0) smc_tc_wait(acc_full(buf), (uint32_t)((n >> 1) & 1), abort_flag, status);
             __syncwarp();
@@ -474,13 +384,6 @@ __global__ void __launch_bounds__(192, 1) dense_tc_kernel(const __grid_constant_
                 smc_tc_ld16(src + (uint32_t)c, r[0]);
                 smc_tc_ld16(src + (uint32_t)c + 16u, r[1]);
                 smc_tc_wait_ld();
-                if constexpr (CS > 1) {  // the loads' stages are free: every one has been multiplied
-                    float *at = part + (quarter * 32 + lane) * PLD + c;
-#pragma unroll
-                    for (int i = 0; i < 32; i += 4)
-                        *reinterpret_cast<uint4 *>(at + i) = make_uint4(r[i >> 4][i & 15], r[i >> 4][(i & 15) + 1], r[i >> 4][(i & 15) + 2], r[i >> 4][(i & 15) + 3]);
-                    continue;
-                }
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int nc = n0 + c + 16 * h;
@@ -488,7 +391,70 @@ __global__ void __launch_bounds__(192, 1) dense_tc_kernel(const __grid_constant_
                     float v[16];
 #pragma unroll
                     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[h][i]);
-                    store_cols<EPI, 16>(o, m, nc, N, v);
+                    constexpr bool PAIRS = EPI == EPI_SILU_PAIRS || EPI == EPI_GELU_PAIRS;
+                    if (PAIRS) {
+                        float f[8];
+                        if (o.y_bf16) {
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) f[i] = act_pair_fast<EPI == EPI_GELU_PAIRS>(v[2 * i], v[2 * i + 1]);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) f[i] = act_pair(EPI == EPI_GELU_PAIRS ? 2 : 1, v[2 * i], v[2 * i + 1]);
+                        }
+                        const int c2 = nc >> 1;
+                        if (o.y_bf16 && nc + 16 <= N && (o.ldy & 7) == 0) {
+                            __nv_bfloat162 p[4];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) p[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+                            *reinterpret_cast<uint4 *>(static_cast<bf16 *>(o.y) + (size_t)m * o.ldy + c2) = *reinterpret_cast<uint4 *>(p);
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 8; ++i)
+                                if (nc + 2 * i + 1 < N) {
+                                    if (o.y_bf16) static_cast<bf16 *>(o.y)[(size_t)m * o.ldy + c2 + i] = __float2bfloat16_rn(f[i]);
+                                    else static_cast<float *>(o.y)[(size_t)m * o.ldy + c2 + i] = f[i];
+                                }
+                        }
+                    } else if (nc + 16 <= N && (o.split == 0 || nc + 16 <= o.split) && (o.ldy & 7) == 0) {
+                        if (EPI == EPI_FINISH) {
+                            if (o.bias) {
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) {
+                                    const float4 b = __ldg(reinterpret_cast<const float4 *>(o.bias + nc) + i);
+                                    v[4 * i] += b.x, v[4 * i + 1] += b.y, v[4 * i + 2] += b.z, v[4 * i + 3] += b.w;
+                                }
+                            }
+                            if (nc >= o.silu_from && nc + 16 <= o.silu_to && o.y_bf16) {
+#pragma unroll
+                                for (int i = 0; i < 16; ++i) v[i] = silu_for<bf16>(v[i]);
+                            } else if (nc < o.silu_to && nc + 16 > o.silu_from) {
+#pragma unroll
+                                for (int i = 0; i < 16; ++i) v[i] = nc + i >= o.silu_from && nc + i < o.silu_to ? silu(v[i]) : v[i];
+                            }
+                            if (o.softcap > 0.f) {
+#pragma unroll
+                                for (int i = 0; i < 16; ++i) v[i] = o.softcap * tanhf(__fdiv_rn(v[i], o.softcap));
+                            }
+                        }
+                        if (o.y_bf16) {
+                            __nv_bfloat162 p[8];
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) p[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+                            uint4 *dst = reinterpret_cast<uint4 *>(static_cast<bf16 *>(o.y) + (size_t)m * o.ldy + nc);
+                            dst[0] = reinterpret_cast<uint4 *>(p)[0], dst[1] = reinterpret_cast<uint4 *>(p)[1];
+                        } else {
+                            float4 *dst = reinterpret_cast<float4 *>(static_cast<float *>(o.y) + (size_t)m * o.ldy + nc);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                if (o.accumulate) add4(reinterpret_cast<float *>(dst + i), v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                                else dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                            }
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i)
+                            if (nc + i < N) put(o, m, nc + i, v[i]);
+                    }
                 }
                 __syncwarp();  // the accumulator reads are warp-wide: lanes without a token rejoin here
             }
@@ -496,34 +462,6 @@ __global__ void __launch_bounds__(192, 1) dense_tc_kernel(const __grid_constant_
             __syncwarp();
             if (lane == 0) smc_mbar_arrive(acc_empty(buf));
         }
-    }
-    if constexpr (CS > 1) {
-        static_assert(BN % CS == 0 && BN / CS >= 8 && 128 * PLD * 4 <= S::OFF_BAR, "shares of a tile");
-        cluster_meet();
-        if (warp >= 2) {  // 128 threads: 128 / CS tokens, CS threads of BN / CS columns per token
-            constexpr int W = BN / CS < 16 ? 8 : 16;
-            const int e = threadIdx.x - 64, tok = rank * (TC_M / CS) + e / CS, c0 = e % CS * (BN / CS);
-            const int tile0 = blockIdx.x / CS, m = (tile0 % mt) * TC_M + tok, n0 = (tile0 / mt) * BN;
-            const uint32_t at = sbase + 4u * (uint32_t)(tok * PLD + c0);
-            for (int c = 0; c < BN / CS; c += W) {
-                if (m >= M || n0 + c0 + c >= N) break;
-                float v[W];
-#pragma unroll
-                for (int p = 0; p < CS; ++p) {
-                    uint32_t from;
-                    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(from) : "r"(at + 4u * c), "r"(p));
-#pragma unroll
-                    for (int i = 0; i < W; i += 4) {
-                        float x[4];
-                        asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3]) : "r"(from + 4u * i) : "memory");
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) v[i + j] = p == 0 ? x[j] : v[i + j] + x[j];
-                    }
-                }
-                store_cols<EPI, W>(o, m, n0 + c0 + c, N, v);
-            }
-        }
-        cluster_meet();  // nobody leaves while its part is read
     }
     smc_tc_fence_before();
     __syncthreads();
@@ -558,21 +496,19 @@ bool make_map(CUtensorMap *map, const void *base, uint64_t cols, uint64_t rows, 
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN, int EPI, int CS = 1>
+template <int BN, int EPI>
 int launch_tc(smc_ctx *ctx, const bf16 *x, int ldx, const bf16 *w, int M, int N, int K, const smc_dense_out &o, cudaStream_t s)
 {
-    using S = TcShape<BN, CS>;
+    using S = TcShape<BN>;
     CUtensorMap mx, mw;
     if (!make_map(&mx, x, K, M, ldx, TC_M) || !make_map(&mw, w, K, N, K, BN)) return smc_fail(ctx, SMC_E_CUDA, "dense matmul: tensor map encoding failed");
     static bool attr_set = false;
     if (!attr_set) {
-        SMC_CUDA(ctx, cudaFuncSetAttribute(dense_tc_kernel<BN, EPI, CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM));
+        SMC_CUDA(ctx, cudaFuncSetAttribute(dense_tc_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM));
         attr_set = true;
     }
     const int tiles = ((M + TC_M - 1) / TC_M) * ((N + BN - 1) / BN);
-    if (CS > 1)
-        smc_launch_dep_cluster(ctx->use_pdl, CS, dense_tc_kernel<BN, EPI, CS>, dim3(tiles * CS), dim3(192), S::SMEM, s, mx, mw, M, N, K, o, ctx->d_status);
-    else smc_launch_dep(ctx->use_pdl, dense_tc_kernel<BN, EPI, CS>, dim3(tiles < ctx->sm_count ? tiles : ctx->sm_count), dim3(192), S::SMEM, s, mx, mw, M, N, K, o,
+    smc_launch_dep(ctx->use_pdl, dense_tc_kernel<BN, EPI>, dim3(tiles < ctx->sm_count ? tiles : ctx->sm_count), dim3(192), S::SMEM, s, mx, mw, M, N, K, o,
                    ctx->d_status);
     SMC_LAUNCH_CHECK(ctx);
     return SMC_OK;
@@ -636,15 +572,9 @@ int smc_launch_dense_rows(smc_ctx *ctx, const void *x, int x_bf16, int ldx, cons
             // at 128), so the narrowest tiles that one wave holds win.  Every output keeps its order of sums.  96 rows of 1024
             // outputs over K = 3072 ran on 8 CTAs (17.4 us); eight such prompts and eight steps of a 16-layer decoder: 16.14 -> 15.35 ms.
             const int slim = mt * ((N + 31) / 32) <= sms ? 32 : mt * ((N + 63) / 64) <= sms ? 64 : 0;
-            // and where clusters of such tiles still fit one wave, a cluster shares a tile, with at least four steps of K per CTA
-            const long long tiles32 = mt * ((N + 31) / 32), steps = (K + TC_K - 1) / TC_K;
-            const int split = 4 * tiles32 <= sms && steps >= 16 ? 4 : 2 * tiles32 <= sms && steps >= 8 ? 2 : 1;
             auto tc = [&](auto epi) {
                 constexpr int E = decltype(epi)::value;
-                if (slim == 32) {
-                    if (split == 4) return launch_tc<32, E, 4>(ctx, xb, ldx, w, M, N, K, o, s);
-                    return split == 2 ? launch_tc<32, E, 2>(ctx, xb, ldx, w, M, N, K, o, s) : launch_tc<32, E>(ctx, xb, ldx, w, M, N, K, o, s);
-                }
+                if (slim == 32) return launch_tc<32, E>(ctx, xb, ldx, w, M, N, K, o, s);
                 if (slim == 64) return launch_tc<64, E>(ctx, xb, ldx, w, M, N, K, o, s);
                 return 5 * wide <= 6 * narrow ? launch_tc<256, E>(ctx, xb, ldx, w, M, N, K, o, s) : launch_tc<128, E>(ctx, xb, ldx, w, M, N, K, o, s);
             };

@@ -107,9 +107,9 @@ def test_dense_matmul_tile_widths_of_short_prompts(cuda, dev, n):
 
 
 @pytest.mark.parametrize("m,n,k", [(33, 40, 512), (96, 1024, 1024), (128, 1184, 1016), (65, 1184, 1080), (96, 2336, 3072), (100, 2400, 520), (300, 200, 4100 // 4 * 8)])
-def test_dense_matmul_with_k_shared_by_a_cluster(cuda, dev, m, n, k):
-    """Few tiles over a long K: two or four CTAs share a tile and K, in whole and ragged steps of 64.  fp32 sums of exact products: against
-    64 bits, 1e-5 of the norms."""
+def test_dense_matmul_of_few_tiles_over_a_long_k(cuda, dev, m, n, k):
+    """Few tiles over whole and ragged steps of 64.  fp32 sums of exact products: against 64 bits, 1e-5 of the norms; and the order of a row's
+    sums is that of every other tile width: the same rows inside a batch that fills the device with wide tiles have the same bits."""
     import torch
 
     from sharpmind_b200 import ops
@@ -118,10 +118,13 @@ def test_dense_matmul_with_k_shared_by_a_cluster(cuda, dev, m, n, k):
     w = torch.randn((n, k), generator=g, device="cuda").to(torch.bfloat16)
     x = torch.randn((m, k), generator=g, device="cuda")
     h = cuda.register_dev(w.view(torch.uint8).reshape(-1), ops.QuantDType.BF16, n, k, repack=False)
-    got = dev.qmatmul(x, h, ops.Mode.ACT_BF16).double()
+    got = dev.qmatmul(x, h, ops.Mode.ACT_BF16)
     x16 = x.to(torch.bfloat16).double()
     bound = 1e-5 * x16.norm(dim=1)[:, None] * w.double().norm(dim=1)[None]
-    assert bool(((got - x16 @ w.double().T).abs() <= bound).all())
+    assert bool(((got.double() - x16 @ w.double().T).abs() <= bound).all())
+    row_tiles = torch.cuda.get_device_properties(0).multi_processor_count // ((n + 63) // 64) + 1  # of 128 rows: no tile of 64 columns fits one wave
+    many = x.repeat((128 * row_tiles + m - 1) // m, 1)
+    assert torch.equal(dev.qmatmul(many, h, ops.Mode.ACT_BF16)[:m].view(torch.int32), got.view(torch.int32))
     cuda.release(h)
     assert cuda.device_status() == 0
 
