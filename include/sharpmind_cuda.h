@@ -22,7 +22,8 @@
  * queue work on the caller's stream; those that keep intermediate data in buffers owned by the context
  * (smc_qmatmul_dev with SMC_ACT_Q8 or SMC_ACT_F32 for M > 1 or shapes the one-row kernel does not take, smc_qmatmul_q8_dev
  * over Q4_K at 64 rows and more, smc_qmatmul_tc_dev,
- * smc_sdpa_decode_dev, smc_argmax_dev, smc_decode_step, smc_forward_last_logits) reuse those buffers in stream
+ * smc_sdpa_decode_dev, smc_sdpa_kv_dev with one query row, smc_argmax_dev, smc_decode_step, smc_forward_last_logits,
+ * smc_forward_logits, smc_forward_rows) reuse those buffers in stream
  * order: all such calls on one context must go to ONE stream (or be ordered by events).  Work that is to run
  * concurrently on several streams takes one context per stream.
  * Such a buffer grows with the first call that needs more of it, after a device-wide synchronisation: make that call outside
@@ -331,7 +332,10 @@ SMC_API int smc_kv_append_dev(smc_ctx *ctx, const float *d_k, const float *d_v, 
  * IKVCache (SharpMind.Model/IKVCache.cs:7-18) on the device: KVCache (fp32, KVCache.cs) and QuantizedKVCache with Q8_0
  * rows (QuantizedKVCache.cs).  One object holds the keys and values of one attention layer for `batch` lock-step
  * sequences that share one position (CurrentPosition), as the reference's caches do.  Host-side state (the length)
- * changes when the call returns; device work is queued on `stream`, so calls on one object go to one stream. */
+ * changes when the call returns; device work is queued on `stream`, so calls on one object go to one stream.
+ * Attention over several query rows (smc_sdpa_kv_dev, headDim 64 or 128) keeps its intermediate data in a buffer of the object: 12 bytes per
+ * element of K for maxSeq positions of one sequence, 256 MB at most, allocated by the object's first such call and freed with it.  So objects
+ * may be attended to on different streams, and a captured call holds as long as its object. */
 typedef struct smc_kv smc_kv;
 enum { SMC_KV_F32 = 0, SMC_KV_Q8_0 = 8 };
 SMC_API int smc_kv_create(smc_ctx *ctx, int batch, int kvHeads, int maxSeq, int headDim, int kind, smc_kv **out);

@@ -236,7 +236,6 @@ void smc_destroy(smc_ctx *ctx)
     cudaFree(ctx->d_stage_aux);
     cudaFree(ctx->d_attn_part);
     cudaFree(ctx->d_prefill);
-    cudaFree(ctx->d_attn_planes);
     cudaFree(ctx->d_argmax);
     cudaFree(ctx->d_status);
     if (ctx->h_pin) cudaFreeHost(ctx->h_pin);

@@ -12,7 +12,7 @@
 // the same way once per CTA.  The score tile's accumulator layout is the A-operand layout of the next MMA for
 // 16-bit types, so P goes from registers to registers.  Online softmax per row as in the scalar kernel.
 // sm_100a runs mma.sync on its legacy tensor path.  smc_attention_tc.cu is the tcgen05 form, with the same bits; this kernel stays for calls of
-// one key tile, outputs off 16 bytes, one head per CTA (an option) and calls that find no room for the other's planes.
+// one key tile, outputs off 16 bytes, one head per CTA (an option) and calls that the other's planes do not reach (a very long cache, a full device).
 #include <cuda_bf16.h>
 
 #include "smc_common.cuh"
@@ -545,8 +545,8 @@ __global__ void __launch_bounds__(256, 2) sdpa_few_rows_kernel(const float *__re
 bool smc_sdpa_prefill_mma_supported(int nh, int nkv, int hd) { return (hd == 64 || hd == 128) && nkv > 0 && nh % nkv == 0; }
 
 // kd == null: kc / vc are fp32 rows; else the int8 planes and fp16 block scales of a Q8_0 cache
-static int launch_prefill_mma(smc_ctx *ctx, const float *q, const void *kc, const void *vc, const __half *kd, const __half *vd, float *out,
-                              int T, int nh, int nkv, int hd, int pos0, int maxSeq, float scale, cudaStream_t s)
+static int launch_prefill_mma(smc_ctx *ctx, smc_attn_planes *planes, const float *q, const void *kc, const void *vc, const __half *kd, const __half *vd,
+                              float *out, int T, int nh, int nkv, int hd, int pos0, int maxSeq, float scale, cudaStream_t s)
 {
     const int G = nh / nkv;
     // the order matters: a few rows over a long fp32 cache, then the tcgen05 kernel; all of them give the same bits
@@ -574,8 +574,8 @@ static int launch_prefill_mma(smc_ctx *ctx, const float *q, const void *kc, cons
     // More than one tile of keys: tcgen05, two launches.  16 heads of 128: 20 rows (one tile) 10.8 us here, 13.1 there; 33 rows of 4 heads
     // 16.0 / 13.8; 64 rows of 32 heads 18.0 / 14.3; 100 rows behind 1900 keys of a Q8_0 cache 398 / 149; 2048 rows 362 / 164.
     if (tiles > 1 && ctx->attn_hpc != 1 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
-        const int rc = smc_launch_sdpa_prefill_tc(ctx, q, kc, vc, kd, vd, out, T, nh, nkv, hd, pos0, maxSeq, scale, s);
-        if (rc != SMC_E_UNSUPPORTED) return rc;  // else there is no room for the planes (a first call under capture, a very long cache)
+        const int rc = smc_launch_sdpa_prefill_tc(ctx, planes, q, kc, vc, kd, vd, out, T, nh, nkv, hd, pos0, maxSeq, scale, s);
+        if (rc != SMC_E_UNSUPPORTED) return rc;  // else the planes do not reach that far (a very long cache, a full device)
     }
     if (kd) {
         if (hd == 128) two ? go(sdpa_prefill_mma_kernel<128, 2, true>, 2) : go(sdpa_prefill_mma_kernel<128, 1, true>, 1);
@@ -588,15 +588,15 @@ static int launch_prefill_mma(smc_ctx *ctx, const float *q, const void *kc, cons
     return SMC_OK;
 }
 
-int smc_launch_sdpa_prefill_mma(smc_ctx *ctx, const float *q, const float *kc, const float *vc, float *out, int T, int nh, int nkv,
+int smc_launch_sdpa_prefill_mma(smc_ctx *ctx, smc_attn_planes *planes, const float *q, const float *kc, const float *vc, float *out, int T, int nh, int nkv,
                                 int hd, int pos0, int maxSeq, float scale, cudaStream_t s)
 {
-    return launch_prefill_mma(ctx, q, kc, vc, nullptr, nullptr, out, T, nh, nkv, hd, pos0, maxSeq, scale, s);
+    return launch_prefill_mma(ctx, planes, q, kc, vc, nullptr, nullptr, out, T, nh, nkv, hd, pos0, maxSeq, scale, s);
 }
 
 // one sequence's Q8_0 cache planes (rows pos0 .. pos0 + T - 1 are the queries' own positions)
-int smc_launch_sdpa_prefill_mma_q8(smc_ctx *ctx, const float *q, const int8_t *kq, const __half *kd, const int8_t *vq, const __half *vd,
-                                   float *out, int T, int nh, int nkv, int hd, int pos0, int maxSeq, float scale, cudaStream_t s)
+int smc_launch_sdpa_prefill_mma_q8(smc_ctx *ctx, smc_attn_planes *planes, const float *q, const int8_t *kq, const __half *kd, const int8_t *vq,
+                                   const __half *vd, float *out, int T, int nh, int nkv, int hd, int pos0, int maxSeq, float scale, cudaStream_t s)
 {
-    return launch_prefill_mma(ctx, q, kq, vq, kd, vd, out, T, nh, nkv, hd, pos0, maxSeq, scale, s);
+    return launch_prefill_mma(ctx, planes, q, kq, vq, kd, vd, out, T, nh, nkv, hd, pos0, maxSeq, scale, s);
 }

@@ -8,7 +8,7 @@
 // the lanes' partial row sums in the shuffle's order.  So an output has the bits it has in the other kernel.
 //
 // attn_planes_kernel first writes the three planes of all keys and values a call sees, in the tensor cores' core-matrix order, V
-// transposed, to the context's scratch: once per KV head instead of once per query head and row tile (split inside the attention kernel,
+// transposed, to scratch of the model or cache object: once per KV head instead of once per query head and row tile (split inside the attention kernel,
 // by eight more warps, 2048 rows of 16 heads took 214 us, over a Q8_0 cache 281).
 //
 // One CTA = 128 query rows of one head; keys in chunks of 64, two tiles of 32.  Warp roles:
@@ -34,7 +34,7 @@
 
 namespace {
 
-constexpr size_t ATTN_PLANES_MOST = 256u << 20;  // 12 bytes an element of K: 21 000 positions of eight heads of 128
+constexpr size_t ATTN_PLANES_MOST = 256u << 20;  // of an object: 12 bytes an element of K, 21 000 positions of eight heads of 128; longer calls run on mma.sync
 constexpr int ROWS = 128, KT = 32, CHUNK = 2 * KT, STAGES = 2;
 constexpr int WARP_LOAD = 8, WARP_MMA = 9, THREADS = 32 * (WARP_MMA + 1);
 
@@ -403,38 +403,34 @@ sdpa_prefill_tc_kernel(const float *__restrict__ q, const uint8_t *__restrict__ 
 
 }  // namespace
 
-// The planes' buffer: grown on demand up to a limit, not under stream capture.  False: the caller takes another kernel.
-static bool planes_fit(smc_ctx *ctx, size_t bytes, cudaStream_t s)
+static size_t stage_bytes(int hd) { return hd == 128 ? Shape<128>::STAGE : Shape<64>::STAGE; }
+
+// One buffer for all lengths that the cache can have, up to a limit: nothing grows with the context and nothing is freed before the object.
+// Without one (a full device) the calls take the mma.sync kernel.  cudaMalloc touches no stream, so the thread may ask for it while it, or
+// another, captures one.
+void smc_attn_planes_reserve(smc_attn_planes *planes, int kvHeads, int headDim, int maxSeq)
 {
-    if (bytes <= ctx->attn_planes_cap) return true;
-    if (bytes > ATTN_PLANES_MOST) return false;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+    if (planes->reserved) return;
+    planes->reserved = true;
+    const size_t want = (size_t)kvHeads * ((maxSeq + (size_t)CHUNK - 1) / CHUNK) * stage_bytes(headDim);
+    planes->bytes = want < ATTN_PLANES_MOST ? want : ATTN_PLANES_MOST;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (cudaMalloc(&planes->d, planes->bytes) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        planes->d = nullptr, planes->bytes = 0;
     }
-    if (ctx->d_attn_planes) {
-        cudaDeviceSynchronize();  // earlier calls may be reading it
-        cudaFree(ctx->d_attn_planes);
-        ctx->d_attn_planes = nullptr, ctx->attn_planes_cap = 0;
-    }
-    if (cudaMalloc(&ctx->d_attn_planes, bytes) != cudaSuccess) {
-        cudaGetLastError();
-        ctx->d_attn_planes = nullptr;
-        return false;
-    }
-    ctx->attn_planes_cap = bytes;
-    return true;
+    cudaThreadExchangeStreamCaptureMode(&mode);
 }
 
-int smc_launch_sdpa_prefill_tc(smc_ctx *ctx, const float *q, const void *kc, const void *vc, const __half *kd, const __half *vd, float *out, int T, int nh,
-                               int nkv, int hd, int pos0, int maxSeq, float scale, cudaStream_t s)
+int smc_launch_sdpa_prefill_tc(smc_ctx *ctx, smc_attn_planes *own, const float *q, const void *kc, const void *vc, const __half *kd, const __half *vd, float *out,
+                               int T, int nh, int nkv, int hd, int pos0, int maxSeq, float scale, cudaStream_t s)
 {
     const int chunks = (pos0 + T + CHUNK - 1) / CHUNK;
-    const size_t bytes = (size_t)nkv * chunks * (hd == 128 ? Shape<128>::STAGE : Shape<64>::STAGE);
-    std::lock_guard<std::mutex> lock(ctx->mu_attn);  // until everything that uses the planes is queued
-    if (!planes_fit(ctx, bytes, s)) return SMC_E_UNSUPPORTED;
-    uint8_t *planes = static_cast<uint8_t *>(ctx->d_attn_planes);
+    std::lock_guard<std::mutex> lock(ctx->mu_attn);  // two threads on the object's stream: not one's attention between the other's two launches
+    smc_attn_planes_reserve(own, nkv, hd, maxSeq);
+    if ((size_t)nkv * chunks * stage_bytes(hd) > own->bytes) return SMC_E_UNSUPPORTED;
+    uint8_t *planes = own->d;
     auto go = [&](auto split, auto kernel, size_t smem) {
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         smc_launch_dep(ctx->use_pdl, split, dim3(chunks, nkv), dim3(256), 0, s, kc, vc, kd, vd, planes, pos0 + T, maxSeq);

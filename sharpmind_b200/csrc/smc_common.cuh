@@ -105,13 +105,20 @@ struct smc_ctx {
     int mt_ring = 0;                              // 2..32 rows, weights through the bulk-copy ring: 0 never, 1 Q4_K, 2 every format
     void *d_argmax = nullptr;          // chunk results and tickets of the argmax
     int argmax_rows = 0, argmax_chunks = 0;
-    std::mutex mu_attn;                // guards d_attn_planes, until the launches that use it are queued
-    void *d_attn_planes = nullptr;     // keys and values of a prompt's attention as bfloat16 planes
-    size_t attn_planes_cap = 0;
+    std::mutex mu_attn;                // held while a prompt attention's two launches, which share its object's planes, are queued
     void *d_prefill = nullptr;         // activation image of the tensor-core matmul
     size_t prefill_cap = 0;
     float *d_attn_part = nullptr;      // split-KV partial results
     size_t attn_part_cap = 0;
+};
+
+// Keys and values of a prompt's attention as bfloat16 planes (smc_attention_tc.cu).  They belong to the model or cache object whose rows they
+// are made from: work on one such object is on one stream, so no other call can write them meanwhile, and they keep their address until the
+// object goes, so a captured call stays valid as long as the object.
+struct smc_attn_planes {
+    uint8_t *d = nullptr;
+    size_t bytes = 0;
+    bool reserved = false;
 };
 
 int smc_fail(smc_ctx *ctx, int code, const char *fmt, ...);
@@ -168,11 +175,12 @@ int smc_launch_prefill_q4k_q8(smc_ctx *, const smc_q8act *a, const smc_weight *,
 bool smc_mma_supported(const smc_weight *, int M);
 bool smc_mt_supported(const smc_weight *, int M);
 bool smc_sdpa_prefill_mma_supported(int nh, int nkv, int hd);
-int smc_launch_sdpa_prefill_tc(smc_ctx *, const float *q, const void *kc, const void *vc, const __half *kd, const __half *vd, float *out, int T, int nh, int nkv,
-                               int hd, int pos0, int maxSeq, float scale, cudaStream_t s);
-int smc_launch_sdpa_prefill_mma(smc_ctx *, const float *q, const float *kc, const float *vc, float *out, int T, int nh, int nkv, int hd,
+void smc_attn_planes_reserve(smc_attn_planes *, int kvHeads, int headDim, int maxSeq);  // the first call allocates, later ones return at once
+int smc_launch_sdpa_prefill_tc(smc_ctx *, smc_attn_planes *, const float *q, const void *kc, const void *vc, const __half *kd, const __half *vd, float *out, int T,
+                               int nh, int nkv, int hd, int pos0, int maxSeq, float scale, cudaStream_t s);
+int smc_launch_sdpa_prefill_mma(smc_ctx *, smc_attn_planes *planes, const float *q, const float *kc, const float *vc, float *out, int T, int nh, int nkv, int hd,
                                 int pos0, int maxSeq, float scale, cudaStream_t s);
-int smc_launch_sdpa_prefill_mma_q8(smc_ctx *ctx, const float *q, const int8_t *kq, const __half *kd, const int8_t *vq, const __half *vd,
+int smc_launch_sdpa_prefill_mma_q8(smc_ctx *ctx, smc_attn_planes *planes, const float *q, const int8_t *kq, const __half *kd, const int8_t *vq, const __half *vd,
                                    float *out, int T, int nh, int nkv, int hd, int pos0, int maxSeq, float scale, cudaStream_t s);
 int smc_launch_gemv_mt(smc_ctx *, const smc_q8act *, const smc_weight *, float *out, cudaStream_t s);
 int smc_launch_gemv_mma(smc_ctx *, const smc_q8act *, const smc_weight *, float *out, cudaStream_t s);
@@ -192,10 +200,10 @@ int smc_launch_repack(smc_ctx *, smc_weight *, cudaStream_t s);
 int smc_sdpa_decode_any(smc_ctx *, const float *d_q, const void *d_k, const void *d_v, const __half *d_kd, const __half *d_vd,
                         float *d_out, int batch, int heads, int kvHeads, int headDim, int kvLen, int maxSeq, float scale,
                         cudaStream_t stream);
-int smc_launch_sdpa_q8_rows(smc_ctx *ctx, const float *q, const int8_t *kq, const __half *kd, const int8_t *vq, const __half *vd, float *out,
+int smc_launch_sdpa_q8_rows(smc_ctx *ctx, smc_attn_planes *planes, const float *q, const int8_t *kq, const __half *kd, const int8_t *vq, const __half *vd, float *out,
                             int batch, int seqLen, int heads, int kvHeads, int hd, int kvLen, int maxSeq, float scale, cudaStream_t s);
 int smc_sdpa_decode_reserve(smc_ctx *, int max_batch, int heads, int kvHeads, int headDim, int maxSeq);
-int smc_launch_sdpa_prefill(smc_ctx *ctx, const float *q, const float *kc, const float *vc, float *out, int T, int nh, int nkv,
+int smc_launch_sdpa_prefill(smc_ctx *ctx, smc_attn_planes *planes, const float *q, const float *kc, const float *vc, float *out, int T, int nh, int nkv,
                             int hd, int pos0, int maxSeq, float scale, cudaStream_t s);
 int smc_launch_sdpa_tile(smc_ctx *, const float *q, const float *k, const float *v, float *o, int seqLen, int kvLen,
                          int hd, float scale, int causal, int qStride, int oStride, float alibi, cudaStream_t s);

@@ -37,6 +37,7 @@ struct smc_model {
     float *cosT = nullptr, *sinT = nullptr;
     float *x = nullptr, *xn = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *att = nullptr, *tmp = nullptr,
           *gu = nullptr, *act = nullptr;
+    smc_attn_planes planes;                  // scratch of a prompt's attention, for one layer of one sequence at a time
     smc_q8act *qa = nullptr, *qb = nullptr;  // quantised activations for batch > 1 (hidden-sized / widest row)
 };
 
@@ -48,7 +49,7 @@ void free_model(smc_ctx *ctx, smc_model *m)
     smc_layered_free(m->layered);
     float *bufs[] = {m->kcache, m->vcache, m->cosT, m->sinT, m->x, m->xn, m->q, m->k, m->v, m->att, m->tmp, m->gu, m->act, m->qkv, m->x2};
     for (float *p : bufs) cudaFree(p);
-    cudaFree(m->kq8), cudaFree(m->vq8), cudaFree(m->kd8), cudaFree(m->vd8);
+    cudaFree(m->kq8), cudaFree(m->vq8), cudaFree(m->kd8), cudaFree(m->vd8), cudaFree(m->planes.d);
     for (smc_weight *w : m->wqkv)
         if (w) smc_weight_release(ctx, w);
     for (float *b : m->bqkv) cudaFree(b);
@@ -463,12 +464,13 @@ int smc_model_create(smc_ctx *ctx, const smc_model_desc *desc, int max_batch, sm
         return rc;
     }
     rc = smc_rope_tables(ctx, d.rope_theta, d.head_dim, d.max_seq, m->cosT, m->sinT);
-    // the attention's scratch for every step this model can run: decoding never allocates
+    // the attention's scratch for every step and prompt this model can run: decoding and later chunks never allocate
     if (!rc && (d.head_dim == 64 || d.head_dim == 128)) rc = smc_sdpa_decode_reserve(ctx, max_batch, d.n_heads, d.n_kv_heads, d.head_dim, d.max_seq);
     if (rc) {
         free_model(ctx, m);
         return rc;
     }
+    if (d.head_dim == 64 || d.head_dim == 128) smc_attn_planes_reserve(&m->planes, d.n_kv_heads, d.head_dim, d.max_seq);
     *out = m;
     return SMC_OK;
 }
@@ -681,10 +683,10 @@ static int forward_tokens(smc_ctx *ctx, smc_model *m, const int *d_tokens, int s
         SMC_TRY(launch_qkv_post(ctx, m, l, kc, vc, T, pos, s, seq));
         if (m->kv_q8) {
             const size_t le = layer_elems(m);
-            SMC_TRY(smc_launch_sdpa_q8_rows(ctx, m->q, m->kq8 + l * le + seq_off, m->kd8 + (l * le + seq_off) / 32, m->vq8 + l * le + seq_off,
+            SMC_TRY(smc_launch_sdpa_q8_rows(ctx, &m->planes, m->q, m->kq8 + l * le + seq_off, m->kd8 + (l * le + seq_off) / 32, m->vq8 + l * le + seq_off,
                                             m->vd8 + (l * le + seq_off) / 32, m->att, 1, T, nh, nkv, hd, pos + T, d.max_seq, scale, s));
         } else {
-            SMC_TRY(smc_launch_sdpa_prefill(ctx, m->q, kc + seq_off, vc + seq_off, m->att, T, nh, nkv, hd, pos, d.max_seq, scale, s));
+            SMC_TRY(smc_launch_sdpa_prefill(ctx, &m->planes, m->q, kc + seq_off, vc + seq_off, m->att, T, nh, nkv, hd, pos, d.max_seq, scale, s));
         }
         if (reuse) SMC_TRY(smc_quantize_q8_dev(ctx, m->att, T, qDim, m->qb, s));
         SMC_TRY(linear(ctx, m->att, m->wo[l], m->tmp, T, mode, reuse ? m->qb : nullptr, s, m->bo[l]));

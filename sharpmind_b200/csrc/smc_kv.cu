@@ -21,6 +21,7 @@ struct smc_kv {
     float *k = nullptr, *v = nullptr;        // fp32 planes
     int8_t *kq = nullptr, *vq = nullptr;     // Q8_0 quants
     __half *kd = nullptr, *vd = nullptr;     // Q8_0 block scales
+    mutable smc_attn_planes planes;          // scratch of attention over several query rows
 };
 
 namespace {
@@ -252,15 +253,15 @@ void smc_kv_planes(const smc_kv *kv, void **k, void **v, __half **kd, __half **v
 }
 
 // q, out [batch, seqLen, heads, hd]; the planes belong to `batch` sequences of kvHeads heads with maxSeq rows each
-int smc_launch_sdpa_q8_rows(smc_ctx *ctx, const float *q, const int8_t *kq, const __half *kd, const int8_t *vq, const __half *vd, float *out,
-                            int batch, int seqLen, int heads, int kvHeads, int hd, int kvLen, int maxSeq, float scale, cudaStream_t s)
+int smc_launch_sdpa_q8_rows(smc_ctx *ctx, smc_attn_planes *planes, const float *q, const int8_t *kq, const __half *kd, const int8_t *vq, const __half *vd,
+                            float *out, int batch, int seqLen, int heads, int kvHeads, int hd, int kvLen, int maxSeq, float scale, cudaStream_t s)
 {
     if (hd != 64 && hd != 128) return smc_fail(ctx, SMC_E_UNSUPPORTED, "a Q8_0 cache with headDim %d (64 and 128 are built)", hd);
     // a chunk of a prompt (16 rows and more): the tensor-core kernel, one sequence at a time, its K / V tiles staged as d * q
     if (ctx->attn_mma && seqLen >= 16 && smc_sdpa_prefill_mma_supported(heads, kvHeads, hd)) {
         const size_t per_seq = (size_t)kvHeads * maxSeq * hd;
         for (int b = 0; b < batch; ++b) {
-            const int rc = smc_launch_sdpa_prefill_mma_q8(ctx, q + (size_t)b * seqLen * heads * hd, kq + b * per_seq, kd + b * (per_seq / 32),
+            const int rc = smc_launch_sdpa_prefill_mma_q8(ctx, planes, q + (size_t)b * seqLen * heads * hd, kq + b * per_seq, kd + b * (per_seq / 32),
                                                           vq + b * per_seq, vd + b * (per_seq / 32), out + (size_t)b * seqLen * heads * hd,
                                                           seqLen, heads, kvHeads, hd, kvLen - seqLen, maxSeq, scale, s);
             if (rc) return rc;
@@ -316,7 +317,7 @@ int smc_kv_destroy(smc_ctx *ctx, smc_kv *kv)
     if (!kv) return smc_fail(ctx, SMC_E_INVALID, "kv_destroy: bad arguments");
     if (ctx) cudaSetDevice(ctx->device);
     cudaDeviceSynchronize();
-    cudaFree(kv->k), cudaFree(kv->v), cudaFree(kv->kq), cudaFree(kv->vq), cudaFree(kv->kd), cudaFree(kv->vd);
+    cudaFree(kv->k), cudaFree(kv->v), cudaFree(kv->kq), cudaFree(kv->vq), cudaFree(kv->kd), cudaFree(kv->vd), cudaFree(kv->planes.d);
     delete kv;
     return SMC_OK;
 }
@@ -467,13 +468,13 @@ int smc_sdpa_kv_dev(smc_ctx *ctx, const smc_kv *kv, const float *d_q, float *d_o
         return smc_sdpa_decode_any(ctx, d_q, kv->k, kv->v, nullptr, nullptr, d_out, batch, heads, kv->kv_heads, hd, kv->length, kv->max_seq, scale, s);
     }
     if (kv->kind == SMC_KV_Q8_0)
-        return smc_launch_sdpa_q8_rows(ctx, d_q, kv->kq, kv->kd, kv->vq, kv->vd, d_out, batch, seqLen, heads, kv->kv_heads, hd, kv->length,
+        return smc_launch_sdpa_q8_rows(ctx, &kv->planes, d_q, kv->kq, kv->kd, kv->vq, kv->vd, d_out, batch, seqLen, heads, kv->kv_heads, hd, kv->length,
                                        kv->max_seq, scale, s);
     // fp32 cache, several query rows: the prompt kernel, one sequence at a time
     if (hd != 64 && hd != 128) return smc_fail(ctx, SMC_E_UNSUPPORTED, "sdpa_kv: several query rows need headDim 64 or 128");
     const size_t per_seq = (size_t)kv->kv_heads * kv->max_seq * hd;
     for (int b = 0; b < batch; ++b) {
-        int rc = smc_launch_sdpa_prefill(ctx, d_q + (size_t)b * seqLen * heads * hd, kv->k + b * per_seq, kv->v + b * per_seq,
+        int rc = smc_launch_sdpa_prefill(ctx, &kv->planes, d_q + (size_t)b * seqLen * heads * hd, kv->k + b * per_seq, kv->v + b * per_seq,
                                          d_out + (size_t)b * seqLen * heads * hd, seqLen, heads, kv->kv_heads, hd, kv->length - seqLen,
                                          kv->max_seq, scale, s);
         if (rc) return rc;

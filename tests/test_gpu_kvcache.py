@@ -313,7 +313,7 @@ def test_prompt_attention_on_tcgen05_gives_the_bits_of_mma_sync(cuda, kind, hd, 
 
 
 def test_prompt_attention_first_called_under_capture():
-    """Without room for its planes, and none to be had under capture, the call takes the mma.sync kernel: same bits."""
+    """The object's planes are allocated by its first call, a captured one too: the bits of an eager call, here and replayed after longer ones."""
     import torch
 
     ctx = ops.CudaContext(0)
@@ -328,6 +328,130 @@ def test_prompt_attention_first_called_under_capture():
     torch.cuda.synchronize()
     want = kv.attention(q, 128 ** -0.5)
     assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+    other = ops.KVCache(ctx, 1, 2, 2000, 128, ops.KVCache.F32)
+    other.Update(*(to_dev(synth.normal("kvcap", "o" + n, (1, 2000, 2, 128))) for n in "kv"))
+    other.attention(to_dev(synth.normal("kvcap", "oq", (1, 300, 4, 128))), 128 ** -0.5)
+    got.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got.view(torch.int32), want.view(torch.int32))
     assert ctx.device_status() == 0
+    graph.reset()
+    kv.Dispose(), other.Dispose()
+    ctx.close()
+
+
+@pytest.mark.parametrize("kind", ["f32", "q8_0"])
+def test_prompt_attention_of_two_caches_on_two_streams(cuda, kind):
+    """Two cache objects of one context, each on a stream of its own, their calls interleaved without a wait: the bits that each gives alone."""
+    import torch
+
+    shapes = [(700, 190), (650, 150)]  # positions, query rows
+    caches, queries, want = [], [], []
+    for i, (n, s) in enumerate(shapes):
+        kv = ops.KVCache(cuda, 2, 2, n, 128, ops.KVCache.Q8_0 if kind == "q8_0" else ops.KVCache.F32)
+        kv.Update(*(to_dev(synth.normal("kv2s", f"{x}{i}", (2, n, 2, 128))) for x in "kv"))
+        caches.append(kv), queries.append(to_dev(synth.normal("kv2s", f"q{i}", (2, s, 4, 128))))
+        want.append(kv.attention(queries[i], 128 ** -0.5))
+    torch.cuda.synchronize()
+    streams, got = [torch.cuda.Stream(), torch.cuda.Stream()], [[], []]
+    for _ in range(30):
+        for i in (0, 1):
+            with torch.cuda.stream(streams[i]):
+                got[i].append(caches[i].attention(queries[i], 128 ** -0.5))
+    torch.cuda.synchronize()
+    for i in (0, 1):
+        assert all(torch.equal(g.view(torch.int32), want[i].view(torch.int32)) for g in got[i]), i
+        caches[i].Dispose()
+    assert cuda.device_status() == 0
+
+
+def test_prompt_attention_allocates_once_per_cache():
+    """The first call over several rows takes room for all positions; the device's free memory stays what it is over the rest of the prompt."""
+    import torch
+
+    n, s, ctx = 4096, 512, ops.CudaContext(0)
+    kv = ops.KVCache(ctx, 1, 8, n, 128, ops.KVCache.F32)
+    k, v = (to_dev(synth.normal("kvone", x, (1, n, 8, 128))) for x in "kv")
+    q = to_dev(synth.normal("kvone", "q", (1, s, 16, 128)))
+    free = []
+    for start in range(0, n, s):
+        kv.Update(k[:, start:start + s].contiguous(), v[:, start:start + s].contiguous())
+        kv.attention(q, 128 ** -0.5)
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+    assert len(set(free)) == 1, free
     kv.Dispose()
     ctx.close()
+
+
+def _prompt_model(oracle, ctx, kv_dtype, max_seq, kv_heads=2):
+    from sharpmind_b200.decoder import Decoder
+
+    cfg = dict(n_layers=2, hidden=256, n_heads=kv_heads * 2, n_kv_heads=kv_heads, head_dim=128, ffn=512, vocab=1024, max_seq=max_seq, dtype=8, eps=1e-6,
+               rope_theta=1.0e6, neox=True, qk_norm=True, kv_dtype=kv_dtype)
+    return Decoder(ctx, cfg, synth.make_decoder_weights(cfg, "kvprompt", oracle.quantize), max_batch=1)
+
+
+@pytest.mark.parametrize("kv_dtype", [0, 8])
+def test_prompt_in_chunks_allocates_nothing(oracle, kv_dtype):
+    """After the first chunk (activation rows) no chunk of a prompt allocates: the attention's planes are there from the model's creation."""
+    import torch
+
+    n, chunk, ctx = 4096, 256, ops.CudaContext(0)
+    dec = _prompt_model(oracle, ctx, kv_dtype, n, kv_heads=16)
+    tokens = torch.from_numpy(synth.token_ids("kvprompt", "chunks", (n,), 1024)).cuda()
+    free = []
+    for start in range(0, n, chunk):
+        dec.forward_last_logits(tokens[start:start + chunk], pos=start)
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+    assert len(set(free)) == 1, free
+    dec.close()
+    ctx.close()
+
+
+@pytest.mark.parametrize("kv_dtype", [0, 8])
+def test_captured_prompt_pass_outlives_longer_contexts(oracle, cuda, kv_dtype):
+    """A captured prompt pass replayed after eager passes further into the cache, of this model and of a larger one: the same logits."""
+    import torch
+
+    n = 256
+    dec, big = _prompt_model(oracle, cuda, kv_dtype, 1024), _prompt_model(oracle, cuda, kv_dtype, 4096)
+    tokens = torch.from_numpy(synth.token_ids("kvprompt", "cap", (1024,), 1024)).cuda()
+    first = tokens[:n].contiguous()
+    want = dec.forward_last_logits(first)[0].clone()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got, _ = dec.forward_last_logits(first)
+    for pos in (n, 2 * n, 3 * n):
+        dec.forward_last_logits(tokens[pos:pos + n], pos=pos)
+    big.forward_last_logits(tokens[:n], pos=3000)
+    torch.cuda.synchronize()
+    got.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+    assert cuda.device_status() == 0
+    graph.reset()
+    dec.close(), big.close()
+
+
+@pytest.mark.parametrize("kind", ["f32", "q8_0"])
+@pytest.mark.parametrize("hd,heads,kvh", [(128, 4, 2), (64, 4, 1), (64, 3, 1)])
+def test_prompt_attention_off_16_byte_outputs(cuda, kind, hd, heads, kvh):
+    """Outputs that the tcgen05 kernel does not take (8 bytes off a multiple of 16) go to the mma.sync kernel, two heads per CTA where they share a
+    KV head: the same bits, over several key tiles and row tiles."""
+    import torch
+
+    for n0, s in ((0, 130), (77, 100)):
+        kv = ops.KVCache(cuda, 1, kvh, n0 + s, hd, ops.KVCache.Q8_0 if kind == "q8_0" else ops.KVCache.F32)
+        kv.Update(*(to_dev(synth.normal("kvoff", f"{x}{hd}{s}", (1, n0 + s, kvh, hd))) for x in "kv"))
+        q = to_dev(synth.normal("kvoff", f"q{hd}{s}", (1, s, heads, hd)))
+        want = kv.attention(q, hd ** -0.5)
+        room = torch.empty(q.numel() + 4, dtype=torch.float32, device="cuda")
+        got = room[2:2 + q.numel()]
+        cuda.check(cuda.lib.smc_sdpa_kv_dev(cuda.h, kv.h, q.data_ptr(), got.data_ptr(), 1, heads, s, hd ** -0.5, kv._stream()))
+        assert torch.equal(got.view(torch.int32), want.flatten().view(torch.int32)), (n0, s)
+        kv.Dispose()
