@@ -1030,9 +1030,13 @@ int smc_launch_gemv_mma(smc_ctx *ctx, const smc_q8act *a, const smc_weight *w, f
     if (const int pt = prompt_tile(ctx, w, M)) {
         auto go = [&](auto kernel, size_t smem, int ncls) {
             cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            smc_launch_dep(ctx->use_pdl, kernel, dim3((N + TILE_ROWS - 1) / TILE_ROWS, (M + 16 * pt - 1) / (16 * pt)), dim3(TILE_THREADS), smem, s,
-                           w->dtype == SMC_Q6_K ? (const uint8_t *)w->q6u : (const uint8_t *)w->q8_qs, (const __half *)w->q8_d, (const int8_t *)a->q, (const float *)a->d,
-                           out, N, K, M, ncls);
+            const int tok = 16 * pt, most = 65535 * tok;  // tokens of a launch: what the grid's y takes
+            for (int t0 = 0; t0 < M; t0 += most) {
+                const int m = M - t0 < most ? M - t0 : most;
+                smc_launch_dep(ctx->use_pdl, kernel, dim3((N + TILE_ROWS - 1) / TILE_ROWS, (m + tok - 1) / tok), dim3(TILE_THREADS), smem, s,
+                               w->dtype == SMC_Q6_K ? (const uint8_t *)w->q6u : (const uint8_t *)w->q8_qs, (const __half *)w->q8_d, (const int8_t *)a->q + (size_t)t0 * K,
+                               (const float *)a->d + (size_t)t0 * (K / 32), out + (size_t)t0 * N, N, K, m, ncls);
+            }
         };
         if (w->dtype == SMC_Q6_K) {
             const int ncls = K >= 8192 ? 16 : 8;

@@ -146,6 +146,28 @@ def test_prompt_tiles_keep_the_small_batch_bits(cuda, dev, dtype, n, m, ks):
         cuda.release(w)
 
 
+def test_more_token_tiles_than_a_grid_holds():
+    """Rows beyond 65535 tiles of tokens: the last ones have the bits they have in a small batch."""
+    import torch
+
+    from sharpmind_b200 import ops
+    from sharpmind_b200.ops import Mode
+
+    n, k, m = 32, 128, 65535 * 128 + 100
+    g = torch.Generator(device="cuda").manual_seed(5)
+    ctx = ops.CudaContext(0)  # its scratch is for this many rows
+    dev = ops.DeviceOps(ctx)
+    w = ctx.register_dev(dev.quantize_weights(Q8_0, torch.randn((n, k), generator=g, device="cuda") * 0.02), Q8_0, n, k)
+    x = torch.randn((m, k), generator=g, device="cuda")
+    got = dev.qmatmul(x, w, Mode.ACT_Q8)
+    for lo in (0, 65535 * 64 - 8, 65535 * 128 - 8, m - 16):
+        want = dev.qmatmul(x[lo:lo + 16].contiguous(), w, Mode.ACT_Q8)
+        assert torch.equal(got[lo:lo + 16].view(torch.int32), want.view(torch.int32)), lo
+    ctx.release(w)
+    ctx.close()
+    torch.cuda.empty_cache()
+
+
 @pytest.mark.parametrize("dtype,n,ref_n,ref_m", [(Q8_0, 4700, 1000, 64), (Q8_0, 1000, 1000, 64), (Q4_K, 4700, 4000, 32), (Q4_K, 6100, 4000, 32), (Q4_K, 18900, 4000, 32),
                                                  (Q4_K, 700, 700, 32)])
 @pytest.mark.parametrize("k", [256, 2304, 4352])
