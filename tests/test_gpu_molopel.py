@@ -398,6 +398,22 @@ def test_wide_heads_many_tiles(cuda):
     m.close()
 
 
+@pytest.mark.parametrize("dim,vdim", [(64, 64), (128, 128), (40, 136)])
+def test_linear_heads_of_a_long_prompt(cuda, dim, vdim):
+    """Enough chunks and heads that a CTA takes a whole chunk (more than a quarter of the SMs have one each): 6 chunks of 8 heads, whole and in portions
+    whose last chunk is ragged."""
+    cfg = lu.molopel([lu.lightning(heads=8, dim=dim, vdim=vdim, ff=0),
+                      lu.parallel(window=40, right_heads=8, right_dim=dim, right_vdim=vdim, rot_dims=16, left_scale=0.1, ff=0)], width=64, vocab=96)
+    t16, w = lu.weights(cfg, 31)
+    tk = toks(1400, 96, 9)
+    want = lo.forward(cfg, w, tk)
+    m = build(cuda, cfg, t16, BF16, slots=2, max_seq=1408, chunk=704)
+    for cuts in ([], [640, 700, 60], [704, 641, 55]):
+        err = lu.rel_err(run(m, tk, cuts), want)
+        assert err.max() < TOL[BF16], (cuts, int(err.argmax()), float(err.max()))
+    m.close()
+
+
 @pytest.mark.parametrize("slots", [5, 9, 18, 40])
 def test_large_batches_decode_like_one(cuda, slots):
     """One token for each of many sequences: every cluster size of the attention and every width of the matmuls."""
