@@ -127,9 +127,9 @@ SMC_API const char *smc_last_error(smc_ctx *ctx);
  *   "prompt_attention_heads_per_cta"  0 (default): the tcgen05 kernel, or the mma.sync kernel with two query heads that
  *                           share a KV head per CTA; 1: the mma.sync kernel with one.  Same bits either way
  *   "small_batch_ring"      2..32 rows in SMC_ACT_Q8: weights through the bulk-copy ring for 1 Q4_K, 2 every format,
- *                           0 (default) never (then the kernel that fetches its fragments from global memory runs; the
- *                           two add a row's blocks in different orders: results agree within the mode's bound, not
- *                           bit for bit)
+ *                           0 (default) never (then the kernels that split a row's blocks over warps run, with their operands
+ *                           staged in shared memory or fetched from global memory, the same bits; the ring kernel adds a
+ *                           row's blocks in another order: results agree within the mode's bound, not bit for bit)
  * No option takes results out of their bounds.  SMC_E_INVALID for an unknown name. */
 SMC_API int smc_set_option(smc_ctx *ctx, const char *name, int value);
 /* QuantizationOps.GetRawTensorByteCount for a [N, K] tensor (QuantizationOps.cs:15-72); -1 if dtype unknown. */

@@ -298,8 +298,9 @@ __global__ void __launch_bounds__(128 * HPC) sdpa_prefill_mma_kernel(const float
 //   3. only O += P V and l follow the tiles in order; CTA r does it for one head and 32 output dims, a warp for 8 of them, while the other four warps
 //      bring V and the weights, those from the CTA that made them through distributed shared memory
 // Shared memory stays below half an SM's: with one CTA per SM fewer than 16 clusters of eight were resident at once, and the
-// 16 head pairs of a 32-head model took two waves.  What bounds it: step 1's MMAs, and step 3's rounds of three tiles (2200 clocks each).  When a CTA did 16 dims of both heads and its MMA warps read the weights themselves, every CTA of the cluster read all weights of both, tile by tile from
-// the same CTA, and 280 bytes of a thread's registers were spilled: 1360 clocks a tile, 740 now.
+// 16 head pairs of a 32-head model took two waves.  What bounds it: step 1's MMAs, and step 3's rounds of three tiles.  When a CTA did 16 dims of
+// both heads and its MMA warps read the weights themselves, all CTAs of the cluster read the weights of a tile of both heads from the same CTA at the
+// same time, and 280 bytes of a thread's registers were spilled.
 // Six rows over 1021 keys, 32 heads on 8 KV heads of 128, one layer: 175 us in the kernel above, 43 -> 33 us here (101 keys 16 -> 13, 2200 keys 78 -> 55);
 // a 32-layer pass of six rows 3557 -> 3241 us, of a small model's 28 layers 1601 -> 1334.  (The request into L2 ahead of the predecessor's end is 0.5 and 5 % of that.)
 // Scores and weights of all of a CTA's tiles are kept in shared memory, which ends at 14 tiles: 3584 keys at head size 128, 1792 at 64.

@@ -5,7 +5,8 @@
 // tcgen05.mma kind::f16 with fp32 accumulators gives the bits of mma.sync.m16n8k16 over the same chain of K = 16 steps (compared
 // over chains of up to 24 steps of mixed magnitudes), and nothing else of the order of sums changes here: scores from two
 // accumulators (even and odd steps of the head size), keys in tiles of 32, running maximum, correction and row sum per tile,
-// the lanes' partial row sums in the shuffle's order.  So an output has the bits it has in the other kernel.
+// the lanes' partial row sums in the shuffle's order.  So an output has the bits it has in the other kernel, where the values that its row's last
+// key tile covers are finite (below).
 //
 // attn_planes_kernel first writes the three planes of all keys and values a call sees, in the tensor cores' core-matrix order, V
 // transposed, to scratch of the model or cache object: once per KV head instead of once per query head and row tile (split inside the attention kernel,
@@ -21,10 +22,10 @@
 //                   tile's threads take their scores of that next chunk before they wait for their turn at O
 // TMEM (512 columns at head size 128): Q 3 x 64, O 128, scores 2 accumulators x 64, P 3 x 16.  An MMA with the A operand in TMEM
 // takes 56 clocks for any N up to 112 (64 at 128): 64 keys at once halve what the scores cost with 32.
-// A row's slice of 16 leaves (O / l is stored) after the last tile that its causal bound reaches, as in the other kernel: what
-// later keys hold, infinities included, never meets it.
-// What bounds it: the softmax threads (4900 clocks a tile, most of it exponentials and splits) and the order S, P, O of the chunks;
-// the MMAs are 4200 clocks of a chunk's 8000.
+// A row's slice of 16 leaves (O / l is stored) after the last tile that its causal bound reaches, as in the other kernel: keys of later tiles never
+// meet it.  Masked keys inside that last tile enter with weight 0, so an infinite or undefined value there makes the row undefined, in both
+// kernels; the other one takes keys past its CTA's 64 rows for zeros, this one those past the whole call.
+// What bounds it: the softmax threads (exponentials and splits) and the order S, P, O of the chunks, which keeps the MMAs from overlapping them.
 // Measured, us a call (sdpa_prefill_mma_kernel before): 2048 rows, 16 heads of 128 on 8 KV heads 362 -> 164 (Q8_0 cache 412 -> 158),
 // 777 rows of 32 heads 140 -> 85, 128 rows behind 1000 keys 206 -> 90, 512 rows of heads of 64 57 -> 33.
 #include <cuda_bf16.h>
