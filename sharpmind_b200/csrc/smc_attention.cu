@@ -391,16 +391,26 @@ int launch_split_g(smc_ctx *ctx, int G, dim3 grid, size_t smem, cudaStream_t s, 
                    const void *v, const __half *kd, const __half *vd, float *part, int heads, int kvHeads, int kvLen, int maxSeq,
                    float scale, int splits, float *out, unsigned *tickets, int hshare)
 {
-    auto go = [&](auto kernel) {
-        smc_launch_dep(ctx->use_pdl, kernel, grid, dim3(SPLIT_THREADS), smem, s, q, k, v, kd, vd, part, heads, kvHeads, kvLen, maxSeq, scale, splits,
-                       out, tickets, hshare);
-    };
     const long long ctas = (long long)grid.x * grid.y * grid.z;
+    // A lane's 64 (32) bytes of an fp32 row are four (two) loads, whose sectors and lines meet in L1.  The staged matmuls between the layers' attentions leave an
+    // SM with some 20 KB of it, too few for more than two CTAs, so such grids ask for it back.  Measured, us a step without / with, 32 layers of 32 heads on 8 of
+    // 128: 32 sequences at 2100 positions 20198 / 9893, 16 at 1000 7102 / 4703, two at 1000 (320 CTAs) 3004 / 2739; 28 layers of 16 heads on 8: 32 at 2100
+    // 8595 / 3624.  Below the line it costs up to 1 % (two at 150, 48 CTAs, 923 / 937; two at 1000, 256 CTAs, 973 / 986), and one sequence, whose matmuls are
+    // others, gains nothing (304 CTAs 2173 / 2179); nor does Q8_0, whose lanes take their row's bytes in one load (16 at 2100 5203 / 5226).
+    const bool own_l1 = !Q8 && grid.z > 1 && ctas > 2LL * ctx->sm_count;
+    auto go = [&](auto kernel, int per_sm) {
+        if (own_l1)
+            smc_launch_dep_l1(ctx->use_pdl, smc_l1_carveout(smem, per_sm), kernel, grid, dim3(SPLIT_THREADS), smem, s, q, k, v, kd, vd, part, heads, kvHeads, kvLen, maxSeq,
+                              scale, splits, out, tickets, hshare);
+        else
+            smc_launch_dep(ctx->use_pdl, kernel, grid, dim3(SPLIT_THREADS), smem, s, q, k, v, kd, vd, part, heads, kvHeads, kvLen, maxSeq, scale, splits,
+                           out, tickets, hshare);
+    };
     if (G == 1) {
-        split_forms_deep<DPL, 1, Q8>(ctas, ctx->sm_count) ? go(sdpa_decode_split_kernel<DPL, 1, Q8, true>) : go(sdpa_decode_split_kernel<DPL, 1, Q8, false>);
+        split_forms_deep<DPL, 1, Q8>(ctas, ctx->sm_count) ? go(sdpa_decode_split_kernel<DPL, 1, Q8, true>, split_form(DPL, 1, Q8, true).ctas) : go(sdpa_decode_split_kernel<DPL, 1, Q8, false>, split_form(DPL, 1, Q8, false).ctas);
     } else {
-        if constexpr (Q8 && DPL == 16) go(sdpa_decode_split_kernel<DPL, 2, Q8, true>);
-        else split_forms_deep<DPL, 2, Q8>(ctas, ctx->sm_count) ? go(sdpa_decode_split_kernel<DPL, 2, Q8, true>) : go(sdpa_decode_split_kernel<DPL, 2, Q8, false>);
+        if constexpr (Q8 && DPL == 16) go(sdpa_decode_split_kernel<DPL, 2, Q8, true>, split_form(DPL, 2, Q8, true).ctas);
+        else split_forms_deep<DPL, 2, Q8>(ctas, ctx->sm_count) ? go(sdpa_decode_split_kernel<DPL, 2, Q8, true>, split_form(DPL, 2, Q8, true).ctas) : go(sdpa_decode_split_kernel<DPL, 2, Q8, false>, split_form(DPL, 2, Q8, false).ctas);
     }
     SMC_LAUNCH_CHECK(ctx);
     return SMC_OK;

@@ -383,6 +383,24 @@ inline void smc_launch_dep(bool allow_overlap, void (*kernel)(KArgs...), dim3 gr
     cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// What the CTAs of a kernel that lives on L1 ask of an SM's memory, in per cent: room for `ctas` of them, the rest being L1.
+inline int smc_l1_carveout(size_t smem, int ctas) { return (int)((ctas * (smem + 1024) * 100 + 228 * 1024 - 1) / (228 * 1024)); }
+
+// smc_launch_dep that asks for a division of the SM's memory for this one launch: without it an SM keeps the division that the kernel before has left.
+template <class... KArgs, class... Args>
+inline void smc_launch_dep_l1(bool allow_overlap, int carveout, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    at[0].val.sharedMemCarveout = (unsigned)carveout;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at, cfg.numAttrs = allow_overlap ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 // The same with the grid's CTAs paired into thread-block clusters of `cluster_x` (the grid must be a multiple of it).
 template <class... KArgs, class... Args>
 inline void smc_launch_dep_cluster(bool allow_overlap, int cluster_x, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,

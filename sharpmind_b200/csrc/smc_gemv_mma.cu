@@ -1007,7 +1007,7 @@ static StagedForm staged_form(const smc_ctx *ctx, const smc_weight *w, int M)
 template <class Kernel>
 static void keep_l1(Kernel kernel, size_t smem, int ctas)
 {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)((ctas * (smem + 1024) * 100 + 228 * 1024 - 1) / (228 * 1024)));
+    cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, smc_l1_carveout(smem, ctas));
 }
 
 template <bool Q4, int WR, int NT, int S>
