@@ -1028,8 +1028,13 @@ int smc_launch_gemv_mma(smc_ctx *ctx, const smc_q8act *a, const smc_weight *w, f
     const int nt = M <= 8 ? 1 : (M <= 16 ? 2 : 4);
     const dim3 grid((N + MMA_ROWS - 1) / MMA_ROWS, (M + 8 * nt - 1) / (8 * nt));
     if (const int pt = prompt_tile(ctx, w, M)) {
-        auto go = [&](auto kernel, size_t smem, int ncls) {
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        // `fit` CTAs share an SM.  A grid of fewer asks for so much shared memory that they cannot: while the kernel before it drains, the first SMs to be free
+        // were given several and others none.  Measured, us (one CTA an SM): fp32 rows over Q6_K 4096 x 14336 with 63 rows (128 CTAs) 315 -> 217, Q8_0 3072 x 1024 with 50
+        // (144 CTAs) 17.2 -> 13.4.
+        auto go = [&](auto kernel, size_t need, int fit, int ncls) {
+            const long long sms = ctx->sm_count, each = ((long long)((N + TILE_ROWS - 1) / TILE_ROWS) * ((M + 16 * pt - 1) / (16 * pt)) + sms - 1) / sms;
+            const size_t alone = 228 * 1024 / 2, apart = each < fit ? 228 * 1024 / (size_t)(each + 1) : 0, smem = need > apart ? need : apart;
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)alone);
             const int tok = 16 * pt, most = 65535 * tok;  // tokens of a launch: what the grid's y takes
             for (int t0 = 0; t0 < M; t0 += most) {
                 const int m = M - t0 < most ? M - t0 : most;
@@ -1040,9 +1045,9 @@ int smc_launch_gemv_mma(smc_ctx *ctx, const smc_q8act *a, const smc_weight *w, f
         };
         if (w->dtype == SMC_Q6_K) {
             const int ncls = K >= 8192 ? 16 : 8;
-            pt == 6 ? go(gemv_mma_tile_kernel<true, 6, 2>, TileShape<true, 6>::SMEM, ncls) : go(gemv_mma_tile_kernel<true, 4, 2>, TileShape<true, 4>::SMEM, ncls);
-        } else if (pt == 8) go(gemv_mma_tile_kernel<false, 8, 2>, TileShape<false, 8>::SMEM, 8);
-        else pt == 6 ? go(gemv_mma_tile_kernel<false, 6, 2>, TileShape<false, 6>::SMEM, 8) : go(gemv_mma_tile_kernel<false, 4, 3>, TileShape<false, 4>::SMEM, 8);
+            pt == 6 ? go(gemv_mma_tile_kernel<true, 6, 2>, TileShape<true, 6>::SMEM, 2, ncls) : go(gemv_mma_tile_kernel<true, 4, 2>, TileShape<true, 4>::SMEM, 2, ncls);
+        } else if (pt == 8) go(gemv_mma_tile_kernel<false, 8, 2>, TileShape<false, 8>::SMEM, 2, 8);
+        else pt == 6 ? go(gemv_mma_tile_kernel<false, 6, 2>, TileShape<false, 6>::SMEM, 2, 8) : go(gemv_mma_tile_kernel<false, 4, 3>, TileShape<false, 4>::SMEM, 3, 8);
     } else if (w->dtype == SMC_Q8_0 && M >= 64) {
         const size_t smem = (size_t)MMA_WARPS * Q8_PASS * RED_LD * sizeof(float);
         cudaFuncSetAttribute(gemv_mma_q8_0_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

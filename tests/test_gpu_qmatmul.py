@@ -146,6 +146,38 @@ def test_prompt_tiles_keep_the_small_batch_bits(cuda, dev, dtype, n, m, ks):
         cuda.release(w)
 
 
+def _us(f):
+    import torch
+
+    times = []
+    for _ in range(4):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        for _ in range(10):
+            f()
+        b.record()
+        torch.cuda.synchronize()
+        times.append(a.elapsed_time(b) * 100.0)
+    return min(times[1:])
+
+
+@pytest.mark.parametrize("few,more", [(63, 66)])
+def test_fewer_fp32_rows_over_q6_k_take_no_longer(cuda, dev, few, more):
+    """Grids on either side of a line in the work's division: where the CTAs do not spread over the SMs, the fewer rows took 1.25 times as long."""
+    import torch
+
+    from sharpmind_b200.ops import Mode
+
+    n, k = 4096, 14336
+    g = torch.Generator(device="cuda").manual_seed(8)
+    w = cuda.register_dev(dev.quantize_weights(Q6_K, torch.randn((n, k), generator=g, device="cuda") * 0.02), Q6_K, n, k)
+    x = torch.randn((more, k), generator=g, device="cuda")
+    less = x[:few].contiguous()
+    a, b = _us(lambda: dev.qmatmul(less, w, Mode.ACT_F32)), _us(lambda: dev.qmatmul(x, w, Mode.ACT_F32))
+    assert a <= 1.05 * b, (a, b)
+    cuda.release(w)
+
+
 def test_more_token_tiles_than_a_grid_holds():
     """Rows beyond 65535 tiles of tokens: the last ones have the bits they have in a small batch."""
     import torch
