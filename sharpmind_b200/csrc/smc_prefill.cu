@@ -545,7 +545,7 @@ prefill_q4k_kernel(const uint8_t *__restrict__ raw, const __half *__restrict__ i
 // What bounds it: the hand-overs.  The tensor pipe is active 51 % of the time; of 1.65 us per 64 elements of K about 1 us stays whichever of
 // drain, fold, unpacking and copies is left out (24 MMAs a stage 447 us, 20 420 us, 12 366 us, before the fold's and the issuing thread's
 // changes).  Before, fp32 rows went through mma.sync as three int8 digit planes, one scaling on the CUDA cores per output, plane and 16 elements.
-// 4096 x 14336 with 500 rows: 1595 -> 371 us (158 useful TFLOP/s); distance from 64 bits 1.84e-7 -> 1.33e-7, 8192 x 28672
+// 4096 x 14336 with 500 rows: 1595 -> 356 us (165 useful TFLOP/s); distance from 64 bits 1.84e-7 -> 1.33e-7, 8192 x 28672
 // 2.26e-7 -> 1.42e-7, 1024 x 4096 1.50e-7 -> 1.26e-7.
 constexpr int Q6_RAW = 208;                        // bytes of a row and block in shared memory: X, Y, Z (64 each), 16 scales: an odd multiple of 16
 constexpr int Q6_NW = 3;                           // blocks in flight
@@ -605,12 +605,12 @@ __device__ __forceinline__ void expand_q6(uint32_t q, __nv_bfloat162 sc, uint32_
 
 __global__ void __launch_bounds__(THREADS, 1)
 prefill_q6k_kernel(const uint8_t *__restrict__ q6u, const __nv_bfloat16 *__restrict__ img, const float *__restrict__ scale, float *__restrict__ out, int N, int K,
-                   int M, int ntt, int *status)
+                   int M, int ntt, int by_tokens, int *status)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t sbase = smem_u32(smem);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int rt = blockIdx.x / ntt, tt = blockIdx.x % ntt, row0 = rt * TM, nsb = K / 256;
+    const int rt = by_tokens ? blockIdx.x % by_tokens : blockIdx.x / ntt, tt = by_tokens ? blockIdx.x / by_tokens : blockIdx.x % ntt, row0 = rt * TM, nsb = K / 256;
     volatile uint32_t *abort_flag = reinterpret_cast<volatile uint32_t *>(smem + Q6_OFF_BAR + Q6_BARS * 8 + 4);
     auto bar = [&](int i) { return sbase + Q6_OFF_BAR + 8u * (uint32_t)i; };
 
@@ -916,7 +916,13 @@ int smc_launch_prefill_q6k(smc_ctx *ctx, const float *x, const smc_weight *w, fl
     prefill_scale_kernel<<<M, 256, 0, s>>>(x, M, K, 64, scale);
     prefill_q6k_image_kernel<<<ntt * (K / 256), 256, 0, s>>>(x, M, K, scale, img);
     SMC_CUDA(ctx, cudaFuncSetAttribute(prefill_q6k_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Q6_SMEM));
-    prefill_q6k_kernel<<<(N / TM) * ntt, THREADS, Q6_SMEM, s>>>(w->q6u, img, scale, out, N, K, M, ntt, ctx->d_status);
+    // In one wave, neighbouring CTAs (and SMs) take the same tokens: the activations are most of what they read, and they stay in step.  With the same weights
+    // instead, a last tile of few tokens ran ahead of its neighbour, whose sums go through `out` more often.  Us, weights / tokens shared: 8192 x 28672 with
+    // 130 rows 836 / 655, 256 rows 680 / 677; 4096 x 14336 with 130 rows 339 .. 366 / 344, 200 rows 337 / 345, 400 rows 412 / 352, 500 rows 361 / 355.
+    // Over several waves the weights are better read once (8192 x 28672, 500 rows 1309 / 1404).
+    const int strips = N / TM, ctas = strips * ntt;
+    const bool by_tokens = ctas <= ctx->sm_count;
+    prefill_q6k_kernel<<<ctas, THREADS, Q6_SMEM, s>>>(w->q6u, img, scale, out, N, K, M, ntt, by_tokens ? strips : 0, ctx->d_status);
     SMC_LAUNCH_CHECK(ctx);
     return SMC_OK;
 }

@@ -161,14 +161,15 @@ def _us(f):
     return min(times[1:])
 
 
-@pytest.mark.parametrize("few,more", [(63, 66)])
-def test_fewer_fp32_rows_over_q6_k_take_no_longer(cuda, dev, few, more):
-    """Grids on either side of a line in the work's division: where the CTAs do not spread over the SMs, the fewer rows took 1.25 times as long."""
+@pytest.mark.parametrize("n,few,more", [(4096, 63, 66), (8192, 130, 256)])
+def test_fewer_fp32_rows_over_q6_k_take_no_longer(cuda, dev, n, few, more):
+    """Grids on either side of a line in the work's division: where the CTAs do not spread over the SMs, or a last tile of few tokens runs out of step
+    with its neighbour, the fewer rows took 1.2 times as long."""
     import torch
 
     from sharpmind_b200.ops import Mode
 
-    n, k = 4096, 14336
+    k = 14336
     g = torch.Generator(device="cuda").manual_seed(8)
     w = cuda.register_dev(dev.quantize_weights(Q6_K, torch.randn((n, k), generator=g, device="cuda") * 0.02), Q6_K, n, k)
     x = torch.randn((more, k), generator=g, device="cuda")
