@@ -12,7 +12,7 @@
 // the same way once per CTA.  The score tile's accumulator layout is the A-operand layout of the next MMA for
 // 16-bit types, so P goes from registers to registers.  Online softmax per row as in the scalar kernel.
 // sm_100a runs mma.sync on its legacy tensor path.  smc_attention_tc.cu is the tcgen05 form, with the same bits; this kernel stays for calls of
-// one key tile, outputs off 16 bytes, one head per CTA (an option) and calls that the other's planes do not reach (a very long cache, a full device).
+// one to a few key tiles, outputs off 16 bytes, one head per CTA (an option) and calls that the other's planes do not reach (a very long cache, a full device).
 #include <cuda_bf16.h>
 
 #include "smc_common.cuh"
@@ -572,9 +572,13 @@ static int launch_prefill_mma(smc_ctx *ctx, smc_attn_planes *planes, const float
         SMC_LAUNCH_CHECK(ctx);
         return SMC_OK;
     }
-    // More than one tile of keys: tcgen05, two launches.  16 heads of 128: 20 rows (one tile) 10.8 us here, 13.1 there; 33 rows of 4 heads
-    // 16.0 / 13.8; 64 rows of 32 heads 18.0 / 14.3; 100 rows behind 1900 keys of a Q8_0 cache 398 / 149; 2048 rows 362 / 164.
-    if (tiles > 1 && ctx->attn_hpc != 1 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+    // From so many tiles of keys on tcgen05, two launches.  What the kernels below take grows with the tiles, 2.3 us each at heads of 64 in a CTA of their own to 6 at
+    // Q8_0 heads of 128 in pairs, whatever the rows; the other takes 2.4 (heads of 64) or 3.0 us a chunk of two and 7 more.  Measured, us, here / there: heads of
+    // 128 in pairs, fp32: 20 keys 10.8 / 13.1, 40 14.1 / 12.4; alone: 40 11.4 / 12.4, 96 with 60 rows 18.3 / 17.8, 128 19.0 / 15.4, Q8_0 40 14.4 / 14.6; heads of 64 in
+    // pairs: 64 9.0 / 9.9, 96 11.9 / 12.3, 128 15.0 / 12.2, Q8_0 96 13.4 / 14.5, 128 16.9 / 14.5; alone: 64 7.7 / 9.9, 128 12.4 / 12.3, 160 14.8 / 16.0,
+    // 192 17.1 / 14.8, Q8_0 96 12.8 / 14.4, 128 16.1 / 14.3.  Longer: 100 rows behind 1900 keys of a Q8_0 cache, heads of 128 398 / 149; 2048 rows 362 / 164.
+    const int first = hd == 128 ? (two || kd ? 2 : 3) : (two || kd ? 4 : 6);
+    if (tiles >= first && ctx->attn_hpc != 1 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
         const int rc = smc_launch_sdpa_prefill_tc(ctx, planes, q, kc, vc, kd, vd, out, T, nh, nkv, hd, pos0, maxSeq, scale, s);
         if (rc != SMC_E_UNSUPPORTED) return rc;  // else the planes do not reach that far (a very long cache, a full device)
     }
