@@ -542,7 +542,7 @@ prefill_q4k_kernel(const uint8_t *__restrict__ raw, const __half *__restrict__ i
 // five places of its unit, so they come by 16-byte asynchronous copies: a warp of the first four (plane 0) fetches the rows of its
 // quarter for both warps of the quarter and the pair meets at a named barrier; plane 0 unpacks the first 32 elements of each
 // stage, plane 1 the second 32.
-// What bounds it: the hand-overs.  The tensor pipe is active 51 % of the time; of 1.65 us per 64 elements of K about 1 us stays whichever of
+// What bounds it: the hand-overs.  The tensor pipe is active 53 % of the time; of 1.65 us per 64 elements of K about 1 us stays whichever of
 // drain, fold, unpacking and copies is left out (24 MMAs a stage 447 us, 20 420 us, 12 366 us, before the fold's and the issuing thread's
 // changes).  Before, fp32 rows went through mma.sync as three int8 digit planes, one scaling on the CUDA cores per output, plane and 16 elements.
 // 4096 x 14336 with 500 rows: 1595 -> 356 us (165 useful TFLOP/s); distance from 64 bits 1.84e-7 -> 1.33e-7, 8192 x 28672
